@@ -26,7 +26,8 @@ struct Level {
     DBuf<float> s_r_w32, s_p_w32;
     // pinned operator: FP64 in the level's slot order [k][n]; FP32 with each
     // row's slots sorted by neighbour index, [k][ld4] (rows padded to a
-    // multiple of 4 with zero weights), indices in sidx
+    // multiple of 4 with zero weights, slots to a multiple of 8 with weight 0
+    // on the row itself, as the transfers' are), indices in sidx
     DBuf<double> A64, dinv64;
     DBuf<double> A64s;  // FP64 copy in the sorted slot order of A32, [k][ld4] (compact FP64 V-cycle)
     DBuf<float> A32, dinv32;
@@ -37,9 +38,16 @@ struct Level {
     DBuf<double> bnd_A64;
     DBuf<float> bnd_A32;
     int nbl = 0;
+    // interior rows with boundary neighbours (SolveLevel): row tags, list, operator copies
+    DBuf<uint8_t> tag;
+    DBuf<int> near_list, near_idx, kb_idx;
+    DBuf<double> near_A64, kb_a64, kb_d64;
+    DBuf<float> near_A32, kb_a32, kb_d32;
+    int nn = 0, ldn = 0, kb = 0;
     double lmax = 2.0;
     // compact FP32-path indices (int16 offsets): off16 [k][ld4] (sorted slots), r_off16/p_off16 [k][n]
     DBuf<short> off16, r_off16, p_off16;
+    DBuf<short> offu16;  // level 0: offsets of idx in the level's own slot order, slots padded to a multiple of 8, [kp][n]
     bool off_ok = false, r_off_ok = false, p_off_ok = false;
     // the compact operator again, tile-major ([ld / kTileRows][k][kTileRows],
     // rows padded to ld), streamed tile by tile into shared memory by bulk copies
@@ -115,7 +123,8 @@ struct mgm_ctx {
     bool compat = false, compat_ready = false;
     DBuf<double> compat_pw, compat_s;
     bool warm_suspended = false;      // no learned warm start in the solve for p_w
-    DBuf<int> tma_err;                // set by a tile-streamed kernel whose bounded wait ran out
+    DBuf<int> tma_err;                // set by a level kernel whose bounded wait ran out
+    DBuf<unsigned> step_sync;         // the level step's counters (zero between launches)
     double *h_pinned = nullptr;
     SmootherProfile prof;
     // captured V-cycles, [0] FP64, [1] FP32 (re-captured when solver settings change)

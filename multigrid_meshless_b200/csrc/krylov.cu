@@ -2,6 +2,7 @@
 // the dense Gauss-Jordan (partial pivoting) used once at set-up for the
 // coarsest-level inverse.
 #include "krylov.cuh"
+#include "rows.cuh"
 
 namespace mgm {
 
@@ -243,7 +244,7 @@ __global__ void k_fg_init(FgState *st, int m, int max_total, int max_restarts, d
     st->max_total = max_total;
     st->max_restarts = max_restarts;
     st->tol = tol;
-    st->j = st->j_done = st->total_it = st->restarts = st->vcycles = 0;
+    st->j = st->j_next = st->j_done = st->total_it = st->restarts = st->vcycles = 0;
     st->reorth = 0;
     st->go_outer = 1;
     st->go_inner = 0;
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(256) k_fg_begin(FgState *st, const double *__r
     if (st->restarts == 0 && st->total_it == 0 && relres > 0 && isfinite(relres))
         st->start_log_relres += log10(relres);
     st->j = 0;
+    st->j_next = 0;
     st->j_done = 0;
     int go = 0;
     if (!isfinite(relres)) {
@@ -328,142 +330,362 @@ __global__ void k_fg_load(int n, const double *__restrict__ V, long ld, const Fg
                           T *__restrict__ out)
 {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = (T)V[st->j * ld + i];
+    if (i < n) out[i] = (T)V[st->j_next * ld + i];
 }
 
-template <class T>
-__global__ void k_fg_store(int n, const T *__restrict__ z, T *__restrict__ Z, long ld, const FgState *__restrict__ st)
+// ---------------------------------------------------------------------------
+// The Arnoldi step after the V-cycle, chained launches.
+//
+//   k_fg_apply   w = A z into V_{j+1}, Z_j = z; on levels below kVecMinRows
+//                rows also the per-CTA partial sums of V_c . w (c <= j) and w . w
+//   k_fg_dots    those partial sums on the larger levels
+//   k_fg_orth1   h = the summed projections; w -= sum h_c V_c; partial sums of
+//                V_c . w and w . w of the result
+//   k_fg_orth2   when the first pass cancelled more than 1 - 1/sqrt(2) of |w|
+//                (the Daniel-Gragg-Kaufman-Stewart test): w -= sum h2_c V_c,
+//                partial sums of w . w
+//   k_fg_end     w /= |w|; CTA 0: Hessenberg column, Givens rotations, the
+//                residual estimate and the inner loop's condition
+//
+// A V-cycle reduces the error by about three, so w = A M v_j is close to v_j
+// and the second pass runs nearly every time: orth1 reads each V_c once for
+// the update and for the second pass's projections (a separate dot pass read
+// them again).  Below kFgSmall rows every CTA sums the partial sums it needs
+// itself; above, where they are up to 592 per vector, k_fg_reduce does.  The
+// small levels' step is 4 launches where it was 13 (36 us of the 128 us a
+// whole step took on 16k rows).
+//
+// Every sum keeps one order whatever kernel takes it: a thread's rows, the
+// lanes of a warp and the warps of a CTA by halving, the CTAs' partial sums
+// the same way from 256 threads.  The FP32 V-cycle inside the iteration
+// amplifies the last bit of an FP64 sum to 1e-8 of the solution, so the order
+// is part of the result.
+// ---------------------------------------------------------------------------
+constexpr int kFgThreads = 256, kFgWarps = kFgThreads / 32;
+constexpr int kFgSmall = 65536;     // rows from which dot products and their reductions are launches of their own
+constexpr int kFgChunk = 16;        // Krylov vectors whose values a thread keeps in registers
+
+// part: [0] projections and |w|^2 of the first pass, [1] of the second, [2] the last |w|^2
+static __host__ __device__ size_t fg_part_stride(int nb) { return (size_t)(kMaxKrylov + 2) * nb; }
+size_t fg_part_doubles(int n) { return 2 * fg_part_stride(dot_blocks(n)) + dot_blocks(n); }
+
+// the lanes' values by halving (lane 0)
+__device__ __forceinline__ double warp_halve(double v)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) Z[st->j * ld + i] = z[i];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
+// eight warps' values by halving
+__device__ __forceinline__ double warps_halve(const double *s)
+{
+    return ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
 }
 
-// V_{j+1} = A Z_j
-template <class T>
-__global__ void __launch_bounds__(256) k_fg_apply(int n, int k, const int *__restrict__ idx,
-                                                  const double *__restrict__ A, const T *__restrict__ Z, long ld,
-                                                  const FgState *__restrict__ st, double *__restrict__ V)
+// out[c] = sum of partial row c (nb values) over the CTA, c < cnt
+__device__ __forceinline__ void block_sum_parts(const double *part, int nb, int cnt, double *out,
+                                                double (*sm)[kFgWarps])
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int j = st->j;
-    V[(long)(j + 1) * ld + i] = ell_row_dot(idx, A, Z + (long)j * ld, n, k, i);
-}
-
-// partial dot products V_c . w (w = V_{j+1}) for c < cnt (pass 0: j+2, pass 1: j+1)
-__global__ void __launch_bounds__(256) k_fg_multidot(int n, const double *__restrict__ V, long ld,
-                                                     const FgState *__restrict__ st, int pass,
-                                                     double *__restrict__ part)
-{
-    if (pass == 1 && !st->reorth) return;
-    __shared__ double sm[32];
-    const int j = st->j;
-    const int cnt = pass == 0 ? j + 2 : j + 1;
-    const double *w = V + (long)(j + 1) * ld;
-    for (int c = 0; c < cnt; c++) {
-        double s = 0.0;
-        const double *vc = V + c * ld;
-        for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-            s = fma(vc[i], w[i], s);
-        s = bsum<256>(s, sm);
-        if (threadIdx.x == 0) part[(long)c * gridDim.x + blockIdx.x] = s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int c0 = 0; c0 < cnt; c0 += kFgChunk) {
+        double v[kFgChunk];
+#pragma unroll
+        for (int q = 0; q < kFgChunk; q++) {
+            v[q] = 0.0;
+            if (c0 + q < cnt)
+                for (int t = threadIdx.x; t < nb; t += kFgThreads) v[q] += __ldcg(part + (size_t)(c0 + q) * nb + t);
+        }
+#pragma unroll
+        for (int q = 0; q < kFgChunk; q++) {
+            if (c0 + q >= cnt) break;
+            const double s = warp_halve(v[q]);
+            if (lane == 0) sm[q][warp] = s;
+        }
+        __syncthreads();
+        if (threadIdx.x < kFgChunk && c0 + threadIdx.x < cnt) out[c0 + threadIdx.x] = warps_halve(sm[threadIdx.x]);
+        __syncthreads();
     }
 }
 
-// h[c] (pass 0) or h2[c] (pass 1) = sum_t part[c * nblk + t], one block per c
-__global__ void k_fg_reduce_dots(const double *__restrict__ part, int nblk, FgState *__restrict__ st, int pass)
+// the CTA's sums of m per-thread values acc into part[(c0 + q) * nb + blk], q < m
+__device__ __forceinline__ void block_store_parts(const double (&acc)[kFgChunk], int m, int c0, double *part, int nb,
+                                                  double (*sm)[kFgWarps])
 {
-    if (pass == 1 && !st->reorth) return;
-    __shared__ double sm[32];
-    const int cnt = pass == 0 ? st->j + 2 : st->j + 1;
-    const int c = blockIdx.x;
-    if (c >= cnt) return;
-    double s = 0.0;
-    for (int t = threadIdx.x; t < nblk; t += blockDim.x) s += part[(long)c * nblk + t];
-    s = bsum<256>(s, sm);
-    if (threadIdx.x == 0) (pass == 0 ? st->h : st->h2)[c] = s;
-}
-
-// w -= sum_{c <= j} h[c] V_c (h2 for pass 1), per-block partial |w|^2
-__global__ void __launch_bounds__(256) k_fg_orth(int n, const double *__restrict__ V, long ld,
-                                                 const FgState *__restrict__ st, int pass, double *__restrict__ part)
-{
-    if (pass == 1 && !st->reorth) return;
-    __shared__ double hs[kMaxKrylov + 1];
-    __shared__ double sm[32];
-    const int j = st->j;
-    const int cnt = j + 1;
-    const double *h = pass == 0 ? st->h : st->h2;
-    for (int c = threadIdx.x; c < cnt; c += blockDim.x) hs[c] = h[c];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < kFgChunk; q++) {
+        if (q >= m) break;
+        const double v = warp_halve(acc[q]);
+        if (lane == 0) sm[q][warp] = v;
+    }
     __syncthreads();
-    double *w = const_cast<double *>(V) + (long)(j + 1) * ld;
-    double acc = 0.0;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        double s = w[i];
-        for (int c = 0; c < cnt; c++) s = fma(-hs[c], V[c * ld + i], s);
-        w[i] = s;
-        acc = fma(s, s, acc);
+    if (threadIdx.x < m) part[(size_t)(c0 + threadIdx.x) * nb + blockIdx.x] = warps_halve(sm[threadIdx.x]);
+    __syncthreads();
+}
+
+// sums of the partial rows c < cnt (SECOND: of the second pass, the last row
+// |w|^2 into st->nrm; third: one row, into st->nrm), one CTA per row
+enum FgReduce { FG_RED_FIRST = 0, FG_RED_SECOND = 1, FG_RED_LAST = 2 };
+template <int WHICH>
+__global__ void __launch_bounds__(kFgThreads) k_fg_reduce(const double *part, int nb, FgState *st)
+{
+    __shared__ double sm[kFgChunk][kFgWarps];
+    __shared__ double out[1];
+    pdl_wait<true>();
+    const int j = __ldcg(WHICH == FG_RED_FIRST ? &st->j_next : &st->j);
+    const int c = blockIdx.x, cnt = WHICH == FG_RED_LAST ? 1 : j + 2;
+    if (c >= cnt || (WHICH == FG_RED_LAST && !__ldcg(&st->reorth))) return;
+    block_sum_parts(part + (size_t)c * nb, nb, 1, out, sm);
+    if (threadIdx.x != 0) return;
+    if (WHICH == FG_RED_FIRST) {
+        st->h[c] = out[0];
+        if (c == 0) st->j = j;
+    } else if (WHICH == FG_RED_SECOND && c <= j) {
+        st->h2[c] = out[0];
+    } else {
+        st->nrm = out[0];
     }
-    acc = bsum<256>(acc, sm);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
 
-__global__ void k_fg_reduce_nrm(const double *__restrict__ part, int nblk, FgState *__restrict__ st, int pass)
+// a row of the operator in the level's own slot order: KC > 0 int16 offsets in
+// padded rows, the first KC slots before the wait; KC = 0 by chunks of 8
+// (IDX: 32-bit indices)
+template <int KC, bool IDX>
+struct FgRow {
+    RowChunk<double, KC ? KC : 8, IDX> R;
+    __device__ __forceinline__ void fetch(const FgOperator &op, int i)
+    {
+        if (KC || op.k >= 8) R.fetch(op.gi, op.A, op.n, i, i, 0);
+    }
+    template <class X>
+    __device__ __forceinline__ double dot(const FgOperator &op, const X *x, int i)
+    {
+        if constexpr (KC > 0) {
+            const double s = R.template dot<true>(x, 0.0);
+            return row_rest<true, double, KC, IDX>(op.gi, op.A, x, op.n, op.kp, i, i, s);
+        } else {
+            return row_big<double, IDX>(R, op.gi, op.A, x, op.n, op.k, i, i);
+        }
+    }
+};
+
+template <class T, int KC, bool IDX, bool SMALL>
+__global__ void __launch_bounds__(kFgThreads) k_fg_apply(FgOperator op, const T *z, T *Z, double *V, long ld,
+                                                         const FgState *st, double *part)
 {
-    if (pass == 1 && !st->reorth) return;
-    __shared__ double sm[32];
-    double s = 0.0;
-    for (int t = threadIdx.x; t < nblk; t += blockDim.x) s += part[t];
-    s = bsum<256>(s, sm);
-    if (threadIdx.x == 0) st->nrm = s;
+    __shared__ double sm[kFgChunk][kFgWarps];
+    const int i0 = blockIdx.x * kFgThreads + threadIdx.x, i = min(i0, op.n - 1);
+    FgRow<KC, IDX> R;
+    R.fetch(op, i);
+    pdl_wait<SMALL>();
+    const int j = __ldcg(&st->j_next);
+    double w = R.dot(op, z, i);
+    const bool live = i0 < op.n;
+    if (live) {
+        Z[(long)j * ld + i] = __ldcg(z + i);
+        V[(long)(j + 1) * ld + i] = w;
+    }
+    if constexpr (SMALL) {
+        // dot_blocks(n) CTAs, one row per thread
+        for (int c0 = 0; c0 <= j + 1; c0 += kFgChunk) {
+            const int m = min(kFgChunk, j + 2 - c0);
+            double acc[kFgChunk];
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++) acc[q] = q < m && c0 + q <= j ? __ldcg(V + (long)(c0 + q) * ld + i) : w;
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++) acc[q] = live ? acc[q] * w : 0.0;
+            block_store_parts(acc, m, c0, part, gridDim.x, sm);
+        }
+    }
 }
 
-// Daniel-Gragg-Kaufman-Stewart test: re-orthogonalise when the first pass
-// cancelled more than 1 - 1/sqrt(2) of |w|
-__global__ void k_fg_dgks(FgState *st)
+__global__ void __launch_bounds__(kFgThreads, 2) k_fg_dots(int n, const double *V, long ld, const FgState *st,
+                                                        double *part)
 {
-    const int j = st->j;
-    for (int i = 0; i <= j; i++) st->h2[i] = 0.0;
-    st->reorth = st->nrm < 0.5 * st->h[j + 1];
+    __shared__ double sm[kFgChunk][kFgWarps];
+    pdl_wait<true>();
+    const int j = __ldcg(&st->j_next);
+    const double *w = V + (long)(j + 1) * ld;
+    for (int c0 = 0; c0 <= j + 1; c0 += kFgChunk) {
+        const int m = min(kFgChunk, j + 2 - c0);
+        double acc[kFgChunk];
+#pragma unroll
+        for (int q = 0; q < kFgChunk; q++) acc[q] = 0.0;
+        const long step = (long)gridDim.x * kFgThreads;
+        for (long i = (long)blockIdx.x * kFgThreads + threadIdx.x; i < n; i += step) {
+            const double wi = __ldcg(w + i);
+            double v[kFgChunk];
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++)
+                if (q < m) v[q] = __ldcg(V + (long)(c0 + q) * ld + i);
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++)
+                if (q < m) acc[q] = fma(v[q], wi, acc[q]);
+        }
+        block_store_parts(acc, m, c0, part, gridDim.x, sm);
+    }
 }
 
-// V_{j+1} /= |w|
-__global__ void k_fg_scale_w(int n, double *__restrict__ V, long ld, const FgState *__restrict__ st)
+template <bool SMALL>
+__global__ void __launch_bounds__(kFgThreads, 2) k_fg_orth1(int n, double *V, long ld, FgState *st,
+                                                            const double *part, double *part2)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double d = sqrt(st->nrm);
-    double *w = V + (long)(st->j + 1) * ld;
-    w[i] = d > 0 ? w[i] / d : 0.0;
+    __shared__ double hs[kMaxKrylov + 2];
+    __shared__ double sm[kFgChunk][kFgWarps];
+    pdl_wait<true>();
+    const int j = __ldcg(&st->j_next), nb = gridDim.x;
+    if constexpr (SMALL) {
+        block_sum_parts(part, nb, j + 2, hs, sm);
+        if (blockIdx.x == 0) {
+            for (int c = threadIdx.x; c < j + 2; c += kFgThreads) st->h[c] = hs[c];
+            if (threadIdx.x == 0) st->j = j;
+        }
+    } else {
+        for (int c = threadIdx.x; c <= j; c += kFgThreads) hs[c] = __ldcg(&st->h[c]);
+        __syncthreads();
+    }
+    double *w = V + (long)(j + 1) * ld;
+    const long step = (long)nb * kFgThreads, first = (long)blockIdx.x * kFgThreads + threadIdx.x;
+    if (j + 2 <= kFgChunk) {
+        // the vectors' values stay in registers between the update and the products
+        double acc[kFgChunk];
+#pragma unroll
+        for (int q = 0; q < kFgChunk; q++) acc[q] = 0.0;
+        for (long i = first; i < n; i += step) {
+            double v[kFgChunk], s = __ldcg(w + i);
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++)
+                if (q <= j) v[q] = __ldcg(V + (long)q * ld + i);
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++)
+                if (q <= j) s = fma(-hs[q], v[q], s);
+            w[i] = s;
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++) {
+                if (q <= j) acc[q] = fma(v[q], s, acc[q]);
+                if (q == j + 1) acc[q] = fma(s, s, acc[q]);
+            }
+        }
+        block_store_parts(acc, j + 2, 0, part2, nb, sm);
+        return;
+    }
+    for (long i = first; i < n; i += step) {
+        double s = __ldcg(w + i);
+        for (int c = 0; c <= j; c++) s = fma(-hs[c], __ldcg(V + (long)c * ld + i), s);
+        w[i] = s;
+    }
+    for (int c0 = 0; c0 <= j + 1; c0 += kFgChunk) {
+        const int m = min(kFgChunk, j + 2 - c0);
+        double acc[kFgChunk];
+#pragma unroll
+        for (int q = 0; q < kFgChunk; q++) acc[q] = 0.0;
+        for (long i = first; i < n; i += step) {
+            const double wi = w[i];
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++)
+                if (q < m) acc[q] = fma(c0 + q <= j ? __ldcg(V + (long)(c0 + q) * ld + i) : wi, wi, acc[q]);
+        }
+        block_store_parts(acc, m, c0, part2, nb, sm);
+    }
 }
 
-// End of an Arnoldi step: Hessenberg column j, the previous Givens rotations
-// applied to it, a new rotation, the updated residual estimate |g_{j+1}| /
-// |b|, and the inner loop's condition.
-__global__ void k_fg_arnoldi_end(FgState *st, FgHandles hd)
+template <bool SMALL>
+__global__ void __launch_bounds__(kFgThreads, 2) k_fg_orth2(int n, double *V, long ld, FgState *st,
+                                                            const double *part2, double *part3)
 {
-    const int j = st->j, m = st->m;
-    double *col = st->H + (long)j * (m + 1);
-    for (int i = 0; i <= j; i++) col[i] = st->h[i] + st->h2[i];
-    col[j + 1] = sqrt(fmax(st->nrm, 0.0));
+    __shared__ double hs[kMaxKrylov + 2];
+    __shared__ double sm[kFgChunk][kFgWarps];
+    pdl_wait<true>();
+    const int j = __ldcg(&st->j), nb = gridDim.x;
+    const double ww = __ldcg(&st->h[j + 1]);
+    bool again;
+    if constexpr (SMALL) {
+        block_sum_parts(part2, nb, j + 2, hs, sm);
+        const double nrm = hs[j + 1];
+        again = nrm < 0.5 * ww;
+        if (blockIdx.x == 0) {
+            for (int c = threadIdx.x; c <= j; c += kFgThreads) st->h2[c] = hs[c];
+            if (threadIdx.x == 0) st->nrm = nrm;
+        }
+    } else {
+        again = __ldcg(&st->nrm) < 0.5 * ww;
+        for (int c = threadIdx.x; c <= j; c += kFgThreads) hs[c] = __ldcg(&st->h2[c]);
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->reorth = again;
+    if (!again) return;
+    double *w = V + (long)(j + 1) * ld;
+    const long step = (long)nb * kFgThreads;
+    double acc[kFgChunk];
+    acc[0] = 0.0;
+    for (long i = (long)blockIdx.x * kFgThreads + threadIdx.x; i < n; i += step) {
+        double s = __ldcg(w + i);
+        for (int c0 = 0; c0 <= j; c0 += kFgChunk) {
+            double v[kFgChunk];
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++)
+                if (c0 + q <= j) v[q] = __ldcg(V + (long)(c0 + q) * ld + i);
+#pragma unroll
+            for (int q = 0; q < kFgChunk; q++)
+                if (c0 + q <= j) s = fma(-hs[c0 + q], v[q], s);
+        }
+        w[i] = s;
+        acc[0] = fma(s, s, acc[0]);
+    }
+    block_store_parts(acc, 1, 0, part3, nb, sm);
+}
+
+// V_{j+1} /= |w|.  CTA 0 ends the step: Hessenberg column j, the previous
+// Givens rotations applied to it, a new rotation, the updated residual
+// estimate |g_{j+1}| / |b|, and the inner loop's condition.  (The other CTAs
+// read st->j, which the next step's first orthogonalisation rewrites;
+// st->j_next is written here.)
+template <bool SMALL>
+__global__ void __launch_bounds__(kFgThreads) k_fg_end(int n, double *V, long ld, FgState *st, const double *part3,
+                                                       int nb, FgHandles hd)
+{
+    __shared__ double s_nrm[1];
+    __shared__ double sm[kFgChunk][kFgWarps];
+    __shared__ double col[kMaxKrylov + 1], cs[kMaxKrylov], sn[kMaxKrylov];
+    pdl_wait<true>();
+    const int j = __ldcg(&st->j);
+    const bool again = __ldcg(&st->reorth) != 0;
+    if (SMALL && again) block_sum_parts(part3, nb, 1, s_nrm, sm);
+    else if (threadIdx.x == 0) s_nrm[0] = __ldcg(&st->nrm);
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i <= j; i += kFgThreads) {
+            col[i] = st->h[i] + (again ? st->h2[i] : 0.0);
+            if (i < j) { cs[i] = st->cs[i]; sn[i] = st->sn[i]; }
+        }
+    __syncthreads();
+    const double nrm = s_nrm[0], d = sqrt(nrm);
+    double *w = V + (long)(j + 1) * ld;
+    for (long i = (long)blockIdx.x * kFgThreads + threadIdx.x; i < n; i += (long)gridDim.x * kFgThreads)
+        w[i] = d > 0 ? __ldcg(w + i) / d : 0.0;
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    const int m = st->m;
+    col[j + 1] = sqrt(fmax(nrm, 0.0));
     for (int i = 0; i < j; i++) {
-        const double t0 = st->cs[i] * col[i] + st->sn[i] * col[i + 1];
-        col[i + 1] = -st->sn[i] * col[i] + st->cs[i] * col[i + 1];
+        const double t0 = cs[i] * col[i] + sn[i] * col[i + 1];
+        col[i + 1] = -sn[i] * col[i] + cs[i] * col[i + 1];
         col[i] = t0;
     }
     const double a = col[j], b = col[j + 1];
     const double rden = hypot(a, b);
-    st->cs[j] = rden > 0 ? a / rden : 1.0;
-    st->sn[j] = rden > 0 ? b / rden : 0.0;
-    col[j] = rden;
-    col[j + 1] = 0.0;
-    st->g[j + 1] = -st->sn[j] * st->g[j];
-    st->g[j] = st->cs[j] * st->g[j];
+    const double csj = rden > 0 ? a / rden : 1.0, snj = rden > 0 ? b / rden : 0.0;
+    st->cs[j] = csj;
+    st->sn[j] = snj;
+    double *H = st->H + (long)j * (m + 1);
+    for (int i = 0; i < j; i++) H[i] = col[i];
+    H[j] = rden;
+    H[j + 1] = 0.0;
+    const double gj = st->g[j], gn = -snj * gj;
+    st->g[j + 1] = gn;
+    st->g[j] = csj * gj;
     st->total_it++;
     st->vcycles++;
     st->vcycles_total++;
     st->j_done = j + 1;
-    const double est = fabs(st->g[j + 1]) / st->bnorm;
+    const double est = fabs(gn) / st->bnorm;
     int go = 0;
     if (!isfinite(est)) {
         // no update from this cycle; the outer loop stops (its condition is
@@ -474,22 +696,62 @@ __global__ void k_fg_arnoldi_end(FgState *st, FgHandles hd)
         st->j_done = 0;
     } else if (!(est < st->tol) && j + 1 < m) {
         go = 1;
-        st->j = j + 1;
+        st->j_next = j + 1;
     }
     st->go_inner = go;
     set_cond(hd.inner, hd.use, go);
 }
 
-// y = H^-1 g (upper triangular, j_done columns); re-asserts the outer loop's
-// condition, which an Arnoldi step may have cleared
-__global__ void k_fg_solve_y(FgState *st, FgHandles hd)
+// r = b - A x, per-CTA {|r|^2, |b|^2}
+template <int KC, bool IDX>
+__global__ void __launch_bounds__(256) k_fg_resid(FgOperator op, const double *__restrict__ b, const double *x,
+                                                  double *__restrict__ r, double *__restrict__ part)
 {
-    set_cond(hd.outer, hd.use, st->go_outer);
-    const int jd = st->j_done, m = st->m;
+    __shared__ double sm[32];
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, i = min(i0, op.n - 1);
+    FgRow<KC, IDX> R;
+    R.fetch(op, i);
+    const double bi = b[i];
+    asm volatile("" ::: "memory");  // the operator loads above stay ahead of the gathers
+    const double ri = bi - R.dot(op, x, i);
+    double rr = 0, bb = 0;
+    if (i0 < op.n) {
+        r[i] = ri;
+        rr = ri * ri;
+        bb = bi * bi;
+    }
+    rr = bsum<256>(rr, sm);
+    bb = bsum<256>(bb, sm);
+    if (threadIdx.x == 0) { part[2 * blockIdx.x] = rr; part[2 * blockIdx.x + 1] = bb; }
+}
+
+// y = H^-1 g (upper triangular, j_done columns); re-asserts the outer loop's
+// condition, which an Arnoldi step may have cleared.  One warp brings the
+// first kSolveCols columns into shared memory, one lane then solves by rows
+// (each row's sum in column order): from global memory that chain of loads
+// took 11 us for 15 columns.
+constexpr int kSolveCols = 48;
+__global__ void __launch_bounds__(32) k_fg_solve_y(FgState *st, FgHandles hd)
+{
+    __shared__ double H[kSolveCols][kSolveCols + 1], y[kMaxKrylov];
+    const int jd = st->j_done, m = st->m, lane = threadIdx.x;
+    if (lane == 0) set_cond(hd.outer, hd.use, st->go_outer);
+    for (int q = 0; q < min(jd, kSolveCols); q++)
+        for (int i = lane; i <= q; i += 32) H[i][q] = st->H[(long)q * (m + 1) + i];
+    for (int i = lane; i < jd; i += 32) y[i] = st->g[i];
+    __syncwarp();
+    if (lane != 0) return;
     for (int i = jd - 1; i >= 0; i--) {
-        double s = st->g[i];
-        for (int q = i + 1; q < jd; q++) s -= st->H[(long)q * (m + 1) + i] * st->y[q];
-        st->y[i] = s / st->H[(long)i * (m + 1) + i];
+        double s = y[i];
+        if (jd <= kSolveCols) {
+#pragma unroll 8
+            for (int q = i + 1; q < jd; q++) s -= H[i][q] * y[q];
+            y[i] = s / H[i][i];
+        } else {
+            for (int q = i + 1; q < jd; q++) s -= st->H[(long)q * (m + 1) + i] * y[q];
+            y[i] = s / st->H[(long)i * (m + 1) + i];
+        }
+        st->y[i] = y[i];
     }
 }
 
@@ -582,54 +844,48 @@ void fg_load(int n, const double *V, long ld, const FgState *st, T *out, cudaStr
 template void fg_load<double>(int, const double *, long, const FgState *, double *, cudaStream_t);
 template void fg_load<float>(int, const double *, long, const FgState *, float *, cudaStream_t);
 template <class T>
-void fg_store(int n, const T *z, T *Z, long ld, const FgState *st, cudaStream_t s)
+void fg_arnoldi(const FgOperator &op, const T *z, T *Z, double *V, long ld, FgState *st, double *part, FgHandles hd,
+                cudaStream_t s, Chain &launch)
 {
-    k_fg_store<T><<<blocks_for(n, 256), 256, 0, s>>>(n, z, Z, ld, st);
-    MGM_LAUNCHED();
+    const int n = op.n, nb = dot_blocks(n), rows = blocks_for(n, kFgThreads), b = kFgThreads;
+    double *part2 = part + fg_part_stride(nb), *part3 = part2 + fg_part_stride(nb);
+    if (n < kFgSmall) {
+        if (!op.idx16) launch(k_fg_apply<T, 0, true, true>, rows, b, 0, s, op, z, Z, V, ld, st, part);
+        else if (op.kp <= 16) launch(k_fg_apply<T, 8, false, true>, rows, b, 0, s, op, z, Z, V, ld, st, part);
+        else if (op.kp <= 24) launch(k_fg_apply<T, 24, false, true>, rows, b, 0, s, op, z, Z, V, ld, st, part);
+        else launch(k_fg_apply<T, 32, false, true>, rows, b, 0, s, op, z, Z, V, ld, st, part);
+        launch(k_fg_orth1<true>, nb, b, 0, s, n, V, ld, st, part, part2);
+        launch(k_fg_orth2<true>, nb, b, 0, s, n, V, ld, st, part2, part3);
+        launch(k_fg_end<true>, rows, b, 0, s, n, V, ld, st, part3, nb, hd);
+        return;
+    }
+    if (op.idx16) launch(k_fg_apply<T, 0, false, false>, rows, b, 0, s, op, z, Z, V, ld, st, part);
+    else launch(k_fg_apply<T, 0, true, false>, rows, b, 0, s, op, z, Z, V, ld, st, part);
+    launch(k_fg_dots, nb, b, 0, s, n, V, ld, st, part);
+    launch(k_fg_reduce<FG_RED_FIRST>, kMaxKrylov + 2, b, 0, s, part, nb, st);
+    launch(k_fg_orth1<false>, nb, b, 0, s, n, V, ld, st, part, part2);
+    launch(k_fg_reduce<FG_RED_SECOND>, kMaxKrylov + 2, b, 0, s, part2, nb, st);
+    launch(k_fg_orth2<false>, nb, b, 0, s, n, V, ld, st, part2, part3);
+    launch(k_fg_reduce<FG_RED_LAST>, 1, b, 0, s, part3, nb, st);
+    launch(k_fg_end<false>, 148 * 8, b, 0, s, n, V, ld, st, part3, nb, hd);
 }
-template void fg_store<double>(int, const double *, double *, long, const FgState *, cudaStream_t);
-template void fg_store<float>(int, const float *, float *, long, const FgState *, cudaStream_t);
-template <class T>
-void fg_apply(int n, int k, const int *idx, const double *A, const T *Z, long ld, const FgState *st, double *V,
-              cudaStream_t s)
+template void fg_arnoldi<double>(const FgOperator &, const double *, double *, double *, long, FgState *, double *,
+                                 FgHandles, cudaStream_t, Chain &);
+template void fg_arnoldi<float>(const FgOperator &, const float *, float *, double *, long, FgState *, double *,
+                                FgHandles, cudaStream_t, Chain &);
+
+void fg_resid(const FgOperator &op, const double *b, const double *x, double *r, double *part, cudaStream_t s)
 {
-    k_fg_apply<T><<<blocks_for(n, 256), 256, 0, s>>>(n, k, idx, A, Z, ld, st, V);
-    MGM_LAUNCHED();
-}
-template void fg_apply<double>(int, int, const int *, const double *, const double *, long, const FgState *,
-                               double *, cudaStream_t);
-template void fg_apply<float>(int, int, const int *, const double *, const float *, long, const FgState *, double *,
-                              cudaStream_t);
-void fg_gram_schmidt(int n, double *V, long ld, FgState *st, int pass, double *part, cudaStream_t s)
-{
-    const int nb = dot_blocks(n);
-    k_fg_multidot<<<nb, 256, 0, s>>>(n, V, ld, st, pass, part);
-    MGM_LAUNCHED();
-    k_fg_reduce_dots<<<kMaxKrylov + 2, 256, 0, s>>>(part, nb, st, pass);
-    MGM_LAUNCHED();
-    k_fg_orth<<<nb, 256, 0, s>>>(n, V, ld, st, pass, part);
-    MGM_LAUNCHED();
-    k_fg_reduce_nrm<<<1, 256, 0, s>>>(part, nb, st, pass);
-    MGM_LAUNCHED();
-}
-void fg_dgks(FgState *st, cudaStream_t s)
-{
-    k_fg_dgks<<<1, 1, 0, s>>>(st);
-    MGM_LAUNCHED();
-}
-void fg_scale_w(int n, double *V, long ld, const FgState *st, cudaStream_t s)
-{
-    k_fg_scale_w<<<blocks_for(n, 256), 256, 0, s>>>(n, V, ld, st);
-    MGM_LAUNCHED();
-}
-void fg_arnoldi_end(FgState *st, FgHandles hd, cudaStream_t s)
-{
-    k_fg_arnoldi_end<<<1, 1, 0, s>>>(st, hd);
-    MGM_LAUNCHED();
+    const int nb = blocks_for(op.n, 256);
+    if (!op.idx16) launch_k(k_fg_resid<0, true>, nb, 256, 0, s, op, b, x, r, part);
+    else if (op.n >= kFgSmall) launch_k(k_fg_resid<0, false>, nb, 256, 0, s, op, b, x, r, part);
+    else if (op.kp <= 16) launch_k(k_fg_resid<8, false>, nb, 256, 0, s, op, b, x, r, part);
+    else if (op.kp <= 24) launch_k(k_fg_resid<24, false>, nb, 256, 0, s, op, b, x, r, part);
+    else launch_k(k_fg_resid<32, false>, nb, 256, 0, s, op, b, x, r, part);
 }
 void fg_solve_y(FgState *st, FgHandles hd, cudaStream_t s)
 {
-    k_fg_solve_y<<<1, 1, 0, s>>>(st, hd);
+    k_fg_solve_y<<<1, 32, 0, s>>>(st, hd);
     MGM_LAUNCHED();
 }
 template <class T>

@@ -47,7 +47,9 @@ struct FgState {
     double beta, bnorm, relres, alpha;
     double tol;
     int m, max_total, max_restarts;
-    int j, j_done, total_it, restarts, vcycles;
+    int j;       // column of the running Arnoldi step, from its orthogonalisation on
+    int j_next;  // column of the step being started (V-cycle and operator product)
+    int j_done, total_it, restarts, vcycles;
     int reorth;
     int go_outer, go_inner;
     int status;
@@ -82,18 +84,23 @@ void fg_begin(FgState *st, const double *part, int nbres, FgHandles hd, cudaStre
 void fg_scale0(int n, double *V, const FgState *st, cudaStream_t s);
 template <class T>
 void fg_load(int n, const double *V, long ld, const FgState *st, T *out, cudaStream_t s);
+// The Arnoldi step after the V-cycle, z its result, chained after it (Chain):
+// V_{j+1} = A z with the projections on V_0..V_j and |w|^2, both Gram-Schmidt
+// passes, the scaling and the step's end (column j of the Hessenberg matrix,
+// Givens rotation, the inner loop's condition).  Z_j = z.  Partial sums in
+// part (fg_part_doubles(n) doubles).
+struct FgOperator {
+    int n, k, kp;       // rows, slots, padded slots (idx16)
+    const void *gi;     // int16 offsets (idx16) [kp][n], or 32-bit indices [k][n]
+    bool idx16;
+    const double *A;    // pinned FP64 operator in the same slot order, [kp][n]
+};
 template <class T>
-void fg_store(int n, const T *z, T *Z, long ld, const FgState *st, cudaStream_t s);
-template <class T>
-void fg_apply(int n, int k, const int *idx, const double *A, const T *Z, long ld, const FgState *st, double *V,
-              cudaStream_t s);
-// one Gram-Schmidt pass against V_0..V_j (pass 0: projections and |w|^2 of
-// V_0..V_{j+1}; pass 1, run only when the first asked for it: V_0..V_j) and
-// the update w -= sum h V with the new |w|^2
-void fg_gram_schmidt(int n, double *V, long ld, FgState *st, int pass, double *part, cudaStream_t s);
-void fg_dgks(FgState *st, cudaStream_t s);
-void fg_scale_w(int n, double *V, long ld, const FgState *st, cudaStream_t s);
-void fg_arnoldi_end(FgState *st, FgHandles hd, cudaStream_t s);
+void fg_arnoldi(const FgOperator &op, const T *z, T *Z, double *V, long ld, FgState *st, double *part, FgHandles hd,
+                cudaStream_t s, Chain &launch);
+size_t fg_part_doubles(int n);
+// r = b - A x and per-block {|r|^2, |b|^2} into part (a pair per 256 rows)
+void fg_resid(const FgOperator &op, const double *b, const double *x, double *r, double *part, cudaStream_t s);
 void fg_solve_y(FgState *st, FgHandles hd, cudaStream_t s);
 template <class T>
 void fg_combine(int n, const T *Z, long ld, const FgState *st, double *x, cudaStream_t s);

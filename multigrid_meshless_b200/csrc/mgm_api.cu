@@ -160,15 +160,21 @@ __global__ void k_make_offsets(int n, int ld, int k, const int *__restrict__ gid
 
 // The FP32 solver operator with each row's slots sorted by neighbour index
 // (consecutive rows then gather from nearby addresses in the same slot), [k][ld]
-// with ld >= n a multiple of 4; padding rows get weight 0 and index 0.
+// with ld >= n a multiple of 4; padding rows get weight 0 and index 0, the
+// padding slots k..kp-1 weight 0 and the row's own index.
 // The same sort gives the FP64 copy of the compact FP64 V-cycle (A64s, the
 // level's slot order permuted the same way).
-__global__ void __launch_bounds__(128) k_sort_slots(int n, int k, int ld, const int *__restrict__ idx,
+__global__ void __launch_bounds__(128) k_sort_slots(int n, int k, int kp, int ld, const int *__restrict__ idx,
                                                     const double *__restrict__ A64, int *__restrict__ sidx,
                                                     float *__restrict__ A32, double *__restrict__ A64s)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ld) return;
+    for (int j = k; j < kp; j++) {
+        sidx[(long)j * ld + i] = i < n ? i : 0;
+        A32[(long)j * ld + i] = 0.f;
+        A64s[(long)j * ld + i] = 0.0;
+    }
     if (i >= n) {
         for (int j = 0; j < k; j++) {
             sidx[(long)j * ld + i] = 0;
@@ -270,6 +276,67 @@ __global__ void k_decode_compact(int n, int k, int ld, const short *__restrict__
     w[t] = W[e];
 }
 
+// Row tags of the level step (SolveLevel): 1 boundary, 2 interior with a
+// boundary neighbour, 0 the other interior rows; 0/1 flags of the two lists
+// and the largest number of boundary slots of a near row.
+__global__ void k_tag_rows(int n, int k, const int *__restrict__ idx, const uint8_t *__restrict__ btag,
+                           uint8_t *__restrict__ tag, int *__restrict__ fb, int *__restrict__ fn,
+                           int *__restrict__ kbmax)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int nbs = 0;
+    const bool bnd = btag[i] != 0;
+    if (!bnd)
+        for (int j = 0; j < k; j++) nbs += btag[idx[(long)j * n + i]] != 0;
+    tag[i] = bnd ? 1 : (nbs ? 2 : 0);
+    fb[i] = bnd;
+    fn[i] = !bnd && nbs;
+    if (nbs) atomicMax(kbmax, nbs);
+}
+
+// list[pos[i]] = i where flag[i]
+__global__ void k_compact_list(int n, const int *__restrict__ flag, const int *__restrict__ pos, int *__restrict__ list)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && flag[i]) list[pos[i]] = i;
+}
+
+// The near rows' operator [k][ldn] in the sorted slot order, and of it the
+// boundary slots alone [kb][ldn].
+__global__ void k_gather_near(int nn, int ldn, const int *__restrict__ list, int k, int ld4,
+                              const int *__restrict__ sidx, const float *__restrict__ A32,
+                              const double *__restrict__ A64s, int *__restrict__ nidx, float *__restrict__ nA32,
+                              double *__restrict__ nA64, int kb, const uint8_t *__restrict__ btag,
+                              const float *__restrict__ dinv32, const double *__restrict__ dinv64,
+                              int *__restrict__ kidx, float *__restrict__ ka32, double *__restrict__ ka64,
+                              float *__restrict__ kd32, double *__restrict__ kd64)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nn) return;
+    const int i = list[t];
+    int m = 0;
+    for (int j = 0; j < k; j++) {
+        const long e = (long)j * ld4 + i, o = (long)j * ldn + t;
+        const int c = sidx[e];
+        nidx[o] = c;
+        nA32[o] = A32[e];
+        nA64[o] = A64s[e];
+        if (btag[c] && m < kb) {
+            const long q = (long)m++ * ldn + t;
+            kidx[q] = c;
+            ka32[q] = A32[e]; ka64[q] = A64s[e];
+            kd32[q] = dinv32[c]; kd64[q] = dinv64[c];
+        }
+    }
+    for (; m < kb; m++) {
+        const long q = (long)m * ldn + t;
+        kidx[q] = i;
+        ka32[q] = kd32[q] = 0.f;
+        ka64[q] = kd64[q] = 0.0;
+    }
+}
+
 // compact copies of the boundary rows of the pinned operator: out[w][j] = A[j][list[w]]
 __global__ void k_gather_rows(int nbl, const int *__restrict__ list, int n, int k, const int *__restrict__ idx,
                               const double *__restrict__ A, int *__restrict__ bidx, double *__restrict__ bA64,
@@ -318,14 +385,23 @@ void build_transfer(const Level &T, const Level &S, const DBuf<int> &pts, int ro
     Monomials mono = monomials(dim, S.poly);
     transfer_weights(nt, T.x.p, T.y.p, T.z.p, T.btag.p, pts.p, rows_from, only_interior, ks, dim, phs, mono, S.x.p,
                      S.y.p, S.z.p, S.cloud.p, rm.p, s);
-    w64.alloc((size_t)nt * ks);
+    // the solver's rows (w32) are padded to a multiple of 8 slots: weight 0, the row's base node
+    const int kp = w32 ? (ks + 7) & ~7 : ks;
+    const size_t nk = (size_t)nt * ks, nkp = (size_t)nt * kp;
+    w64.alloc(nkp);
     transpose_rowmajor_to_ell_d(rm.p, w64.p, nt, ks, s);
-    gidx.alloc((size_t)nt * ks);
-    k_gather_idx<<<blocks_for((long)nt * ks, 256), 256, 0, s>>>(nt, ks, pts.p, S.cloud.p, gidx.p);
+    gidx.alloc(nkp);
+    k_gather_idx<<<blocks_for((long)nk, 256), 256, 0, s>>>(nt, ks, pts.p, S.cloud.p, gidx.p);
     MGM_LAUNCHED();
     if (w32) {
-        w32->alloc((size_t)nt * ks);
-        convert_d2f(w64.p, w32->p, (long)nt * ks, s);
+        w32->alloc(nkp);
+        convert_d2f(w64.p, w32->p, (long)nk, s);
+        for (int j = ks; j < kp; j++)
+            MGM_CUDA(cudaMemcpyAsync(gidx.p + (size_t)j * nt, pts.p, sizeof(int) * nt, cudaMemcpyDeviceToDevice, s));
+        if (kp > ks) {
+            MGM_CUDA(cudaMemsetAsync(w64.p + nk, 0, sizeof(double) * (nkp - nk), s));
+            MGM_CUDA(cudaMemsetAsync(w32->p + nk, 0, sizeof(float) * (nkp - nk), s));
+        }
     }
     MGM_CUDA(cudaStreamSynchronize(s));
 }
@@ -340,9 +416,13 @@ std::vector<SolveLevel<double>> solve_levels<double>(mgm_ctx *c)
     for (int l = 0; l < c->nl; l++) {
         Level &L = c->L[l];
         SolveLevel<double> S{};
-        S.n = L.n; S.k = L.k; S.ld = L.n; S.nb_list = L.nbl;
-        S.idx = L.idx.p; S.A = L.A64.p; S.dinv = L.dinv64.p; S.btag = L.btag.p; S.bnd_list = L.bnd_list.p;
+        S.n = L.n; S.k = L.k; S.ld = L.ld4; S.nb_list = L.nbl;
+        S.idx = L.sidx.p; S.A = L.A64s.p; S.dinv = L.dinv64.p; S.btag = L.btag.p; S.bnd_list = L.bnd_list.p;
         S.bnd_idx = L.bnd_idx.p; S.bnd_A = L.bnd_A64.p;
+        S.tag = L.tag.p; S.nn = L.nn; S.ldn = L.ldn; S.kb = L.kb;
+        S.near_list = L.near_list.p; S.near_idx = L.near_idx.p; S.near_A = L.near_A64.p;
+        S.kb_idx = L.kb_idx.p; S.kb_a = L.kb_a64.p; S.kb_d = L.kb_d64.p;
+        S.sync = c->step_sync.p; S.tma_err = c->tma_err.p;
         S.r = L.r64.p; S.e = L.e64.p; S.e2 = L.e64b.p; S.d = L.d64.p; S.q = L.q64.p;
         S.kr = l > 0 ? c->L[l - 1].k : 0; S.r_idx = L.s_r_idx.p; S.r_w = L.s_r_w64.p;
         S.kp = l < c->nl - 1 ? c->L[l + 1].k : 0; S.p_idx = L.s_p_idx.p; S.p_w = L.s_p_w64.p;
@@ -350,7 +430,7 @@ std::vector<SolveLevel<double>> solve_levels<double>(mgm_ctx *c)
         if (c->compact) {
             // the FP32 path's layout with FP64 weights: slots sorted by
             // neighbour, int16 offsets, four rows per thread on large levels
-            if (L.off_ok) { S.ld = L.ld4; S.idx = L.sidx.p; S.A = L.A64s.p; S.off = L.off16.p; }
+            if (L.off_ok) S.off = L.off16.p;
             S.r_off = L.r_off_ok ? L.r_off16.p : nullptr; S.r_base = L.rpts.p;
             S.p_off = L.p_off_ok ? L.p_off16.p : nullptr; S.p_base = L.ppts.p;
         }
@@ -369,6 +449,10 @@ std::vector<SolveLevel<float>> solve_levels<float>(mgm_ctx *c)
         S.n = L.n; S.k = L.k; S.ld = L.ld4; S.nb_list = L.nbl;
         S.idx = L.sidx.p; S.A = L.A32.p; S.dinv = L.dinv32.p; S.btag = L.btag.p; S.bnd_list = L.bnd_list.p;
         S.bnd_idx = L.bnd_idx.p; S.bnd_A = L.bnd_A32.p;
+        S.tag = L.tag.p; S.nn = L.nn; S.ldn = L.ldn; S.kb = L.kb;
+        S.near_list = L.near_list.p; S.near_idx = L.near_idx.p; S.near_A = L.near_A32.p;
+        S.kb_idx = L.kb_idx.p; S.kb_a = L.kb_a32.p; S.kb_d = L.kb_d32.p;
+        S.sync = c->step_sync.p; S.tma_err = c->tma_err.p;
         S.r = L.r32.p; S.e = L.e32.p; S.e2 = L.e32b.p; S.d = L.d32.p; S.q = L.q32.p;
         S.kr = l > 0 ? c->L[l - 1].k : 0; S.r_idx = L.s_r_idx.p; S.r_w = L.s_r_w32.p;
         S.kp = l < c->nl - 1 ? c->L[l + 1].k : 0; S.p_idx = L.s_p_idx.p; S.p_w = L.s_p_w32.p;
@@ -378,7 +462,7 @@ std::vector<SolveLevel<float>> solve_levels<float>(mgm_ctx *c)
             S.r_off = L.r_off_ok ? L.r_off16.p : nullptr; S.r_base = L.rpts.p;
             S.p_off = L.p_off_ok ? L.p_off16.p : nullptr; S.p_base = L.ppts.p;
             if (c->use_tma && L.ldt > 0) {
-                S.At = L.A32t.p; S.offt = L.off16t.p; S.ldt = L.ldt; S.tma_err = c->tma_err.p;
+                S.At = L.A32t.p; S.offt = L.off16t.p; S.ldt = L.ldt;
             }
             if (c->half_operator && L.h_ok) { S.W16 = L.W16.p; S.ldi = L.ldi; }
         }
@@ -497,9 +581,10 @@ void check_wait_flags(mgm_ctx *c, cudaStream_t s)
     if (h_err) {
         c->tma_err.zero(s);
         c->fused_bar.zero(s);
+        c->step_sync.zero(s);
         MGM_CUDA(cudaStreamSynchronize(s));
-        throw Error{MGM_ERR_TIMEOUT, "Poisson solve: a level kernel's bounded wait ran out (tile copies or the "
-                                     "fused coarse V-cycle's grid barrier)"};
+        throw Error{MGM_ERR_TIMEOUT, "Poisson solve: a level kernel's bounded wait ran out (tile copies, a level "
+                                     "step's boundary rows or the fused coarse V-cycle's grid barrier)"};
     }
 }
 
@@ -517,12 +602,13 @@ void drop_graphs(mgm_ctx *c)
 // most of them on launch-latency-bound coarse levels).  Returns the level-0
 // correction buffer.
 template <class T>
-const T *run_vcycle(mgm_ctx *c, std::vector<SolveLevel<T>> &levels, const CoarseSolve<T> &cs)
+const T *run_vcycle(mgm_ctx *c, std::vector<SolveLevel<T>> &levels, const CoarseSolve<T> &cs, const double *V, long ldv,
+                    const FgState *st)
 {
     cudaStream_t s = c->s;
     if (!c->use_graphs) {
         const FusedCtl fc = fused_ctl(c);
-        vcycle<T>(levels, cs, c->cheb_deg, c->cheb_ratio, s, &c->prof, c->chain_launches, &fc);
+        vcycle<T>(levels, cs, c->cheb_deg, c->cheb_ratio, s, &c->prof, c->chain_launches, &fc, V, ldv, st);
         return levels[0].e;
     }
     auto &G = c->vg[sizeof(T) == 4 ? 1 : 0];
@@ -542,7 +628,8 @@ const T *run_vcycle(mgm_ctx *c, std::vector<SolveLevel<T>> &levels, const Coarse
         MGM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         try {
             const FusedCtl fc = fused_ctl(c);
-            vcycle<T>(cap, cs, c->cheb_deg, c->cheb_ratio, s, c->prof.on ? &c->prof : nullptr, c->chain_launches, &fc);
+            vcycle<T>(cap, cs, c->cheb_deg, c->cheb_ratio, s, c->prof.on ? &c->prof : nullptr, c->chain_launches, &fc, V,
+                      ldv, st);
         } catch (...) {
             cudaGraph_t junk = nullptr;
             cudaStreamEndCapture(s, &junk);
@@ -595,6 +682,7 @@ struct FgRun {
     double *V;
     long ld;
     int n, k, nbres;
+    FgOperator op;
     FgState *st;
     const double *b;
     double *p;
@@ -649,32 +737,26 @@ void capture_body(cudaGraph_t body, cudaStream_t bs, F &&fn)
     MGM_CUDA(cudaStreamEndCapture(bs, &out));
 }
 
-// one Arnoldi step: z_j = M v_j (V-cycle), w = A z_j, classical Gram-Schmidt
-// (projections and |w|^2 in one pass, the update with the norm of the result
-// in a second, a re-orthogonalisation pass only when the first cancelled more
-// than 1 - 1/sqrt(2) of |w|: the Daniel-Gragg-Kaufman-Stewart test), the
-// Givens update and the convergence test
+// one Arnoldi step: z_j = M v_j (V-cycle), then w = A z_j, classical
+// Gram-Schmidt with a re-orthogonalisation pass when the first cancelled more
+// than 1 - 1/sqrt(2) of |w| (the Daniel-Gragg-Kaufman-Stewart test), the
+// Givens update and the convergence test (fg_arnoldi)
 template <class T>
 void arnoldi_step(FgRun<T> &R, cudaStream_t s, FgHandles hd, bool captured)
 {
     mgm_ctx *c = R.c;
-    Level &L0 = c->L[0];
-    fg_load<T>(R.n, R.V, R.ld, R.st, R.levels[0].r, s);
     const T *z;
     if (captured) {
         const FusedCtl fc = fused_ctl(c);
-        vcycle<T>(R.levels, R.cs, c->cheb_deg, c->cheb_ratio, s, nullptr, c->chain_launches, &fc);
+        vcycle<T>(R.levels, R.cs, c->cheb_deg, c->cheb_ratio, s, nullptr, c->chain_launches, &fc, R.V, R.ld, R.st);
         z = R.levels[0].e;
     } else {
-        z = run_vcycle<T>(c, R.levels, R.cs);
+        z = run_vcycle<T>(c, R.levels, R.cs, R.V, R.ld, R.st);
     }
-    fg_store<T>(R.n, z, R.Z, R.ld, R.st, s);
-    fg_apply<T>(R.n, R.k, L0.idx.p, L0.A64.p, R.Z, R.ld, R.st, R.V, s);
-    fg_gram_schmidt(R.n, R.V, R.ld, R.st, 0, c->kpart.p, s);
-    fg_dgks(R.st, s);
-    fg_gram_schmidt(R.n, R.V, R.ld, R.st, 1, c->kpart.p, s);
-    fg_scale_w(R.n, R.V, R.ld, R.st, s);
-    fg_arnoldi_end(R.st, hd, s);
+    Chain launch;
+    launch.enabled = c->chain_launches;
+    launch.after_kernel = captured;  // the V-cycle's last kernel precedes it in the captured body
+    fg_arnoldi<T>(R.op, z, R.Z, R.V, R.ld, R.st, c->kpart.p, hd, s, launch);
     if (!captured && c->prof.on) {
         // the events of this V-cycle must have completed before they are read
         MGM_CUDA(cudaStreamSynchronize(c->s));
@@ -690,8 +772,7 @@ template <class T>
 void restart_cycle(FgRun<T> &R, cudaStream_t s, FgHandles hd, bool captured, long long *k_inner)
 {
     mgm_ctx *c = R.c;
-    Level &L0 = c->L[0];
-    resid64(R.n, R.k, L0.idx.p, L0.A64.p, R.b, R.p, R.V, c->kpart.p, s);
+    fg_resid(R.op, R.b, R.p, R.V, c->kpart.p, s);
     fg_begin(R.st, c->kpart.p, R.nbres, hd, s);
     fg_scale0(R.n, R.V, R.st, s);
     if (captured) {
@@ -770,6 +851,10 @@ void fgmres(mgm_ctx *c, const double *b, double *p, bool captured = false, long 
     R.k = L0.k;
     R.ld = L0.n;
     R.nbres = blocks_for(L0.n, 256);
+    R.op.n = L0.n; R.op.k = L0.k; R.op.kp = (L0.k + 7) & ~7;
+    R.op.idx16 = L0.off_ok;
+    R.op.gi = L0.off_ok ? (const void *)L0.offu16.p : (const void *)L0.idx.p;
+    R.op.A = L0.A64.p;
     R.levels = solve_levels<T>(c);
     R.cs.n = c->L[c->nl - 1].n;
     if constexpr (sizeof(T) == 8) R.cs.inv = (const T *)c->cinv64.p; else R.cs.inv = (const T *)c->cinv32.p;
@@ -1043,7 +1128,8 @@ void alloc_solver_buffers(mgm_ctx *c)
         c->hist_ok.zero(c->s);
     }
     c->bvec.alloc(n);
-    c->kpart.alloc((size_t)std::max(2 * blocks_for(n, 256), (kMaxKrylov + 1) * dot_blocks(n)) + 16);
+    c->kpart.alloc(std::max({(size_t)2 * blocks_for(n, 256), (size_t)(kMaxKrylov + 1) * dot_blocks(n),
+                             fg_part_doubles(n)}) + 16);
     c->kscal.alloc(3 * kMaxKrylov + 16);
     if (!c->fg.p) {
         c->fg.alloc(1);
@@ -1421,46 +1507,85 @@ void prepare_solver(mgm_ctx *c)
         Level &L = c->L[l];
         const size_t nk = (size_t)L.n * L.k;
         L.ld4 = (L.n + 3) & ~3;
-        const size_t nk4 = (size_t)L.ld4 * L.k;
-        L.A64.alloc(nk); L.A32.alloc(nk4); L.A64s.alloc(nk4); L.sidx.alloc(nk4); L.dinv64.alloc(L.n);
+        const int kp8 = (L.k + 7) & ~7;
+        const size_t nk4 = (size_t)L.ld4 * kp8;
+        L.A64.alloc((size_t)kp8 * L.n); L.A32.alloc(nk4); L.A64s.alloc(nk4); L.sidx.alloc(nk4); L.dinv64.alloc(L.n);
         L.dinv32.alloc(L.n);
         k_pin_operator<<<blocks_for((long)nk, 256), 256, 0, s>>>(L.n, L.k, L.lapP.p, L.A64.p, L.dinv64.p,
                                                                L.dinv32.p);
         MGM_LAUNCHED();
-        k_sort_slots<<<blocks_for(L.ld4, 128), 128, 0, s>>>(L.n, L.k, L.ld4, L.idx.p, L.A64.p, L.sidx.p, L.A32.p,
+        if (kp8 > L.k) MGM_CUDA(cudaMemsetAsync(L.A64.p + nk, 0, sizeof(double) * (size_t)(kp8 - L.k) * L.n, s));
+        k_sort_slots<<<blocks_for(L.ld4, 128), 128, 0, s>>>(L.n, L.k, kp8, L.ld4, L.idx.p, L.A64.p, L.sidx.p, L.A32.p,
                                                             L.A64s.p);
         MGM_LAUNCHED();
-        std::vector<uint8_t> hb(L.n);
-        L.btag.download(hb.data(), L.n, s);
-        MGM_CUDA(cudaStreamSynchronize(s));
-        std::vector<int> bl;
-        for (int i = 0; i < L.n; i++) if (hb[i]) bl.push_back(i);
-        L.nbl = (int)bl.size();
-        L.bnd_list.upload(bl.data(), bl.size(), s);
+        // boundary rows, and the interior rows next to them
+        {
+            DBuf<int> fb(L.n), fn(L.n), pos(L.n), tot(3);
+            tot.zero(s);
+            L.tag.alloc(L.n);
+            k_tag_rows<<<blocks_for(L.n, 256), 256, 0, s>>>(L.n, L.k, L.idx.p, L.btag.p, L.tag.p, fb.p, fn.p,
+                                                          tot.p + 2);
+            MGM_LAUNCHED();
+            L.bnd_list.alloc(L.n);
+            scan_exclusive(fb.p, pos.p, L.n, tot.p, s);
+            k_compact_list<<<blocks_for(L.n, 256), 256, 0, s>>>(L.n, fb.p, pos.p, L.bnd_list.p);
+            MGM_LAUNCHED();
+            L.near_list.alloc(L.n);
+            scan_exclusive(fn.p, pos.p, L.n, tot.p + 1, s);
+            k_compact_list<<<blocks_for(L.n, 256), 256, 0, s>>>(L.n, fn.p, pos.p, L.near_list.p);
+            MGM_LAUNCHED();
+            int h_tot[3] = {0, 0, 0};
+            tot.download(h_tot, 3, s);
+            MGM_CUDA(cudaStreamSynchronize(s));
+            L.nbl = h_tot[0];
+            L.nn = h_tot[1];
+            L.kb = h_tot[2];
+            L.ldn = (L.nn + 31) & ~31;
+            const size_t nkn = (size_t)L.k * L.ldn, nkb = (size_t)L.kb * L.ldn;
+            L.near_idx.alloc(nkn); L.near_A32.alloc(nkn); L.near_A64.alloc(nkn);
+            L.kb_idx.alloc(nkb); L.kb_a32.alloc(nkb); L.kb_a64.alloc(nkb); L.kb_d32.alloc(nkb); L.kb_d64.alloc(nkb);
+            if (L.nn > 0) {
+                k_gather_near<<<blocks_for(L.nn, 128), 128, 0, s>>>(
+                    L.nn, L.ldn, L.near_list.p, L.k, L.ld4, L.sidx.p, L.A32.p, L.A64s.p, L.near_idx.p, L.near_A32.p,
+                    L.near_A64.p, L.kb, L.btag.p, L.dinv32.p, L.dinv64.p, L.kb_idx.p, L.kb_a32.p, L.kb_a64.p,
+                    L.kb_d32.p, L.kb_d64.p);
+                MGM_LAUNCHED();
+            }
+        }
         L.bnd_idx.alloc((size_t)L.nbl * L.k);
         L.bnd_A64.alloc((size_t)L.nbl * L.k);
         L.bnd_A32.alloc((size_t)L.nbl * L.k);
-        k_gather_rows<<<blocks_for((long)L.nbl * L.k, 256), 256, 0, s>>>(L.nbl, L.bnd_list.p, L.n, L.k, L.idx.p,
-                                                                       L.A64.p, L.bnd_idx.p, L.bnd_A64.p,
-                                                                       L.bnd_A32.p);
-        MGM_LAUNCHED();
+        if (L.nbl > 0) {
+            k_gather_rows<<<blocks_for((long)L.nbl * L.k, 256), 256, 0, s>>>(L.nbl, L.bnd_list.p, L.n, L.k, L.idx.p,
+                                                                           L.A64.p, L.bnd_idx.p, L.bnd_A64.p,
+                                                                           L.bnd_A32.p);
+            MGM_LAUNCHED();
+        }
         // compact FP32-path indices
         {
             DBuf<int> ovf(3);
             ovf.zero(s);
             L.off16.alloc(nk4);
-            k_make_offsets<<<blocks_for((long)nk4, 256), 256, 0, s>>>(L.n, L.ld4, L.k, L.sidx.p, nullptr, L.off16.p,
+            k_make_offsets<<<blocks_for((long)nk4, 256), 256, 0, s>>>(L.n, L.ld4, kp8, L.sidx.p, nullptr, L.off16.p,
                                                                     ovf.p);
             MGM_LAUNCHED();
+            if (l == 0) {
+                // the outer iteration's operator, in the level's own slot order
+                L.offu16.alloc((size_t)kp8 * L.n);
+                MGM_CUDA(cudaMemsetAsync(L.offu16.p, 0, sizeof(short) * (size_t)kp8 * L.n, s));
+                k_make_offsets<<<blocks_for((long)nk, 256), 256, 0, s>>>(L.n, L.n, L.k, L.idx.p, nullptr, L.offu16.p,
+                                                                       ovf.p);
+                MGM_LAUNCHED();
+            }
             if (l > 0) {
-                const int kr = c->L[l - 1].k;
+                const int kr = (c->L[l - 1].k + 7) & ~7;
                 L.r_off16.alloc((size_t)L.n * kr);
                 k_make_offsets<<<blocks_for((long)L.n * kr, 256), 256, 0, s>>>(L.n, L.n, kr, L.s_r_idx.p, L.rpts.p,
                                                                              L.r_off16.p, ovf.p + 1);
                 MGM_LAUNCHED();
             }
             if (l < c->nl - 1) {
-                const int kp = c->L[l + 1].k;
+                const int kp = (c->L[l + 1].k + 7) & ~7;
                 L.p_off16.alloc((size_t)L.n * kp);
                 k_make_offsets<<<blocks_for((long)L.n * kp, 256), 256, 0, s>>>(L.n, L.n, kp, L.s_p_idx.p, L.ppts.p,
                                                                              L.p_off16.p, ovf.p + 2);
@@ -1512,14 +1637,13 @@ void prepare_solver(mgm_ctx *c)
     }
     {
         // the power iteration reads the operator in the level's own slot order
-        const bool compact = c->compact;
-        c->compact = false;
+        auto lv = solve_levels<double>(c);
         for (int l = 0; l < c->nl - 1; l++) {
-            auto lv = solve_levels<double>(c);
+            lv[l].idx = c->L[l].idx.p;
+            lv[l].A = c->L[l].A64.p;
             estimate_lmax<double>(lv[l], s);
             c->L[l].lmax = lv[l].lmax;
         }
-        c->compact = compact;
     }
     Level &Lc = c->L[c->nl - 1];
     MGM_REQUIRE(Lc.n <= 8192, "mgm_setup: coarsest level too large for the dense solve (use more levels)");
@@ -1538,6 +1662,8 @@ void prepare_solver(mgm_ctx *c)
     c->tma_err.zero(s);
     c->fused_bar.alloc(2);
     c->fused_bar.zero(s);
+    c->step_sync.alloc(2);
+    c->step_sync.zero(s);
     c->fused_blocks = fused_vcycle_blocks();
     MGM_CUDA(cudaStreamSynchronize(s));
     if (!cooperative_in_conditional_ok(c)) c->fused_blocks = 0;  // the per-operation kernels then

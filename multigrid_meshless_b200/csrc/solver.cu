@@ -16,6 +16,8 @@
 // Outer: flexible GMRES in FP64 (residuals, Krylov basis, solution updates).
 #include <cmath>
 
+#include "krylov.cuh"
+#include "rows.cuh"
 #include "stencil.cuh"
 
 namespace mgm {
@@ -49,95 +51,176 @@ __device__ __forceinline__ T ldv(const T *p)
     else return *p;
 }
 
-template <class T, bool COH = false>
-__device__ __forceinline__ void start_row(int i, const uint8_t *__restrict__ btag, const T *__restrict__ dinv,
-                                          const T *r, T *e)
-{
-    e[i] = btag[i] ? ldv<COH>(r + i) * dinv[i] : T(0);
-}
-// boundary row w of the list, by the 32 lanes of a warp
-template <class T, bool COH = false>
-__device__ __forceinline__ void bnd_row_warp(int w, int lane, const int *__restrict__ list, int k,
-                                             const int *__restrict__ bidx, const T *__restrict__ bA,
-                                             const T *__restrict__ dinv, const T *r, T *e)
-{
-    const int i = list[w];
-    T s = T(0);
-    for (int j = lane; j < k; j += 32) s += bA[(long)w * k + j] * ldv<COH>(e + bidx[(long)w * k + j]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) e[i] = ldv<COH>(e + i) + (ldv<COH>(r + i) - s) * dinv[i];
-}
-
-// Start of a smoothing pass from e = 0: interior rows 0, boundary rows their
-// exact solve r_i / a_ii (they couple only to interior nodes).
+// A boundary row by the lanes of a warp: its stencil (fetch: the first 64
+// slots), then its exact solve from the current e (value: lane 0).  A
+// boundary row couples only to itself and interior nodes, so rows can be
+// updated in place; the rows are stored row-major [nbl][k].
 template <class T>
-__global__ void __launch_bounds__(256) k_start_e(int n, const uint8_t *__restrict__ btag, const T *__restrict__ dinv,
-                                                 const T *__restrict__ r, T *__restrict__ e)
-{
-    pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) start_row(i, btag, dinv, r, e);
-}
+struct BndRow {
+    static constexpr int Q = 2;
+    int i = 0, w = 0, c[Q];
+    T a[Q], di;
+    __device__ __forceinline__ void fetch(int row, int lane, int nbl, const int *__restrict__ list, int k,
+                                          const int *__restrict__ bidx, const T *__restrict__ bA,
+                                          const T *__restrict__ dinv)
+    {
+        w = min(row, nbl - 1);
+        i = ldk(list + w);
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const long o = (long)w * k + min(lane + 32 * q, k - 1);
+            c[q] = ldk(bidx + o);
+            a[q] = ldk(bA + o);
+        }
+        di = ldk(dinv + i);
+    }
+    __device__ __forceinline__ T value(int lane, int k, const int *__restrict__ bidx, const T *__restrict__ bA,
+                                       const T *r, const T *e) const
+    {
+        T v[Q], s = T(0);
+        const T ri = __ldcg(r + i), ei = __ldcg(e + i);
+#pragma unroll
+        for (int q = 0; q < Q; q++) v[q] = __ldcg(e + c[q]);
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            if (lane + 32 * q < k) s = fma_rn(a[q], v[q], s);
+        for (int j = lane + 32 * Q; j < k; j += 32)
+            s = fma_rn(__ldg(bA + (long)w * k + j), __ldcg(e + __ldg(bidx + (long)w * k + j)), s);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        return fma_rn(ri - s, di, ei);
+    }
+};
 
-// Exact solve of the boundary rows, one warp per row.  A boundary row couples
-// only to itself and interior nodes, so rows can be updated in place.  The
-// rows are stored compactly (row-major [nbl][k]) so that a warp reads them
-// with coalesced loads.
-template <class T>
+// Exact solve of the boundary rows, one warp per row.
+template <class T, bool EARLY>
 __global__ void __launch_bounds__(256) k_bnd_exact(int nbl, const int *__restrict__ list, int k,
                                                    const int *__restrict__ bidx, const T *__restrict__ bA,
-                                                   const T *__restrict__ dinv, const T *__restrict__ r,
-                                                   T *__restrict__ e)
+                                                   const T *__restrict__ dinv, const T *r, T *e)
 {
-    pdl_enter();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= nbl) return;
-    bnd_row_warp(w, lane, list, k, bidx, bA, dinv, r, e);
+    BndRow<T> B;
+    B.fetch(w, lane, nbl, list, k, bidx, bA, dinv);
+    pdl_wait<EARLY>();
+    const T v = B.value(lane, k, bidx, bA, r, e);
+    if (lane == 0 && w < nbl) e[B.i] = v;
 }
 
-// One Chebyshev step on interior rows: q = r - A e, d = c1*d + c2*D^-1 q, e' = e + d.
-// Boundary rows copy e.  zero_start: e is zero except on boundary rows.
+// The first step of a smoothing pass from e = 0.  There e is zero but on the
+// boundary rows (their exact solve r_b / a_bb), so A e vanishes exactly on
+// the rows without boundary neighbours and the step needs no operator:
+// d = c2 D^-1 r, e' = d.  The rows with boundary neighbours (the near list)
+// subtract those neighbours' terms, stored compactly in slot order (ELL
+// [kb][ldn]: neighbour, weight, the neighbour's 1 / diagonal); the zero terms
+// that are left out change no bit of the sum.  16 bytes per row instead of
+// the operator's 6 k: 41.7 -> 6 us on level 0 of the 1M cavity.
+// FROMV: r is converted here from the FP64 Krylov vector V_j (j = st->j_next)
+// and stored for the later steps.
 template <class T>
-__global__ void __launch_bounds__(256) k_cheb(int n, int ld, int k, const int *__restrict__ idx, const T *__restrict__ A,
-                                              const T *__restrict__ dinv, const uint8_t *__restrict__ btag,
-                                              const T *__restrict__ r, const T *__restrict__ e, T *__restrict__ eout,
-                                              T *__restrict__ d, T c1, T c2, int first)
+struct FirstArgs {
+    int n, nn, kb, ldn, nrow;   // nrow: CTAs of the row part (the near rows' CTAs follow)
+    const uint8_t *tag;         // 0 far, 1 boundary, 2 near
+    const T *dinv;
+    T *r, *out, *d;
+    T c2;
+    const int *near_list, *kb_idx;
+    const T *kb_a, *kb_d;
+    const double *V;
+    long ldv;
+    const FgState *st;
+};
+
+template <class T, bool FROMV>
+__device__ __forceinline__ void first_row(const FirstArgs<T> &a, int i, int tg, T di)
 {
-    pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const T ei = e[i];
-    if (btag[i]) { eout[i] = ei; return; }
-    const T q = r[i] - ell_row_dot(idx, A, e, ld, k, i);
-    const T di = first ? c2 * dinv[i] * q : c1 * d[i] + c2 * dinv[i] * q;
-    d[i] = di;
-    eout[i] = ei + di;
+    T ri;
+    if constexpr (FROMV) {
+        ri = (T)__ldcg(a.V + (long)__ldcg(&a.st->j_next) * a.ldv + i);
+        a.r[i] = ri;
+    } else {
+        ri = __ldcg(a.r + i);
+    }
+    if (tg == 1) {
+        a.out[i] = ri * di;
+    } else if (tg == 0) {
+        const T dv = a.c2 * di * ri;
+        a.d[i] = dv;
+        a.out[i] = T(0) + dv;
+    }
 }
 
-// residual on interior rows (boundary rows are solved exactly: 0)
+constexpr int kFirstKB = 12;  // boundary slots of a near row fetched together
 template <class T>
-__global__ void __launch_bounds__(256) k_residual(int n, int ld, int k, const int *__restrict__ idx,
-                                                  const T *__restrict__ A, const uint8_t *__restrict__ btag,
-                                                  const T *__restrict__ r, const T *__restrict__ e, T *__restrict__ q)
+struct FirstNear {
+    int i, c[kFirstKB];
+    T w[kFirstKB], dn[kFirstKB], di;
+    __device__ __forceinline__ void slots(const FirstArgs<T> &a, int t, int q0)
+    {
+#pragma unroll
+        for (int q = 0; q < kFirstKB; q++) {
+            const bool in = q0 + q < a.kb;
+            const long o = (long)(in ? q0 + q : 0) * a.ldn + t;
+            c[q] = ldk(a.kb_idx + o);
+            w[q] = ldk(a.kb_a + o);
+            dn[q] = ldk(a.kb_d + o);
+            if (!in) w[q] = T(0);
+        }
+    }
+    __device__ __forceinline__ void fetch(const FirstArgs<T> &a, int t)
+    {
+        i = ldk(a.near_list + t);
+        di = ldk(a.dinv + i);
+        slots(a, t, 0);
+    }
+    template <bool FROMV>
+    __device__ __forceinline__ void finish(const FirstArgs<T> &a, int t)
+    {
+        const double *Vj = nullptr;
+        if constexpr (FROMV) Vj = a.V + (long)__ldcg(&a.st->j_next) * a.ldv;
+        auto rhs = [&](int x) -> T {
+            if constexpr (FROMV) return (T)__ldcg(Vj + x);
+            else return __ldcg(a.r + x);
+        };
+        const T ri = rhs(i);
+        T s = T(0);
+        for (int q0 = 0; q0 < a.kb; q0 += kFirstKB) {
+            if (q0 > 0) slots(a, t, q0);
+            T v[kFirstKB];
+#pragma unroll
+            for (int q = 0; q < kFirstKB; q++) v[q] = rhs(c[q]) * dn[q];
+#pragma unroll
+            for (int q = 0; q < kFirstKB; q++) s = fma_rn(w[q], v[q], s);
+        }
+        const T q = ri - s;
+        const T dv = a.c2 * di * q;
+        a.d[i] = dv;
+        a.out[i] = T(0) + dv;
+    }
+};
+
+template <class T, bool FROMV>
+__device__ __forceinline__ void first_near(const FirstArgs<T> &a, int t)
 {
-    pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (btag[i]) { q[i] = T(0); return; }
-    q[i] = r[i] - ell_row_dot(idx, A, e, ld, k, i);
+    FirstNear<T> F;
+    F.fetch(a, t);
+    F.template finish<FROMV>(a, t);
 }
 
-// coarse rhs: r_c[i] = sum_j Rw[j][i] q_f[Ridx[j][i]] on interior coarse rows, 0 elsewhere
-template <class T>
-__global__ void __launch_bounds__(256) k_restrict(int n, int k, const int *__restrict__ ridx, const T *__restrict__ rw,
-                                                  const uint8_t *__restrict__ btag, const T *__restrict__ qf,
-                                                  T *__restrict__ rc)
+template <class T, bool FROMV, bool EARLY>
+__global__ void __launch_bounds__(256) k_first_step(const __grid_constant__ FirstArgs<T> a)
 {
-    pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (btag[i] || i == 0) { rc[i] = T(0); return; }
-    rc[i] = ell_row_dot(ridx, rw, qf, n, k, i);
+    if ((int)blockIdx.x < a.nrow) {
+        const int i0 = blockIdx.x * blockDim.x + threadIdx.x, i = min(i0, a.n - 1);
+        const int tg = ldk(a.tag + i);
+        const T di = ldk(a.dinv + i);
+        pdl_wait<EARLY>();
+        if (i0 < a.n) first_row<T, FROMV>(a, i, tg, di);
+        return;
+    }
+    const int t0 = ((int)blockIdx.x - a.nrow) * blockDim.x + threadIdx.x, t = min(t0, a.nn - 1);
+    FirstNear<T> F;
+    F.fetch(a, t);
+    pdl_wait<EARLY>();
+    if (t0 < a.nn) F.template finish<FROMV>(a, t);
 }
 
 // (P e_c)[0], the prolongated correction at the pinned node, by the 32 lanes
@@ -158,26 +241,6 @@ __device__ __forceinline__ T row0_dot_warp(int k, Op operand)
         for (int q = 0; q < m; q++) s = fma_rn(__shfl_sync(0xffffffffu, a, q), __shfl_sync(0xffffffffu, x, q), s);
     }
     return s;
-}
-
-// e_f[i] += (P e_c)[i] - (P e_c)[0]  (the shift keeps the pinned node uncorrected)
-template <class T>
-__global__ void __launch_bounds__(256) k_prolong(int n, int k, const int *__restrict__ pidx, const T *__restrict__ pw,
-                                                 const T *__restrict__ ec, T *__restrict__ ef)
-{
-    pdl_enter();
-    __shared__ T shift;
-    if (threadIdx.x < 32) {
-        const T s = row0_dot_warp<T>(k, [&](int j, T &a, T &x) {
-            a = pw[(long)j * n];
-            x = ec[pidx[(long)j * n]];
-        });
-        if (threadIdx.x == 0) shift = s;
-    }
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    ef[i] += ell_row_dot(pidx, pw, ec, n, k, i) - shift;
 }
 
 // ---------------------------------------------------------------------------
@@ -226,48 +289,157 @@ __device__ __forceinline__ T ell_row_dot_o(const short *__restrict__ off, const 
 // Chebyshev step q = r - A e, d = c1 d + c2 D^-1 q, e' = e + d on interior
 // rows (boundary rows copy e); MODE 1: residual q = r - A e on interior rows,
 // 0 on boundary rows.
-template <int MODE, class T, bool COH = false>
-__device__ __forceinline__ void level_row_out(int i, T s, const T *__restrict__ dinv,
-                                              const uint8_t *__restrict__ btag, const T *r, const T *e, T *out, T *d,
-                                              T c1, T c2, int first)
-{
-    if (MODE == 0) {
-        const T ei = ldv<COH>(e + i);
-        if (btag[i]) { out[i] = ei; return; }
-        const T q = ldv<COH>(r + i) - s;
-        const T di = first ? c2 * dinv[i] * q : c1 * ldv<COH>(d + i) + c2 * dinv[i] * q;
-        d[i] = di;
-        out[i] = ei + di;
-    } else {
-        out[i] = btag[i] ? T(0) : ldv<COH>(r + i) - s;
-    }
-}
+// ---------------------------------------------------------------------------
+// One step on a level: the boundary rows' exact solve from the current e,
+// then the Chebyshev step (MODE 0) or the residual (MODE 1) of the interior
+// rows.  Only the near rows (interior rows with boundary neighbours) see the
+// boundary rows' new values.
+//
+// Levels below kVecMinRows rows: two chained launches (k_bnd_exact,
+// k_level_c1), each with its operands in registers before its wait.
+// The larger levels (k_level_v4): one launch in three parts --
+//   boundary  a warp per boundary row: e[b] (and out[b]); then one release
+//             increment of sync[0] per CTA;
+//   far       the interior rows without boundary neighbours;
+//   near      a thread per near row, after a bounded wait for the boundary
+//             part's increments; rows as their own ELL copy [k][ldn],
+//             gathers from L2.
+// The boundary part is dispatched before the near part (block order) and
+// waits for nothing, so the near part's wait ends; it is bounded all the
+// same: when it runs out the CTA sets *err (MGM_ERR_TIMEOUT on the host).
+// The last near CTA to pass resets the two counters for the next launch.
+// Same operands in the same order as separate launches: the same bits.
+// ---------------------------------------------------------------------------
+template <class T>
+struct StepArgsL {
+    int n, ld, k, kp, nbl, nn, ldn;
+    int nbc, nfar, nnc, fb;  // CTAs of the three parts; far CTAs dispatched before the boundary part
+    const void *gi;          // int16 offsets [k][ld] or 32-bit indices
+    const T *A, *dinv;
+    const uint8_t *tag;      // 0 far, 1 boundary, 2 near
+    const T *r;
+    T *e, *out, *d;
+    T c1, c2;
+    int first;
+    const int *bnd_list, *bnd_idx;
+    const T *bnd_A;
+    const int *near_list, *near_idx;
+    const T *near_A;
+    unsigned *sync;          // {boundary CTAs done, near CTAs passed}
+    int *err;
+};
 
-template <int MODE, class T, bool COHERENT = false>
-__device__ __forceinline__ void c1_row(int i, int ld, int k, const short *__restrict__ off, const T *__restrict__ A,
-                                       const T *__restrict__ dinv, const uint8_t *__restrict__ btag,
-                                       const T *__restrict__ r, const T *__restrict__ e, T *__restrict__ out,
-                                       T *__restrict__ d, T c1, T c2, int first)
+// the level's output of row i from its sum s
+template <int MODE, class T>
+__device__ __forceinline__ void step_out(const StepArgsL<T> &a, int i, T ri, T ei, T dprev, T di, T s)
 {
-    if (btag[i]) {
-        out[i] = MODE == 0 ? ldv<COHERENT>(e + i) : T(0);
-        return;
+    const T q = ri - s;
+    if (MODE == 0) {
+        const T dv = a.first ? a.c2 * di * q : a.c1 * dprev + a.c2 * di * q;
+        a.d[i] = dv;
+        a.out[i] = ei + dv;
+    } else {
+        a.out[i] = q;
     }
-    level_row_out<MODE, T, COHERENT>(i, ell_row_dot_o<T, T, COHERENT>(off, A, e, ld, k, i, i), dinv, btag, r, e, out,
-                                     d, c1, c2, first);
 }
 
 template <int MODE, class T>
-__global__ void __launch_bounds__(256) k_level_c1(int n, int ld, int k, const short *__restrict__ off,
-                                                  const T *__restrict__ A, const T *__restrict__ dinv,
-                                                  const uint8_t *__restrict__ btag, const T *__restrict__ r,
-                                                  const T *__restrict__ e, T *__restrict__ out,
-                                                  T *__restrict__ d, T c1, T c2, int first)
+__device__ __forceinline__ void step_bnd_part(const StepArgsL<T> &a, int blk)
 {
-    pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    c1_row<MODE, T>(i, ld, k, off, A, dinv, btag, r, e, out, d, c1, c2, first);
+    const int w = (blk * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    BndRow<T> B;
+    B.fetch(w, lane, a.nbl, a.bnd_list, a.k, a.bnd_idx, a.bnd_A, a.dinv);
+    pdl_wait<false>();
+    const T v = B.value(lane, a.k, a.bnd_idx, a.bnd_A, a.r, a.e);
+    if (lane == 0 && w < a.nbl) {
+        a.e[B.i] = v;
+        a.out[B.i] = MODE == 0 ? v : T(0);
+    }
+    if (a.nnc == 0) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.sync) : "memory");
+    }
+}
+
+template <int MODE, class T>
+__device__ __forceinline__ void step_near_part(const StepArgsL<T> &a, int blk)
+{
+    __shared__ int go;
+    const int t = blk * blockDim.x + threadIdx.x;
+    const bool live = t < a.nn;
+    const int tc = live ? t : 0;
+    const int i = ldk(a.near_list + tc);
+    const T di = ldk(a.dinv + i);
+    pdl_wait<false>();
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        if (a.nbc > 0) {
+            unsigned seen;
+            long spins = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.sync) : "memory");
+                if (++spins > (1L << 20)) {
+                    atomicExch(a.err, 1);
+                    ok = 0;
+                    break;
+                }
+            } while (seen < (unsigned)a.nbc);
+        }
+        go = ok;
+    }
+    __syncthreads();
+    if (live && go) {
+        const T ri = __ldcg(a.r + i);
+        T ei = T(0), dprev = T(0), s = T(0);
+        if (MODE == 0) {
+            ei = __ldcg(a.e + i);
+            if (!a.first) dprev = __ldcg(a.d + i);
+        }
+        int j = 0;
+        for (; j + 8 <= a.k; j += 8) {
+            RowChunk<T, 8, true> R;
+            R.fetch(a.near_idx, a.near_A, a.ldn, t, 0, j);
+            s = R.template dot<true>(a.e, s);
+        }
+        for (; j < a.k; j++) {
+            const long o = (long)j * a.ldn + t;
+            s = fma_rn(__ldg(a.near_A + o), __ldcg(a.e + __ldg(a.near_idx + o)), s);
+        }
+        step_out<MODE>(a, i, ri, ei, dprev, di, s);
+    }
+    if (threadIdx.x == 0 && go && a.nbc > 0 && atomicAdd(a.sync + 1, 1u) + 1u == (unsigned)a.nnc) {
+        atomicExch(a.sync + 1, 0u);
+        atomicExch(a.sync, 0u);
+    }
+}
+
+// The step of the levels below kVecMinRows rows (and of any level whose
+// neighbours do not fit int16 offsets, IDX), after k_bnd_exact: a thread per
+// row, the whole row of up to KC slots in registers before the wait,
+// 128-thread CTAs (twice the CTAs to spread over the SMs).
+template <int MODE, class T, int KC, bool IDX>
+__global__ void __launch_bounds__(128) k_level_c1(const __grid_constant__ StepArgsL<T> a)
+{
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = min(i0, a.n - 1);
+    RowChunk<T, KC, IDX> R;
+    R.fetch(a.gi, a.A, a.ld, i, i, 0);
+    const T di = ldk(a.dinv + i);
+    const int tg = ldk(a.tag + i);
+    pdl_wait<true>();
+    const T ri = __ldcg(a.r + i), ei = __ldcg(a.e + i);
+    T dprev = T(0);
+    if (MODE == 0 && !a.first) dprev = __ldcg(a.d + i);
+    T s = R.template dot<true>(a.e, T(0));
+    s = row_rest<true, T, KC, IDX>(a.gi, a.A, a.e, a.ld, a.kp, i, i, s);
+    if (i0 >= a.n) return;
+    if (tg == 1) {
+        a.out[i] = MODE == 0 ? ei : T(0);
+        return;
+    }
+    step_out<MODE>(a, i, ri, ei, dprev, di, s);
 }
 
 // the four weights of rows i0..i0+3 in slot o (evict-first)
@@ -283,21 +455,31 @@ __device__ __forceinline__ void load4(const double *A, long o, double (&a)[4])
     a[0] = v0.x; a[1] = v0.y; a[2] = v1.x; a[3] = v1.y;
 }
 
-// FP32: 4 CTAs of 256 per SM (64 registers); FP64: 3 (twice the weight registers)
+// FP32: 4 CTAs of 256 per SM (64 registers); FP64: 3 (twice the weight
+// registers).  The first slots' operator loads are issued before the wait for
+// the predecessor, so that they fill its tail.
 template <int MODE, class T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) k_level_v4(
-    int n, int ld, int k, const short *__restrict__ off, const T *__restrict__ A, const T *__restrict__ dinv,
-    const uint8_t *__restrict__ btag, const T *__restrict__ r, const T *__restrict__ e, T *__restrict__ out,
-    T *__restrict__ d, T c1, T c2, int first)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) k_level_v4(const __grid_constant__ StepArgsL<T> g)
 {
-    pdl_enter();
-    const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (i0 >= n) return;
+    const int b = blockIdx.x;
+    if (b >= g.fb && b < g.fb + g.nbc) {
+        step_bnd_part<MODE, T>(g, b - g.fb);
+        return;
+    }
+    if (b >= g.nfar + g.nbc) {
+        step_near_part<MODE, T>(g, b - g.nfar - g.nbc);
+        return;
+    }
+    const int n = g.n, ld = g.ld, k = g.k;
+    const T *__restrict__ A = g.A;
+    const short *__restrict__ off = static_cast<const short *>(g.gi);
+    const T *__restrict__ e = g.e;
+    const int i0 = ((b < g.fb ? b : b - g.nbc) * blockDim.x + threadIdx.x) * 4;
+    const bool live = i0 < n;
     T s[4] = {T(0), T(0), T(0), T(0)};
-    int j = 0;
-    for (; j + 4 <= k; j += 4) {
-        T a[4][4];
-        int c[4][4];
+    T a[4][4];
+    int c[4][4];
+    auto fetch = [&](int j) {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const long o = (long)(j + q) * ld + i0;
@@ -308,22 +490,38 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) k_level_v4(
             c[q][2] = i0 + 2 + (int)(short)(ov.y & 0xffffu);
             c[q][3] = i0 + 3 + (int)(short)(ov.y >> 16);
         }
+    };
+    auto use = [&] {
         // padding rows (i >= n) carry weight 0 and offset 0: clamp their gathers into the vector
 #pragma unroll
         for (int q = 0; q < 4; q++)
 #pragma unroll
-            for (int v = 0; v < 4; v++) s[v] += a[q][v] * __ldg(e + min(c[q][v], n - 1));
+            for (int v = 0; v < 4; v++) s[v] = fma_rn(a[q][v], __ldg(e + min(c[q][v], n - 1)), s[v]);
+    };
+    if (live && k >= 4) fetch(0);
+    pdl_wait<false>();
+    if (!live) return;
+    int j = 0;
+    if (k >= 4) {
+        use();
+        for (j = 4; j + 4 <= k; j += 4) {
+            fetch(j);
+            use();
+        }
     }
     for (; j < k; j++) {
 #pragma unroll
         for (int v = 0; v < 4; v++) {
             const long o = (long)j * ld + i0 + v;
-            s[v] += __ldcs(A + o) * __ldg(e + min(i0 + v + (int)__ldcs(off + o), n - 1));
+            s[v] = fma_rn(__ldcs(A + o), __ldg(e + min(i0 + v + (int)__ldcs(off + o), n - 1)), s[v]);
         }
     }
 #pragma unroll
-    for (int v = 0; v < 4; v++)
-        if (i0 + v < n) level_row_out<MODE, T>(i0 + v, s[v], dinv, btag, r, e, out, d, c1, c2, first);
+    for (int v = 0; v < 4; v++) {
+        const int i = i0 + v;
+        if (i >= n || __ldg(g.tag + i) != 0) continue;
+        step_out<MODE>(g, i, g.r[i], MODE == 0 ? e[i] : T(0), MODE == 0 && !g.first ? g.d[i] : T(0), g.dinv[i], s[v]);
+    }
 }
 
 // k_level_h4: k_level_v4 on the FP16 operator W ~ D^-1 A, four rows per
@@ -417,23 +615,43 @@ __global__ void __launch_bounds__(256, 4) k_level_h4(int n, int ld, int k, const
     }
 }
 
-template <int MODE, class T>
-static void launch_compact(const SolveLevel<T> &L, const T *e, T *out, T c1, T c2, int first, cudaStream_t s,
-                           Chain &launch)
+template <class T>
+static StepArgsL<T> step_args_of(const SolveLevel<T> &L, T *e, T *out, T c1, T c2, int first)
 {
-    if constexpr (sizeof(T) == 4) {
-        if (L.W16) {
-            launch(k_level_h4<MODE>, blocks_for(L.ldi / 4, 256), 256, 0, s, L.n, L.ldi, L.k, L.W16, L.dinv, L.btag,
-                     L.r, e, out, L.d, c1, c2, first);
-            return;
-        }
-    }
-    if (L.n >= kVecMinRows)
-        launch(k_level_v4<MODE, T>, blocks_for((L.n + 3) / 4, 256), 256, 0, s, L.n, L.ld, L.k, L.off, L.A, L.dinv,
-               L.btag, L.r, e, out, L.d, c1, c2, first);
+    StepArgsL<T> a{};
+    a.n = L.n; a.ld = L.ld; a.k = L.k; a.kp = (L.k + 7) & ~7; a.nbl = L.nb_list; a.nn = L.nn; a.ldn = L.ldn;
+    a.gi = L.off ? (const void *)L.off : (const void *)L.idx;
+    a.A = L.A; a.dinv = L.dinv; a.tag = L.tag;
+    a.r = L.r; a.e = e; a.out = out; a.d = L.d;
+    a.c1 = c1; a.c2 = c2; a.first = first;
+    a.bnd_list = L.bnd_list; a.bnd_idx = L.bnd_idx; a.bnd_A = L.bnd_A;
+    a.near_list = L.near_list; a.near_idx = L.near_idx; a.near_A = L.near_A;
+    a.sync = L.sync; a.err = L.tma_err;
+    return a;
+}
+
+template <class T>
+static void launch_bnd(const SolveLevel<T> &L, T *e, cudaStream_t s, Chain &launch)
+{
+    const int nbb = blocks_for((long)L.nb_list * 32, 256);
+    if (nbb == 0) return;
+    if (L.n < kVecMinRows)
+        launch(k_bnd_exact<T, true>, nbb, 256, 0, s, L.nb_list, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv, L.r, e);
     else
-        launch(k_level_c1<MODE, T>, blocks_for(L.n, 256), 256, 0, s, L.n, L.ld, L.k, L.off, L.A, L.dinv, L.btag,
-               L.r, e, out, L.d, c1, c2, first);
+        launch(k_bnd_exact<T, false>, nbb, 256, 0, s, L.nb_list, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv, L.r, e);
+}
+
+// the one-row-per-thread step: the smallest chunk that holds the row, so that
+// the whole row is fetched before the wait (the rest of a wider row after it)
+template <int MODE, class T, bool IDX>
+static void launch_c1(const SolveLevel<T> &L, T *e, T *out, T c1, T c2, int first, cudaStream_t s, Chain &launch)
+{
+    const StepArgsL<T> a = step_args_of(L, e, out, c1, c2, first);
+    const int grid = blocks_for(L.n, 128);
+    if (a.kp <= 16) launch(k_level_c1<MODE, T, 8, IDX>, grid, 128, 0, s, a);
+    else if (a.kp <= 24) launch(k_level_c1<MODE, T, 24, IDX>, grid, 128, 0, s, a);
+    else if (a.kp <= 32 || sizeof(T) == 8) launch(k_level_c1<MODE, T, 32, IDX>, grid, 128, 0, s, a);
+    else launch(k_level_c1<MODE, T, 40, IDX>, grid, 128, 0, s, a);
 }
 
 template <class T, bool COHERENT = false>
@@ -464,33 +682,144 @@ __device__ __forceinline__ void prolong_row(int i, int n, int k, const short *__
     ef[i] = ldv<COHERENT>(ef + i) + (ell_row_dot_o<T, T, COHERENT>(off, pw, ec, n, k, i, base[i]) - shift);
 }
 
+// Restriction into a level: r_c[i] = sum_j Rw[j][i] q_f[...] on interior rows
+// but row 0, 0 elsewhere.  FIRST (every level but the coarsest): the first
+// smoothing step of the pass from e = 0 with it (k_first_step): the boundary
+// rows' right-hand side is 0 there, so their e is 0 and d = c2 D^-1 r_c,
+// e = d on every interior row.  EARLY: rows padded to a multiple of 8 slots,
+// KC of them fetched before the wait.
 template <class T>
-__global__ void __launch_bounds__(256) k_restrict_o(int n, int k, const short *__restrict__ off,
-                                                    const int *__restrict__ base, const T *__restrict__ rw,
-                                                    const uint8_t *__restrict__ btag, const T *__restrict__ qf,
-                                                    T *__restrict__ rc)
+struct TransferArgs {
+    int n, k, kp;
+    const void *gi;        // int16 offsets from base[i], or 32-bit indices, [k][n]
+    const int *base;
+    const T *w;
+    const uint8_t *btag;
+    const T *in;
+    T *out;                // restriction: r_c; prolongation: e_f
+    const T *dinv;
+    T *d, *e;
+    T c2;
+};
+
+template <class T, int KC, bool IDX, bool EARLY>
+struct TransferRow {
+    RowChunk<T, KC, IDX> R;
+    int base = 0;
+    __device__ __forceinline__ void fetch(const TransferArgs<T> &a, int i)
+    {
+        if constexpr (!IDX) base = ldk(a.base + i);
+        if (EARLY || a.k >= KC) R.fetch(a.gi, a.w, a.n, i, base, 0);
+    }
+    __device__ __forceinline__ T dot(const TransferArgs<T> &a, int i)
+    {
+        if constexpr (EARLY) {
+            const T s = R.template dot<true>(a.in, T(0));
+            return row_rest<true, T, KC, IDX>(a.gi, a.w, a.in, a.n, a.kp, i, base, s);
+        } else {
+            static_assert(KC == 8, "row_big takes chunks of 8");
+            return row_big<T, IDX>(R, a.gi, a.w, a.in, a.n, a.k, i, base);
+        }
+    }
+};
+
+template <class T, int KC, bool IDX, bool EARLY, bool FIRST>
+__global__ void __launch_bounds__(128) k_restrict(const __grid_constant__ TransferArgs<T> a)
 {
-    pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    restrict_row(i, n, k, off, base, rw, btag, qf, rc);
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = min(i0, a.n - 1);
+    const bool inner = !ldk(a.btag + i);
+    TransferRow<T, KC, IDX, EARLY> R;
+    R.fetch(a, i);
+    T di = T(0);
+    if (FIRST) di = ldk(a.dinv + i);
+    pdl_wait<EARLY>();
+    T s = R.dot(a, i);
+    if (i0 >= a.n) return;
+    if (!inner || i == 0) s = T(0);
+    a.out[i] = s;
+    if (FIRST) {
+        if (!inner) {
+            a.e[i] = s * di;
+        } else {
+            const T dv = a.c2 * di * s;
+            a.d[i] = dv;
+            a.e[i] = T(0) + dv;
+        }
+    }
+}
+
+// Prolongation: e_f[i] += (P e_c)[i] - (P e_c)[0] (the shift keeps the pinned
+// node uncorrected).  Warp 0 sums row 0 while the other warps sum their rows.
+template <class T, int KC, bool IDX, bool EARLY, int BS>
+__global__ void __launch_bounds__(BS) k_prolong(const __grid_constant__ TransferArgs<T> a)
+{
+    __shared__ T shift;
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = min(i0, a.n - 1);
+    TransferRow<T, KC, IDX, EARLY> R;
+    R.fetch(a, i);
+    // row 0's slots, one per lane of warp 0 (the first 32 before the wait)
+    RowChunk<T, 1, IDX> R0;
+    int b0 = 0;
+    const int lane0 = min((int)threadIdx.x, a.k - 1);
+    if (threadIdx.x < 32) {
+        if constexpr (!IDX) b0 = ldk(a.base);
+        R0.fetch(a.gi, a.w, a.n, 0, b0, lane0);
+    }
+    pdl_wait<EARLY>();
+    if (threadIdx.x < 32) {
+        const T s0 = row0_dot_warp<T>(a.k, [&](int j, T &w, T &x) {
+            if (j >= 32) R0.fetch(a.gi, a.w, a.n, 0, b0, j);
+            w = R0.a[0];
+            x = __ldcg(a.in + R0.c[0]);
+        });
+        if (threadIdx.x == 0) shift = s0;
+    }
+    const T ei = __ldcg(a.out + i);
+    const T s = R.dot(a, i);
+    __syncthreads();
+    if (i0 < a.n) a.out[i] = ei + (s - shift);
+}
+
+template <class T, bool IDX, bool FIRST>
+static void launch_restrict_k(const TransferArgs<T> &a, cudaStream_t s, Chain &launch)
+{
+    const int grid = blocks_for(a.n, 128);
+    if (a.n >= kVecMinRows) launch(k_restrict<T, 8, IDX, false, FIRST>, grid, 128, 0, s, a);
+    else if (a.kp <= 16) launch(k_restrict<T, 8, IDX, true, FIRST>, grid, 128, 0, s, a);
+    else if (a.kp <= 24) launch(k_restrict<T, 24, IDX, true, FIRST>, grid, 128, 0, s, a);
+    else launch(k_restrict<T, 32, IDX, true, FIRST>, grid, 128, 0, s, a);
+}
+
+template <class T, bool FIRST>
+static void launch_restrict(const SolveLevel<T> &C, const T *qf, T c2, cudaStream_t s, Chain &launch)
+{
+    TransferArgs<T> a{};
+    a.n = C.n; a.k = C.kr; a.kp = (C.kr + 7) & ~7; a.base = C.r_base; a.w = C.r_w; a.btag = C.btag; a.in = qf;
+    a.out = C.r; a.dinv = C.dinv; a.d = C.d; a.e = C.e; a.c2 = c2;
+    a.gi = C.r_off ? (const void *)C.r_off : (const void *)C.r_idx;
+    if (C.r_off) launch_restrict_k<T, false, FIRST>(a, s, launch);
+    else launch_restrict_k<T, true, FIRST>(a, s, launch);
+}
+
+template <class T, bool IDX>
+static void launch_prolong_k(const TransferArgs<T> &a, cudaStream_t s, Chain &launch)
+{
+    if (a.n >= kVecMinRows) launch(k_prolong<T, 8, IDX, false, 256>, blocks_for(a.n, 256), 256, 0, s, a);
+    else if (a.kp <= 16) launch(k_prolong<T, 8, IDX, true, 128>, blocks_for(a.n, 128), 128, 0, s, a);
+    else if (a.kp <= 24) launch(k_prolong<T, 24, IDX, true, 128>, blocks_for(a.n, 128), 128, 0, s, a);
+    else launch(k_prolong<T, 32, IDX, true, 128>, blocks_for(a.n, 128), 128, 0, s, a);
 }
 
 template <class T>
-__global__ void __launch_bounds__(256) k_prolong_o(int n, int k, const short *__restrict__ off,
-                                                   const int *__restrict__ base, const T *__restrict__ pw,
-                                                   const T *__restrict__ ec, T *__restrict__ ef)
+static void launch_prolong(const SolveLevel<T> &L, const T *ec, cudaStream_t s, Chain &launch)
 {
-    pdl_enter();
-    __shared__ T shift;
-    if (threadIdx.x < 32) {
-        const T s = prolong_shift_warp(n, k, off, base, pw, ec);
-        if (threadIdx.x == 0) shift = s;
-    }
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    prolong_row(i, n, k, off, base, pw, ec, ef, shift);
+    TransferArgs<T> a{};
+    a.n = L.n; a.k = L.kp; a.kp = (L.kp + 7) & ~7; a.base = L.p_base; a.w = L.p_w; a.in = ec; a.out = L.e;
+    a.gi = L.p_off ? (const void *)L.p_off : (const void *)L.p_idx;
+    if (L.p_off) launch_prolong_k<T, false>(a, s, launch);
+    else launch_prolong_k<T, true>(a, s, launch);
 }
 
 // ---------------------------------------------------------------------------
@@ -801,14 +1130,28 @@ __device__ __forceinline__ void dense_row_warp(int w, int lane, int n, const T *
     if (lane == 0) e[w] = s;
 }
 
+// The first 1024 columns' operands are fetched before the wait.
 template <class T>
-__global__ void __launch_bounds__(256) k_dense_solve(int n, const T *__restrict__ inv, const T *__restrict__ r,
-                                                     T *__restrict__ e)
+__global__ void __launch_bounds__(256) k_dense_solve(int n, const T *__restrict__ inv, const T *r, T *e)
 {
-    pdl_enter();
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    dense_row_warp(warp, lane, n, inv, r, e);
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const T *row = inv + (long)w * n;
+    constexpr int Q = 32;
+    T a[Q];
+    if (w < n) {
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            if (lane + 32 * q < n) a[q] = ldk(row + lane + 32 * q);
+    }
+    pdl_wait<true>();
+    if (w >= n) return;
+    T s = T(0);
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+        if (lane + 32 * q < n) s = fma_rn(a[q], __ldcg(r + lane + 32 * q), s);
+    for (int j = lane + 32 * Q; j < n; j += 32) s = fma_rn(__ldg(row + j), __ldcg(r + j), s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) e[w] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -832,6 +1175,10 @@ struct FusedLevel {
     const uint8_t *btag;
     const int *bnd_list, *bnd_idx;
     const T *bnd_A;
+    const uint8_t *tag;   // near rows and their boundary slots (SolveLevel)
+    int nn, ldn, kb;
+    const int *near_list, *kb_idx;
+    const T *kb_a, *kb_d;
     T *r, *e, *e2, *d, *q;
     const short *r_off;   // restriction into this level (compact)
     const int *r_base;
@@ -899,26 +1246,54 @@ __global__ void __launch_bounds__(kFusedThreads) k_coarse_vcycle(const __grid_co
 #define MGM_SYNC() \
     if (!grid_barrier(a.bar, a.err, gen)) return
     T *cur[kFusedMaxLevels], *nxt[kFusedMaxLevels];
+    auto bnd = [&](int l) -> bool {
+        const FusedLevel<T> &L = a.L[l];
+        for (int w = wid; w < L.nb_list; w += nwarp) {
+            BndRow<T> B;
+            B.fetch(w, lane, L.nb_list, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv);
+            const T v = B.value(lane, L.k, L.bnd_idx, L.bnd_A, L.r, cur[l]);
+            if (lane == 0) cur[l][B.i] = v;
+        }
+        return grid_barrier(a.bar, a.err, gen);
+    };
+    auto pass = [&](int l, int mode, T c1, T c2, int first, T *out) -> bool {
+        const FusedLevel<T> &L = a.L[l];
+        StepArgsL<T> g{};
+        g.out = out; g.d = L.d; g.c1 = c1; g.c2 = c2; g.first = first;
+        const T *e = cur[l];
+        for (int i = tid; i < L.n; i += nth) {
+            const T ei = __ldcg(e + i);
+            if (L.btag[i]) {
+                out[i] = mode == 0 ? ei : T(0);
+                continue;
+            }
+            const T s = ell_row_dot_o<T, T, true>(L.off, L.A, e, L.ld, L.k, i, i);
+            const T ri = __ldcg(L.r + i), dprev = mode == 0 && !first ? __ldcg(L.d + i) : T(0);
+            if (mode == 0) step_out<0>(g, i, ri, ei, dprev, L.dinv[i], s);
+            else step_out<1>(g, i, ri, ei, dprev, L.dinv[i], s);
+        }
+        return grid_barrier(a.bar, a.err, gen);
+    };
     // one smoothing pass on level l: deg Chebyshev steps, each followed by
-    // the boundary rows' exact solve; from e = 0 or from the current e
+    // the boundary rows' exact solve; from e = 0 (the first step by first_row
+    // and first_near) or from the current e
     auto smooth = [&](int l, bool zero_start) -> bool {
         const FusedLevel<T> &L = a.L[l];
-        if (zero_start) {
-            for (int i = tid; i < L.n; i += nth) start_row<T, true>(i, L.btag, L.dinv, L.r, cur[l]);
-        } else {
-            for (int w = wid; w < L.nb_list; w += nwarp)
-                bnd_row_warp<T, true>(w, lane, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv, L.r, cur[l]);
-        }
-        if (!grid_barrier(a.bar, a.err, gen)) return false;
+        if (!zero_start && !bnd(l)) return false;
         for (int st = 0; st < a.deg; st++) {
-            for (int i = tid; i < L.n; i += nth)
-                c1_row<0, T, true>(i, L.ld, L.k, L.off, L.A, L.dinv, L.btag, L.r, cur[l], nxt[l], L.d, L.c1[st],
-                                   L.c2[st], st == 0 ? 1 : 0);
-            if (!grid_barrier(a.bar, a.err, gen)) return false;
+            if (st == 0 && zero_start) {
+                FirstArgs<T> f{};
+                f.n = L.n; f.nn = L.nn; f.kb = L.kb; f.ldn = L.ldn; f.tag = L.tag; f.dinv = L.dinv;
+                f.r = L.r; f.out = nxt[l]; f.d = L.d; f.c2 = L.c2[0]; f.near_list = L.near_list;
+                f.kb_idx = L.kb_idx; f.kb_a = L.kb_a; f.kb_d = L.kb_d;
+                for (int i = tid; i < L.n; i += nth) first_row<T, false>(f, i, L.tag[i], L.dinv[i]);
+                for (int t = tid; t < L.nn; t += nth) first_near<T, false>(f, t);
+                if (!grid_barrier(a.bar, a.err, gen)) return false;
+            } else if (!pass(l, 0, L.c1[st], L.c2[st], st == 0 ? 1 : 0, nxt[l])) {
+                return false;
+            }
             T *t = cur[l]; cur[l] = nxt[l]; nxt[l] = t;
-            for (int w = wid; w < L.nb_list; w += nwarp)
-                bnd_row_warp<T, true>(w, lane, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv, L.r, cur[l]);
-            if (!grid_barrier(a.bar, a.err, gen)) return false;
+            if (!bnd(l)) return false;
         }
         return true;
     };
@@ -926,9 +1301,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_coarse_vcycle(const __grid_co
     for (int l = a.first; l < a.nl - 1; l++) {
         const FusedLevel<T> &L = a.L[l], &C = a.L[l + 1];
         if (!smooth(l, true)) return;
-        for (int i = tid; i < L.n; i += nth)
-            c1_row<1, T, true>(i, L.ld, L.k, L.off, L.A, L.dinv, L.btag, L.r, cur[l], L.q, L.d, T(0), T(0), 0);
-        MGM_SYNC();
+        if (!pass(l, 1, T(0), T(0), 0, L.q)) return;
         for (int i = tid; i < C.n; i += nth)
             restrict_row<T, true>(i, C.n, C.kr, C.r_off, C.r_base, C.r_w, C.btag, L.q, C.r);
         MGM_SYNC();
@@ -988,6 +1361,8 @@ static void launch_fused(std::vector<SolveLevel<T>> &Ls, const CoarseSolve<T> &c
         F.n = S.n; F.ld = S.ld; F.k = S.k; F.nb_list = S.nb_list; F.kr = S.kr; F.kp = S.kp;
         F.off = S.off; F.A = S.A; F.dinv = S.dinv; F.btag = S.btag;
         F.bnd_list = S.bnd_list; F.bnd_idx = S.bnd_idx; F.bnd_A = S.bnd_A;
+        F.tag = S.tag; F.nn = S.nn; F.ldn = S.ldn; F.kb = S.kb; F.near_list = S.near_list;
+        F.kb_idx = S.kb_idx; F.kb_a = S.kb_a; F.kb_d = S.kb_d;
         F.r = S.r; F.e = S.e; F.e2 = S.e2; F.d = S.d; F.q = S.q;
         F.r_off = S.r_off; F.r_base = S.r_base; F.r_w = S.r_w;
         F.p_off = S.p_off; F.p_base = S.p_base; F.p_w = S.p_w;
@@ -1112,61 +1487,139 @@ SmootherProfile::~SmootherProfile()
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
 }
 
-template <class T>
-static void smooth(SolveLevel<T> &L, int degree, double ratio, bool zero_start, cudaStream_t s,
-                   SmootherProfile *prof, Chain &launch)
-{
-    const double lM = 1.05 * L.lmax, lm = L.lmax / ratio;
-    const double th = 0.5 * (lM + lm), de = 0.5 * (lM - lm), sig = th / de;
-    double rho = 1.0 / sig;
-    const int nb = blocks_for(L.n, 256), nbb = blocks_for((long)L.nb_list * 32, 256);
-    if (zero_start)
-        launch(k_start_e<T>, nb, 256, 0, s, L.n, L.btag, L.dinv, L.r, L.e);
-    else
-        launch(k_bnd_exact<T>, nbb, 256, 0, s, L.nb_list, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv, L.r, L.e);
-    for (int step = 0; step < degree; step++) {
-        double c1 = 0, c2;
-        if (step == 0) c2 = 1.0 / th;
-        else {
+// step coefficients of the Chebyshev polynomial on [lmax / ratio, 1.05 lmax]
+struct ChebCoef {
+    double th, de, sig, rho;
+    ChebCoef(double lmax, double ratio)
+    {
+        const double lM = 1.05 * lmax, lm = lmax / ratio;
+        th = 0.5 * (lM + lm);
+        de = 0.5 * (lM - lm);
+        sig = th / de;
+        rho = 1.0 / sig;
+    }
+    void next(int step, double &c1, double &c2)
+    {
+        c1 = 0;
+        if (step == 0) {
+            c2 = 1.0 / th;
+        } else {
             const double rn = 1.0 / (2.0 * sig - rho);
             c1 = rn * rho;
             c2 = 2.0 * rn / de;
             rho = rn;
         }
+    }
+};
+
+// One step on a level (MODE 0 Chebyshev, MODE 1 residual) with the boundary
+// rows' exact solve before it, by the level's variant: the tile-streamed and
+// FP16 kernels take the boundary rows as a launch of their own.
+template <int MODE, class T>
+static void launch_step(const SolveLevel<T> &L, T *e, T *out, T c1, T c2, int first, cudaStream_t s, Chain &launch,
+                        SmootherProfile *prof)
+{
+    auto mark = [&] {
         if (prof) {
             prof->mark(s);
             launch.broken();
         }
-        bool done = false;
-        if constexpr (sizeof(T) == 4) {
-            if (L.At) {
-                launch_tiled<0>(L, L.e, L.e2, (float)c1, (float)c2, step == 0 ? 1 : 0, s, launch);
-                done = true;
-            }
+    };
+    if constexpr (sizeof(T) == 4) {
+        if (L.At || L.W16) {
+            launch_bnd(L, e, s, launch);
+            mark();
+            if (L.At)
+                launch_tiled<MODE>(L, e, out, (float)c1, (float)c2, first, s, launch);
+            else
+                launch(k_level_h4<MODE>, blocks_for(L.ldi / 4, 256), 256, 0, s, L.n, L.ldi, L.k, L.W16, L.dinv,
+                       L.btag, L.r, (const float *)e, out, L.d, c1, c2, first);
+            mark();
+            return;
         }
-        if (done) {
-        } else if (L.off) {
-            launch_compact<0, T>(L, L.e, L.e2, (T)c1, (T)c2, step == 0 ? 1 : 0, s, launch);
-        } else {
-            launch(k_cheb<T>, nb, 256, 0, s, L.n, L.ld, L.k, L.idx, L.A, L.dinv, L.btag, L.r, L.e, L.e2, L.d, (T)c1,
-                   (T)c2, step == 0 ? 1 : 0);
-        }
-        if (prof) {
-            prof->mark(s);
-            launch.broken();
-        }
+    }
+    const bool big = L.off && L.n >= kVecMinRows;
+    if (!big) launch_bnd(L, e, s, launch);
+    mark();
+    if (big) {
+        StepArgsL<T> a = step_args_of(L, e, out, c1, c2, first);
+        a.nbc = blocks_for((long)L.nb_list * 32, 256);
+        a.nfar = blocks_for(L.n, 1024);
+        a.nnc = blocks_for(L.nn, 256);
+        // more far CTAs than the chip holds at once: the boundary part goes
+        // in the middle, where it fills freed slots; else after them
+        a.fb = a.nfar > 148 * 4 ? a.nfar / 2 : a.nfar;
+        launch(k_level_v4<MODE, T>, a.nbc + a.nfar + a.nnc, 256, 0, s, a);
+    } else if (L.off) {
+        launch_c1<MODE, T, false>(L, e, out, c1, c2, first, s, launch);
+    } else {
+        launch_c1<MODE, T, true>(L, e, out, c1, c2, first, s, launch);
+    }
+    mark();
+}
+
+// where the first smoothing step of level 0 takes its right-hand side from:
+// the FP64 Krylov vector V_j (V non-null), else the level's r
+struct FirstSrc {
+    const double *V = nullptr;
+    long ld = 0;
+    const FgState *st = nullptr;
+};
+
+// the first step of a pass from e = 0, into L.e2; then the buffers swap
+template <class T>
+static void first_step(SolveLevel<T> &L, double ratio, const FirstSrc &src, cudaStream_t s, Chain &launch)
+{
+    double c1, c2;
+    ChebCoef(L.lmax, ratio).next(0, c1, c2);
+    FirstArgs<T> a{};
+    a.n = L.n; a.nn = L.nn; a.kb = L.kb; a.ldn = L.ldn;
+    a.nrow = blocks_for(L.n, 256);
+    a.tag = L.tag; a.dinv = L.dinv; a.r = L.r; a.out = L.e2; a.d = L.d; a.c2 = (T)c2;
+    a.near_list = L.near_list; a.kb_idx = L.kb_idx; a.kb_a = L.kb_a; a.kb_d = L.kb_d;
+    a.V = src.V; a.ldv = src.ld; a.st = src.st;
+    const int grid = a.nrow + blocks_for(L.nn, 256);
+    const bool early = L.n < kVecMinRows;
+    if (src.V) {
+        if (early) launch(k_first_step<T, true, true>, grid, 256, 0, s, a);
+        else launch(k_first_step<T, true, false>, grid, 256, 0, s, a);
+    } else {
+        if (early) launch(k_first_step<T, false, true>, grid, 256, 0, s, a);
+        else launch(k_first_step<T, false, false>, grid, 256, 0, s, a);
+    }
+    std::swap(L.e, L.e2);
+}
+
+// Chebyshev steps from .. degree - 1 of a pass, each after the boundary rows'
+// exact solve from the current e; the pass's last boundary solve is the
+// caller's (the residual step does its own)
+template <class T>
+static void smooth_steps(SolveLevel<T> &L, int from, int degree, double ratio, cudaStream_t s, SmootherProfile *prof,
+                         Chain &launch)
+{
+    ChebCoef cc(L.lmax, ratio);
+    for (int step = 0; step < degree; step++) {
+        double c1, c2;
+        cc.next(step, c1, c2);
+        if (step < from) continue;
+        launch_step<0, T>(L, L.e, L.e2, (T)c1, (T)c2, step == 0 ? 1 : 0, s, launch, prof);
         std::swap(L.e, L.e2);
-        launch(k_bnd_exact<T>, nbb, 256, 0, s, L.nb_list, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv, L.r, L.e);
     }
 }
 
 template <class T>
 static void vcycle_rec(std::vector<SolveLevel<T>> &Ls, const CoarseSolve<T> &cs, int l, int deg, double ratio,
-                       cudaStream_t s, SmootherProfile *prof, Chain &launch, const FusedCtl *fused)
+                       cudaStream_t s, SmootherProfile *prof, Chain &launch, const FusedCtl *fused,
+                       const FirstSrc &src)
 {
     SmootherProfile *lp = (l == 0 && prof && prof->on) ? prof : nullptr;
     SolveLevel<T> &L = Ls[l];
     const int nl = (int)Ls.size();
+    if (l == 0 && (nl == 1 || (fused && fused->on && fusable(Ls, 0, deg))) && src.V) {
+        // level 0 itself is the fused or the dense level: r on its own
+        fg_load<T>(L.n, src.V, src.ld, src.st, L.r, s);
+        launch.broken();
+    }
     if (fused && fused->on && fusable(Ls, l, deg)) {
         // levels l..nl-1 in one cooperative launch; each level's correction
         // ends in its e buffer, as after the 2 deg swaps of the per-level path
@@ -1178,43 +1631,37 @@ static void vcycle_rec(std::vector<SolveLevel<T>> &Ls, const CoarseSolve<T> &cs,
         launch(k_dense_solve<T>, blocks_for((long)L.n * 32, 256), 256, 0, s, cs.n, cs.inv, L.r, L.e);
         return;
     }
-    smooth(L, deg, ratio, true, s, lp, launch);  // from e = 0
+    // from e = 0; below level 0 the restriction into the level did the first step (into e2)
+    if (l == 0) first_step(L, ratio, src, s, launch);
+    smooth_steps(L, 1, deg, ratio, s, lp, launch);
+    launch_step<1, T>(L, L.e, L.q, T(0), T(0), 0, s, launch, nullptr);
     SolveLevel<T> &C = Ls[l + 1];
-    bool tiled = false;
-    if constexpr (sizeof(T) == 4) {
-        if (L.At) {
-            launch_tiled<1>(L, L.e, L.q, 0.f, 0.f, 0, s, launch);
-            tiled = true;
-        }
-    }
-    if (tiled) {
-    } else if (L.off) {
-        launch_compact<1, T>(L, L.e, L.q, T(0), T(0), 0, s, launch);
+    if (l + 1 == nl - 1 || (fused && fused->on && fusable(Ls, l + 1, deg))) {
+        launch_restrict<T, false>(C, L.q, T(0), s, launch);
     } else {
-        launch(k_residual<T>, blocks_for(L.n, 256), 256, 0, s, L.n, L.ld, L.k, L.idx, L.A, L.btag, L.r, L.e, L.q);
+        double c1, c2;
+        ChebCoef(C.lmax, ratio).next(0, c1, c2);
+        std::swap(C.e, C.e2);
+        launch_restrict<T, true>(C, L.q, (T)c2, s, launch);
     }
-    if (C.r_off)
-        launch(k_restrict_o<T>, blocks_for(C.n, 256), 256, 0, s, C.n, C.kr, C.r_off, C.r_base, C.r_w, C.btag, L.q,
-               C.r);
-    else
-        launch(k_restrict<T>, blocks_for(C.n, 256), 256, 0, s, C.n, C.kr, C.r_idx, C.r_w, C.btag, L.q, C.r);
-    vcycle_rec(Ls, cs, l + 1, deg, ratio, s, prof, launch, fused);
-    if (L.p_off) {
-        launch(k_prolong_o<T>, blocks_for(L.n, 256), 256, 0, s, L.n, L.kp, L.p_off, L.p_base, L.p_w, (const T *)C.e,
-               L.e);
-    } else {
-        launch(k_prolong<T>, blocks_for(L.n, 256), 256, 0, s, L.n, L.kp, L.p_idx, L.p_w, (const T *)C.e, L.e);
-    }
-    smooth(L, deg, ratio, false, s, lp, launch);
+    vcycle_rec(Ls, cs, l + 1, deg, ratio, s, prof, launch, fused, src);
+    launch_prolong<T>(L, C.e, s, launch);
+    smooth_steps(L, 0, deg, ratio, s, lp, launch);
+    launch_bnd(L, L.e, s, launch);
 }
 
 template <class T>
 void vcycle(std::vector<SolveLevel<T>> &Ls, const CoarseSolve<T> &cs, int cheb_degree, double cheb_ratio,
-            cudaStream_t s, SmootherProfile *prof, bool chain, const FusedCtl *fused)
+            cudaStream_t s, SmootherProfile *prof, bool chain, const FusedCtl *fused, const double *V, long ldv,
+            const FgState *st)
 {
     Chain launch;
     launch.enabled = chain;
-    vcycle_rec(Ls, cs, 0, cheb_degree, cheb_ratio, s, prof, launch, fused);
+    FirstSrc src;
+    src.V = V;
+    src.ld = ldv;
+    src.st = st;
+    vcycle_rec(Ls, cs, 0, cheb_degree, cheb_ratio, s, prof, launch, fused, src);
 }
 
 // Chebyshev smoothing of A e = r on one level from e = 0 (r already in L.r);
@@ -1224,16 +1671,18 @@ const T *smooth_from_zero(SolveLevel<T> &L, int degree, double ratio, cudaStream
 {
     Chain launch;
     launch.enabled = chain;
-    smooth(L, degree, ratio, true, s, nullptr, launch);  // from e = 0
+    first_step(L, ratio, FirstSrc(), s, launch);
+    smooth_steps(L, 1, degree, ratio, s, (SmootherProfile *)nullptr, launch);
+    launch_bnd(L, L.e, s, launch);
     return L.e;
 }
 template const double *smooth_from_zero<double>(SolveLevel<double> &, int, double, cudaStream_t, bool);
 template const float *smooth_from_zero<float>(SolveLevel<float> &, int, double, cudaStream_t, bool);
 
 template void vcycle<double>(std::vector<SolveLevel<double>> &, const CoarseSolve<double> &, int, double, cudaStream_t,
-                             SmootherProfile *, bool, const FusedCtl *);
+                             SmootherProfile *, bool, const FusedCtl *, const double *, long, const FgState *);
 template void vcycle<float>(std::vector<SolveLevel<float>> &, const CoarseSolve<float> &, int, double, cudaStream_t,
-                            SmootherProfile *, bool, const FusedCtl *);
+                            SmootherProfile *, bool, const FusedCtl *, const double *, long, const FgState *);
 
 // ---------------------------------------------------------------------------
 // spectral radius of D^-1 A restricted to interior rows (power iteration)

@@ -6,6 +6,8 @@
 
 namespace mgm {
 
+struct FgState;  // krylov.cuh
+
 // level-0 state of one fractional step (device pointers; operators ELL [k][n])
 struct StepArgs {
     int n, k;
@@ -57,8 +59,8 @@ void ref_multigrid(std::vector<RefLevel> &Ls, double w1, double w2, int num_rela
 template <class T>
 struct SolveLevel {
     int n, k, nb_list;            // rows, stencil width, number of boundary rows
-    int ld;                       // leading dimension of idx, A and off (>= n; a multiple of 4 on FP32 levels)
-    const int *idx;               // ELL [k][ld]
+    int ld;                       // leading dimension of idx, A and off (>= n; a multiple of 4)
+    const int *idx;               // ELL [kp][ld], kp = k rounded up to 8 (padding slots: weight 0, the row itself)
     const T *A;                   // lap_Poison, row 0 replaced by the pin (A[0][0] = 1, rest 0)
     const T *dinv;                // 1 / diagonal
     const uint8_t *btag;
@@ -66,7 +68,7 @@ struct SolveLevel {
     const int *bnd_idx;           // their stencils, row-major [nb_list][k]
     const T *bnd_A;
     T *r, *e, *e2, *d, *q;        // rhs, correction (double-buffered), Chebyshev direction, residual
-    // restriction into this level (coarse row i <- fine interior residual), ELL [kf][n]
+    // restriction into this level (coarse row i <- fine interior residual), ELL [kf][n], slots padded like A's
     int kr;
     const int *r_idx;
     const T *r_w;
@@ -75,6 +77,16 @@ struct SolveLevel {
     const int *p_idx;
     const T *p_w;
     double lmax;                  // spectral radius estimate of D^-1 A on interior rows
+    // interior rows split by their neighbours: tag 0 far (no boundary
+    // neighbour), 1 boundary row, 2 near (at least one); the near rows'
+    // operator as its own ELL copy [k][ldn] with 32-bit indices in the slot
+    // order of A, and of it the boundary slots alone [kb][ldn] (neighbour,
+    // weight, the neighbour's 1 / diagonal; padded with weight 0)
+    const uint8_t *tag = nullptr;
+    int nn = 0, ldn = 0, kb = 0;
+    const int *near_list = nullptr, *near_idx = nullptr, *kb_idx = nullptr;
+    const T *near_A = nullptr, *kb_a = nullptr, *kb_d = nullptr;
+    unsigned *sync = nullptr;     // counters of the level step's boundary part (zero between launches)
     // compact indices (each used when non-null; A then holds each row's slots
     // sorted by neighbour index, [k][ld], ld a multiple of 4): neighbours as
     // int16 offsets c - i [k][ld]; transfer gathers as int16 offsets from a
@@ -88,7 +100,7 @@ struct SolveLevel {
     const float *At = nullptr;
     const short *offt = nullptr;
     int ldt = 0;
-    int *tma_err = nullptr;
+    int *tma_err = nullptr;       // set when a bounded device-side wait runs out
     // FP16 copy of the compact operator (levels of at least kVecMinRows rows;
     // used when non-null): D^-1 A with the row sum in the diagonal slot, one
     // uint4 {4 FP16 weights, 4 int16 offsets} per slot and thread, the
@@ -145,10 +157,14 @@ cudaError_t launch_barrier_selftest(cudaStream_t s, unsigned *bar, int *err);
 
 // chain: launch the kernels after the first with programmatic stream
 // serialisation (Chain in mgm_internal.cuh); fused (when on): the levels
-// below kVecMinRows rows run as one cooperative launch (k_coarse_vcycle)
+// below kVecMinRows rows run as one cooperative launch (k_coarse_vcycle).
+// V non-null: the right-hand side is the FP64 Krylov vector V + st->j_next * ldv,
+// converted into level 0's r by the cycle's first kernel; else level 0's r.
 template <class T>
 void vcycle(std::vector<SolveLevel<T>> &Ls, const CoarseSolve<T> &cs, int cheb_degree, double cheb_ratio,
-            cudaStream_t s, SmootherProfile *prof = nullptr, bool chain = false, const FusedCtl *fused = nullptr);
+            cudaStream_t s, SmootherProfile *prof = nullptr, bool chain = false, const FusedCtl *fused = nullptr,
+            const double *V = nullptr, long ldv = 0, const FgState *st = nullptr);
+// (L.idx, L.A: the operator in the level's own slot order, [k][n])
 template <class T>
 void estimate_lmax(SolveLevel<T> &L, cudaStream_t s);
 template <class T>
