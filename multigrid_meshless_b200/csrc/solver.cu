@@ -519,7 +519,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) k_level_v4(const 
 #pragma unroll
     for (int v = 0; v < 4; v++) {
         const int i = i0 + v;
-        if (i >= n || __ldg(g.tag + i) != 0) continue;
+        if (i >= n) continue;
+        const int tg = __ldg(g.tag + i);
+        if (g.nbc == 0 && tg == 1) g.out[i] = MODE == 0 ? e[i] : T(0);
+        if (tg == 1 || (tg == 2 && g.nbc)) continue;
         step_out<MODE>(g, i, g.r[i], MODE == 0 ? e[i] : T(0), MODE == 0 && !g.first ? g.d[i] : T(0), g.dinv[i], s[v]);
     }
 }
@@ -1539,16 +1542,25 @@ static void launch_step(const SolveLevel<T> &L, T *e, T *out, T c1, T c2, int fi
         }
     }
     const bool big = L.off && L.n >= kVecMinRows;
-    if (!big) launch_bnd(L, e, s, launch);
+    // One launch with the boundary part pays while that part is small beside
+    // the far part (the 500^2 cavity, 250 CTAs beside 245: 17.4 us against
+    // 16.0 + 4.2); in 3D it is not (the 64^3 cube, 2883 beside 245: 44 us
+    // against 19.6 + 6.3, the far part waits for slots).
+    const int nbc = blocks_for((long)L.nb_list * 32, 256), nfar = blocks_for(L.n, 1024);
+    const bool one = big && nbc <= 2 * nfar;
+    if (!one) launch_bnd(L, e, s, launch);
     mark();
     if (big) {
         StepArgsL<T> a = step_args_of(L, e, out, c1, c2, first);
-        a.nbc = blocks_for((long)L.nb_list * 32, 256);
-        a.nfar = blocks_for(L.n, 1024);
-        a.nnc = blocks_for(L.nn, 256);
-        // more far CTAs than the chip holds at once: the boundary part goes
-        // in the middle, where it fills freed slots; else after them
-        a.fb = a.nfar > 148 * 4 ? a.nfar / 2 : a.nfar;
+        a.nfar = nfar;
+        a.fb = nfar;
+        if (one) {
+            a.nbc = nbc;
+            a.nnc = blocks_for(L.nn, 256);
+            // more far CTAs than the chip holds at once: the boundary part
+            // goes in the middle, where it fills freed slots; else after them
+            if (nfar > 148 * 4) a.fb = nfar / 2;
+        }
         launch(k_level_v4<MODE, T>, a.nbc + a.nfar + a.nnc, 256, 0, s, a);
     } else if (L.off) {
         launch_c1<MODE, T, false>(L, e, out, c1, c2, first, s, launch);
