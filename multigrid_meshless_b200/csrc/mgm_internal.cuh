@@ -162,6 +162,16 @@ void transfer_weights(int nt, const double *tx, const double *ty, const double *
                       const Monomials &mono, const double *sx, const double *sy, const double *sz,
                       const int *scloud_rowmajor, double *W, cudaStream_t s);
 
+// the same with the systems in registers (weights_reg.cu); false: the order is too large
+bool derivative_weights_reg(int n, int k, int dim, int phs, const Monomials &mono, const double *x, const double *y,
+                            const double *z, const double *nx, const double *ny, const double *nz,
+                            const uint8_t *btag, const int *cloud, double *Dx, double *Dy, double *Dz, double *lap,
+                            double *lapP, cudaStream_t s);
+bool transfer_weights_reg(int nt, const double *tx, const double *ty, const double *tz, const uint8_t *tbtag,
+                          const int *src_pt, int rows_from, int only_interior, int ks, int dim, int phs,
+                          const Monomials &mono, const double *sx, const double *sy, const double *sz,
+                          const int *scloud, double *W, cudaStream_t s);
+
 // layout helpers
 void transpose_rowmajor_to_ell_d(const double *in, double *out, int n, int k, cudaStream_t s);
 void transpose_rowmajor_to_ell_i(const int *in, int *out, int n, int k, cudaStream_t s);

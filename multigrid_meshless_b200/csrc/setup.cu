@@ -548,6 +548,7 @@ void derivative_weights(int n, int k, int dim, int phs, const Monomials &mono, c
 {
     MGM_REQUIRE(k >= 2 && k <= kMaxK && k + mono.np <= kMaxN, "weights: stencil too large");
     if (n <= 0) return;
+    if (derivative_weights_reg(n, k, dim, phs, mono, x, y, z, nx, ny, nz, btag, cloud, Dx, Dy, Dz, lap, lapP, s)) return;
     size_t smem = weights_smem(k, mono.np);
     MGM_REQUIRE(smem <= 227 * 1024, "weights: system does not fit in shared memory");
     MGM_CUDA(cudaFuncSetAttribute(k_derivative_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -600,6 +601,9 @@ void transfer_weights(int nt, const double *tx, const double *ty, const double *
 {
     MGM_REQUIRE(ks >= 2 && ks <= kMaxK && ks + mono.np <= kMaxN, "transfer weights: stencil too large");
     if (nt <= 0) return;
+    if (transfer_weights_reg(nt, tx, ty, tz, tbtag, src_pt, rows_from, only_interior, ks, dim, phs, mono, sx, sy, sz,
+                             scloud, W, s))
+        return;
     const int N = ks + mono.np;
     size_t smem = sizeof(double) * ((size_t)N * 2 * N + 3 * ks + 2 * N) + sizeof(int) * N;
     MGM_REQUIRE(smem <= 227 * 1024, "transfer weights: system does not fit in shared memory");
