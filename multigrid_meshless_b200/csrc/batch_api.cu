@@ -29,6 +29,7 @@ void check_batch(mgm_batch *b)
 {
     MGM_REQUIRE(b != nullptr, "null batch context");
     MGM_CUDA(cudaSetDevice(b->device));
+    alloc_stream(b->s);
 }
 
 BLevel &level_of(mgm_batch *b, int lev)
@@ -74,12 +75,14 @@ void mgm_batch_destroy(mgm_batch *b)
     if (!b) return;
     cudaSetDevice(b->device);
     if (b->s) cudaStreamSynchronize(b->s);
+    alloc_stream(nullptr);
     batch_free_solver(b);
     if (b->h_pinned) cudaFreeHost(b->h_pinned);
     for (cudaEvent_t e : b->ev) if (e) cudaEventDestroy(e);
     cudaStream_t s = b->s;
     delete b;
     if (s) cudaStreamDestroy(s);
+    trim_memory();
 }
 
 int mgm_batch_set_level(mgm_batch *b, int lev, int n, int nb, const double *x, const double *y, const double *z,

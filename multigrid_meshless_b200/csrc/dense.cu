@@ -80,6 +80,7 @@ int mgm_gauss_jordan(int order, const double *A, double *inverse)
         const size_t nn = (size_t)order * order;
         cudaStream_t s = nullptr;
         MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        const AllocScope scope(s);
         try {
             DBuf<double> dA(nn), aug(2 * nn), t(order), dinv(nn);
             DBuf<int> perm(order);
@@ -107,6 +108,7 @@ int mgm_laplacian_for_poisson(int n, int k, int dim, const double *Dx, const dou
         const size_t nk = (size_t)n * k;
         cudaStream_t s = nullptr;
         MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        const AllocScope scope(s);
         try {
             DBuf<double> dx(nk), dy(nk), dz(dim == 3 ? nk : 1), dl(nk), vx(n), vy(n), vz(n), out(nk);
             DBuf<unsigned char> bt(n);

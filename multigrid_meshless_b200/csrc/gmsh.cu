@@ -226,6 +226,7 @@ mgm_mesh *read_mesh(const char *path, int dim)
     {
         cudaStream_t s;
         MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        const AllocScope scope(s);
         try {
             DBuf<double> dx(nn), dy(nn), dz(nn), dnx(nn), dny(nn), dnz(nn);
             DBuf<int4> dev(std::max<size_t>(be.size(), 1));

@@ -156,6 +156,7 @@ int mgm_heat_init(mgm_ctx *c, int wave_number)
     return hguard([&] {
         MGM_REQUIRE(c != nullptr, "null context");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done, "mgm_heat_init: call mgm_setup first");
         MGM_REQUIRE(c->dim == 2, "mgm_heat_init: the heat-conduction program is two-dimensional");
         heat_init(c, wave_number);
@@ -167,6 +168,7 @@ int mgm_heat_step(mgm_ctx *c, double *steady_err)
     return hguard([&] {
         MGM_REQUIRE(c != nullptr, "null context");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done && c->heat_ready, "mgm_heat_step: call mgm_heat_init first");
         const double e = heat_step(c);
         if (steady_err) *steady_err = e;

@@ -200,6 +200,7 @@ int mgm_write_solution(mgm_ctx *c, const char *path, int pressure_field)
     return ioguard([&] {
         MGM_REQUIRE(c != nullptr && path != nullptr, "mgm_write_solution: null argument");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done, "mgm_write_solution: call mgm_setup first");
         MGM_CUDA(cudaStreamSynchronize(c->s));
         write_solution(c, path, pressure_field);
@@ -211,6 +212,7 @@ int mgm_checkpoint_save(mgm_ctx *c, const char *path)
     return ioguard([&] {
         MGM_REQUIRE(c != nullptr && path != nullptr, "mgm_checkpoint_save: null argument");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done, "mgm_checkpoint_save: call mgm_setup first");
         MGM_CUDA(cudaStreamSynchronize(c->s));
         save(c, path);
@@ -222,6 +224,7 @@ int mgm_checkpoint_load(mgm_ctx *c, const char *path)
     return ioguard([&] {
         MGM_REQUIRE(c != nullptr && path != nullptr, "mgm_checkpoint_load: null argument");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done, "mgm_checkpoint_load: call mgm_setup first");
         MGM_CUDA(cudaStreamSynchronize(c->s));
         load(c, path);

@@ -49,6 +49,7 @@ cudaStream_t tmp_stream()
 {
     static thread_local cudaStream_t s = nullptr;
     if (!s) MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    alloc_stream(s);
     return s;
 }
 
@@ -56,6 +57,7 @@ void check_ctx(mgm_ctx *c)
 {
     MGM_REQUIRE(c != nullptr, "null context");
     MGM_CUDA(cudaSetDevice(c->device));
+    alloc_stream(c->s);
 }
 
 __global__ void k_gather_idx(int n, int k, const int *__restrict__ pts, const int *__restrict__ src_cloud,
@@ -1384,6 +1386,7 @@ void mgm_destroy(mgm_ctx *c)
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->s) cudaStreamSynchronize(c->s);
+    alloc_stream(nullptr);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
     if (c->h_fg) cudaFreeHost(c->h_fg);
     drop_graphs(c);
@@ -1393,6 +1396,7 @@ void mgm_destroy(mgm_ctx *c)
         if (bs) cudaStreamDestroy(bs);
     if (c->s) cudaStreamDestroy(c->s);
     delete c;
+    trim_memory();
 }
 
 int mgm_set_level(mgm_ctx *c, int lev, int n, int nb, const double *x, const double *y, const double *z,
@@ -1687,6 +1691,7 @@ int mgm_setup(mgm_ctx *c, int flags)
         pipeline_transfer(c, c->have_ref_transfer);
         pipeline_derivatives(c);
         prepare_solver(c);
+        trim_memory();
     });
 }
 

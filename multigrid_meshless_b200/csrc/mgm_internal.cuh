@@ -80,6 +80,23 @@ __device__ __forceinline__ T ell_row_dot(const int *__restrict__ idx, const T *_
     return s;
 }
 
+// Device memory of the buffers (mem.cu): stream-ordered on the stream that the
+// running API call names for its thread (null: none, the object's work is done).
+void alloc_stream(cudaStream_t s);
+cudaStream_t alloc_stream();
+void *dev_alloc(size_t bytes);
+void dev_free(void *p) noexcept;
+void trim_memory() noexcept;  // gives back what the pool holds beyond its bound
+
+// names a stream for a scope
+struct AllocScope {
+    cudaStream_t before;
+    explicit AllocScope(cudaStream_t s) : before(alloc_stream()) { alloc_stream(s); }
+    ~AllocScope() { alloc_stream(before); }
+    AllocScope(const AllocScope &) = delete;
+    AllocScope &operator=(const AllocScope &) = delete;
+};
+
 // device buffer with RAII
 template <class T>
 struct DBuf {
@@ -97,13 +114,10 @@ struct DBuf {
     ~DBuf() { release(); }
     void alloc(size_t count) {
         release();
+        if (count) p = static_cast<T *>(dev_alloc(count * sizeof(T)));
         n = count;
-        if (count) {
-            cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-            if (e != cudaSuccess) { p = nullptr; n = 0; throw Error{5, std::string("cudaMalloc: ") + cudaGetErrorString(e)}; }
-        }
     }
-    void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
+    void release() { dev_free(p); p = nullptr; n = 0; }
     void zero(cudaStream_t s) { if (n) { cudaError_t e = cudaMemsetAsync(p, 0, n * sizeof(T), s); if (e != cudaSuccess) throw Error{1, cudaGetErrorString(e)}; } }
     void upload(const T *h, size_t count, cudaStream_t s) {
         if (count > n) alloc(count);

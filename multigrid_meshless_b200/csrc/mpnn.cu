@@ -820,6 +820,7 @@ static void init_params(std::vector<float> &P, unsigned long long seed)
 MpnnState &state(mgm_ctx *c)
 {
     MGM_REQUIRE(c->mpnn && c->mpnn->ready, "learned warm start not initialised (mgm_mpnn_init)");
+    alloc_stream(c->s);
     return *c->mpnn;
 }
 
@@ -902,6 +903,7 @@ int mgm_mpnn_init(mgm_ctx *c, unsigned long long seed, int dataset_capacity)
         MGM_REQUIRE(c && c->setup_done, "mgm_mpnn_init: call mgm_setup first");
         MGM_REQUIRE(dataset_capacity >= 0, "mgm_mpnn_init: negative capacity");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         cudaStream_t s = c->s;
         Level &L = c->L[0];
         MGM_REQUIRE(L.k <= 64, "mgm_mpnn_init: stencils wider than 64 are not supported by the network");

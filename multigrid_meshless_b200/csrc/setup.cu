@@ -53,18 +53,14 @@ __global__ void k_scan_total(const int *in, const int *out, int n, int *total)
 static void scan_rec(const int *d_in, int *d_out, int n, cudaStream_t s)
 {
     int nb = blocks_for(n, SCAN_TILE);
-    int *sums = nullptr, *sums_scan = nullptr;
-    MGM_CUDA(cudaMallocAsync(&sums, sizeof(int) * (size_t)std::max(nb, 1), s));
-    MGM_CUDA(cudaMallocAsync(&sums_scan, sizeof(int) * (size_t)std::max(nb, 1), s));
-    k_scan_tile<<<nb, SCAN_BS, 0, s>>>(d_in, d_out, n, sums);
+    DBuf<int> sums(std::max(nb, 1)), sums_scan(std::max(nb, 1));
+    k_scan_tile<<<nb, SCAN_BS, 0, s>>>(d_in, d_out, n, sums.p);
     MGM_LAUNCHED();
     if (nb > 1) {
-        scan_rec(sums, sums_scan, nb, s);
-        k_scan_add<<<blocks_for(n, 256), 256, 0, s>>>(d_out, n, sums_scan);
+        scan_rec(sums.p, sums_scan.p, nb, s);
+        k_scan_add<<<blocks_for(n, 256), 256, 0, s>>>(d_out, n, sums_scan.p);
         MGM_LAUNCHED();
     }
-    MGM_CUDA(cudaFreeAsync(sums, s));
-    MGM_CUDA(cudaFreeAsync(sums_scan, s));
 }
 
 void scan_exclusive(const int *d_in, int *d_out, int n, int *d_total, cudaStream_t s)

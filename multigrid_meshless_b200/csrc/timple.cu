@@ -381,6 +381,7 @@ int mgm_set_timple(mgm_ctx *c, int iter_timple, int iter_momentum, double facRe,
     return tguard([&] {
         MGM_REQUIRE(c != nullptr, "null context");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(iter_timple >= 1 && iter_momentum >= 1 && facdt > 0, "mgm_set_timple: bad parameters");
         c->iter_timple = iter_timple;
         c->iter_momentum = iter_momentum;
@@ -394,6 +395,7 @@ int mgm_timple_part(mgm_ctx *c, int part, int mode)
     return tguard([&] {
         MGM_REQUIRE(c != nullptr, "null context");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done && c->dt > 0, "mgm_timple_part: call mgm_setup and mgm_set_flow first");
         timple_part(c, part, mode);
     });
@@ -404,6 +406,7 @@ int mgm_timple_run(mgm_ctx *c, int mode, int nsteps, double *step_ms, long long 
     return tguard([&] {
         MGM_REQUIRE(c != nullptr, "null context");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done && c->dt > 0, "mgm_timple_run: call mgm_setup and mgm_set_flow first");
         MGM_REQUIRE(nsteps >= 0, "mgm_timple_run: nsteps < 0");
         cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -436,6 +439,7 @@ int mgm_timple_step(mgm_ctx *c, int mode, double *steady_err)
     return tguard([&] {
         MGM_REQUIRE(c != nullptr, "null context");
         MGM_CUDA(cudaSetDevice(c->device));
+        alloc_stream(c->s);
         MGM_REQUIRE(c->setup_done && c->dt > 0, "mgm_timple_step: call mgm_setup and mgm_set_flow first");
         const double e = timple_step(c, mode);
         if (steady_err) *steady_err = e;
