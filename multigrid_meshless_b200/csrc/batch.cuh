@@ -42,6 +42,7 @@ struct BLevel {
     DBuf<double> A64, dinv64;
     DBuf<float> A32, dinv32;
     DBuf<int> bnd_list;
+    DBuf<uint8_t> near;  // rows with boundary neighbours
     int nbl = 0;
     double lmax = 2.0;
     std::vector<int> h_kk;  // host copy of kk (task list)

@@ -11,12 +11,14 @@
 // every gathered neighbour is one contiguous B-wide access.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "batch.cuh"
 
 namespace mgm {
 
 constexpr int kBatchMaxRestart = 32;
+constexpr int kRowThreads = 768;  // most threads of a row kernel's CTA
 
 template <class T, int Q>
 __device__ __forceinline__ void ldq(const T *p, T (&v)[Q])
@@ -44,61 +46,101 @@ __device__ __forceinline__ void stq(T *p, const T (&v)[Q])
 }
 
 // acc[q] = sum_j A[beg + j] * x[col[beg + j]][lane*Q + q], j ascending.  The
-// row's indices and weights are loaded by the lanes 32 at a time and
-// broadcast; eight gathers are in flight per warp.
+// lanes load 32 (index, weight) pairs at a time, the next 32 ahead, and pass
+// them on through shared memory, where two FP32 pairs are one broadcast load:
+// the row kernels are bound by instruction issue and L1, and with two shuffles
+// and a predicate per slot an FP32 step of 107k rows x 64 columns took 17.8
+// instructions a slot.  Eight gathers are in flight per warp.  The last slots
+// are rounded up to four with weight 0 on the row's last index.
+template <class T>
+struct alignas(2 * sizeof(T)) SlotPair {
+    T a;
+    int c;
+};
+
 template <class T, int Q, class X>
 __device__ __forceinline__ void row_dot_b(const int *__restrict__ col, const T *__restrict__ A, int beg, int cnt,
-                                          const X *__restrict__ x, int B, int lane, T (&acc)[Q])
+                                          const X *__restrict__ x, int lane, T (&acc)[Q])
 {
+    __shared__ alignas(16) SlotPair<T> slots[kRowThreads / 32][32];
+    SlotPair<T> *const sl = slots[threadIdx.x >> 5];
+    const X *const xl = x + lane * Q;
 #pragma unroll
     for (int q = 0; q < Q; q++) acc[q] = T(0);
+    SlotPair<T> nx{T(0), 0};
+    if (cnt > 0) {
+        nx.c = __ldg(col + beg + min(lane, cnt - 1));
+        if (lane < cnt) nx.a = __ldg(A + beg + lane);
+    }
+    auto chunk = [&](int t, auto CH) {
+        constexpr int C = decltype(CH)::value;
+        SlotPair<T> p[C];
+        X xv[C][Q];
+        if constexpr (sizeof(T) == 4) {
+#pragma unroll
+            for (int u = 0; u < C; u += 2) {
+                const int4 v = *(const int4 *)(sl + t + u);
+                p[u] = {__int_as_float(v.x), v.y};
+                p[u + 1] = {__int_as_float(v.z), v.w};
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < C; u++) p[u] = sl[t + u];
+        }
+#pragma unroll
+        for (int u = 0; u < C; u++) ldgq<X, Q>(xl + (long)p[u].c * (32 * Q), xv[u]);
+#pragma unroll
+        for (int u = 0; u < C; u++)
+#pragma unroll
+            for (int q = 0; q < Q; q++) acc[q] += p[u].a * (T)xv[u][q];
+    };
     for (int j0 = 0; j0 < cnt; j0 += 32) {
-        const int jj = j0 + lane;
-        int c = 0;
-        T a = T(0);
-        if (jj < cnt) { c = __ldg(col + beg + jj); a = __ldg(A + beg + jj); }
+        __syncwarp();
+        sl[lane] = nx;
+        __syncwarp();
+        const int jn = j0 + 32 + lane;
+        nx.a = T(0);
+        if (j0 + 32 < cnt) {
+            nx.c = __ldg(col + beg + min(jn, cnt - 1));
+            if (jn < cnt) nx.a = __ldg(A + beg + jn);
+        }
         const int m = min(32, cnt - j0);
         int t = 0;
-        for (; t + 8 <= m; t += 8) {
-            int cc[8];
-            T aa[8];
-            X xv[8][Q];
-#pragma unroll
-            for (int u = 0; u < 8; u++) { cc[u] = __shfl_sync(0xffffffffu, c, t + u); aa[u] = __shfl_sync(0xffffffffu, a, t + u); }
-#pragma unroll
-            for (int u = 0; u < 8; u++) ldgq<X, Q>(x + (long)cc[u] * B + lane * Q, xv[u]);
-#pragma unroll
-            for (int u = 0; u < 8; u++)
-#pragma unroll
-                for (int q = 0; q < Q; q++) acc[q] += aa[u] * (T)xv[u][q];
-        }
-        for (; t < m; t++) {
-            const int ct = __shfl_sync(0xffffffffu, c, t);
-            const T at = __shfl_sync(0xffffffffu, a, t);
-            X xv[Q];
-            ldgq<X, Q>(x + (long)ct * B + lane * Q, xv);
-#pragma unroll
-            for (int q = 0; q < Q; q++) acc[q] += at * (T)xv[q];
-        }
+        for (; t + 4 < m; t += 8) chunk(t, std::integral_constant<int, 8>{});
+        if (t < m) chunk(t, std::integral_constant<int, 4>{});
     }
 }
 
-// Row-kernel shape: a CTA of 8 warps owns kRowsPerCta consecutive rows and
-// its warps step through them together (warp w: rows w, w + 8, ...).  In the
-// breadth-first order consecutive rows share most neighbours, so the gathered
-// neighbour rows of one CTA are served from L1 after their first use.
-constexpr int kRowsPerCta = 64;
-inline int rows_grid(long rows) { return blocks_for(rows, kRowsPerCta); }
+// Row-kernel shape: a CTA owns rpc consecutive rows, its warps step through
+// them together (warp w: rows w, w + warps, ...).  In the breadth-first order
+// consecutive rows share most neighbours, so a long run of rows per CTA has its
+// gathers served from L1: two CTAs of 24 warps per SM with all rows split among
+// them (FP32 step of 107k rows x 64 columns: 65% L1 hits, 80 us; 64 rows per
+// 8-warp CTA had 49%).  That needs about two rows per warp; below it, as for the
+// boundary rows, fewer warps per CTA and one or two rows per warp keep every SM
+// busy (3.6k boundary rows: 11 us, 17 as large CTAs).
+struct RowShape {
+    int grid, threads, rpc;
+};
+inline RowShape row_shape(long rows)
+{
+    if (rows >= 2L * 148 * 40) {
+        const int rpc = (int)((rows + 295) / 296);
+        return {blocks_for(rows, rpc), kRowThreads, rpc};
+    }
+    const int rpc = rows <= 8L * 148 * 5 ? 8 : 16;
+    return {blocks_for(rows, rpc), 256, rpc};
+}
 #define MGM_CTA_ROWS(r, count)                                                                     \
-    for (int r##_k = (int)(threadIdx.x >> 5), r = blockIdx.x * kRowsPerCta + r##_k;                \
-         r##_k < kRowsPerCta && r < (count); r##_k += 8, r += 8)
+    for (int r##_k = (int)(threadIdx.x >> 5), r = blockIdx.x * rpc + r##_k;                        \
+         r##_k < rpc && r < (count); r##_k += (int)(blockDim.x >> 5), r += (int)(blockDim.x >> 5))
 
 // exact solve of the boundary rows (they couple only to themselves and interior nodes)
 template <class T, int Q>
-__global__ void __launch_bounds__(256) k_b_bnd(int nbl, const int *__restrict__ list, const int *__restrict__ rp,
+__global__ void __launch_bounds__(kRowThreads, 2) k_b_bnd(int nbl, const int *__restrict__ list, const int *__restrict__ rp,
                                                const int *__restrict__ col, const T *__restrict__ A,
                                                const T *__restrict__ dinv, const T *__restrict__ r, T *e, int B,
-                                               int zero_start)
+                                               int rpc)
 {
     const int lane = threadIdx.x & 31;
     MGM_CTA_ROWS(w, nbl) {
@@ -107,27 +149,75 @@ __global__ void __launch_bounds__(256) k_b_bnd(int nbl, const int *__restrict__ 
         T rv[Q], ev[Q];
         ldq<T, Q>(r + o, rv);
         const T di = dinv[i];
-        if (zero_start) {
+        T acc[Q];
+        row_dot_b<T, Q, T>(col, A, rp[i], rp[i + 1] - rp[i], e, lane, acc);
+        ldq<T, Q>(e + o, ev);
+#pragma unroll
+        for (int q = 0; q < Q; q++) ev[q] = ev[q] + (rv[q] - acc[q]) * di;
+        stq<T, Q>(e + o, ev);
+    }
+}
+
+// The first step of a smoothing pass from e = 0 (interior 0, boundary rows
+// their exact solve r / a): rows without boundary neighbours (near 0) need no
+// operator, the others only their boundary neighbours' terms; the zero terms
+// left out change no bit of a sum.
+template <class T, int Q>
+__global__ void __launch_bounds__(kRowThreads, 2) k_b_first(int n, const int *__restrict__ rp, const int *__restrict__ col,
+                                                 const T *__restrict__ A, const T *__restrict__ dinv,
+                                                 const uint8_t *__restrict__ btag, const uint8_t *__restrict__ near,
+                                                 const T *__restrict__ r, T *__restrict__ eout, T *__restrict__ d,
+                                                 int B, T c2, int rpc)
+{
+    const int lane = threadIdx.x & 31;
+    MGM_CTA_ROWS(i, n) {
+        const long o = (long)i * B + lane * Q;
+        T rv[Q], ev[Q], dv[Q], acc[Q];
+        ldq<T, Q>(r + o, rv);
+        const T di = dinv[i];
+        if (btag[i]) {
 #pragma unroll
             for (int q = 0; q < Q; q++) ev[q] = rv[q] * di;
-        } else {
-            T acc[Q];
-            row_dot_b<T, Q, T>(col, A, rp[i], rp[i + 1] - rp[i], e, B, lane, acc);
-            ldq<T, Q>(e + o, ev);
-#pragma unroll
-            for (int q = 0; q < Q; q++) ev[q] = ev[q] + (rv[q] - acc[q]) * di;
+            stq<T, Q>(eout + o, ev);
+            continue;
         }
-        stq<T, Q>(e + o, ev);
+#pragma unroll
+        for (int q = 0; q < Q; q++) acc[q] = T(0);
+        if (near[i]) {
+            const int end = rp[i + 1];
+            for (int j0 = rp[i]; j0 < end; j0 += 32) {
+                const bool in = j0 + lane < end;
+                const int c = in ? col[j0 + lane] : 0;
+                const bool isb = in && btag[c];
+                const T a = isb ? A[j0 + lane] : T(0), dc = isb ? dinv[c] : T(0);
+                for (unsigned left = __ballot_sync(0xffffffffu, isb); left; left &= left - 1) {
+                    const int t = __ffs(left) - 1;
+                    T rc[Q];
+                    ldgq<T, Q>(r + (long)__shfl_sync(0xffffffffu, c, t) * B + lane * Q, rc);
+                    const T at = __shfl_sync(0xffffffffu, a, t), dt = __shfl_sync(0xffffffffu, dc, t);
+#pragma unroll
+                    for (int q = 0; q < Q; q++) acc[q] += at * (rc[q] * dt);
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const T qv = rv[q] - acc[q];
+            dv[q] = c2 * di * qv;
+            ev[q] = T(0) + dv[q];
+        }
+        stq<T, Q>(d + o, dv);
+        stq<T, Q>(eout + o, ev);
     }
 }
 
 // one Chebyshev step on interior rows: q = r - A e, d = c1 d + c2 D^-1 q, e' = e + d
 template <class T, int Q>
-__global__ void __launch_bounds__(256) k_b_cheb(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(kRowThreads, 2) k_b_cheb(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                 const T *__restrict__ A, const T *__restrict__ dinv,
                                                 const uint8_t *__restrict__ btag, const T *__restrict__ r,
                                                 const T *__restrict__ e, T *__restrict__ eout, T *__restrict__ d,
-                                                int B, T c1, T c2, int first)
+                                                int B, T c1, T c2, int first, int rpc)
 {
     const int lane = threadIdx.x & 31;
     MGM_CTA_ROWS(i, n) {
@@ -136,7 +226,7 @@ __global__ void __launch_bounds__(256) k_b_cheb(int n, const int *__restrict__ r
         ldq<T, Q>(e + o, ev);
         if (btag[i]) { stq<T, Q>(eout + o, ev); continue; }
         T acc[Q], rv[Q], dv[Q];
-        row_dot_b<T, Q, T>(col, A, rp[i], rp[i + 1] - rp[i], e, B, lane, acc);
+        row_dot_b<T, Q, T>(col, A, rp[i], rp[i + 1] - rp[i], e, lane, acc);
         ldq<T, Q>(r + o, rv);
         if (!first) ldq<T, Q>(d + o, dv);
         const T di = dinv[i];
@@ -152,10 +242,10 @@ __global__ void __launch_bounds__(256) k_b_cheb(int n, const int *__restrict__ r
 }
 
 template <class T, int Q>
-__global__ void __launch_bounds__(256) k_b_residual(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(kRowThreads, 2) k_b_residual(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                     const T *__restrict__ A, const uint8_t *__restrict__ btag,
                                                     const T *__restrict__ r, const T *__restrict__ e,
-                                                    T *__restrict__ qo, int B)
+                                                    T *__restrict__ qo, int B, int rpc)
 {
     const int lane = threadIdx.x & 31;
     MGM_CTA_ROWS(i, n) {
@@ -166,7 +256,7 @@ __global__ void __launch_bounds__(256) k_b_residual(int n, const int *__restrict
             for (int q = 0; q < Q; q++) out[q] = T(0);
         } else {
             T acc[Q], rv[Q];
-            row_dot_b<T, Q, T>(col, A, rp[i], rp[i + 1] - rp[i], e, B, lane, acc);
+            row_dot_b<T, Q, T>(col, A, rp[i], rp[i + 1] - rp[i], e, lane, acc);
             ldq<T, Q>(r + o, rv);
 #pragma unroll
             for (int q = 0; q < Q; q++) out[q] = rv[q] - acc[q];
@@ -177,36 +267,36 @@ __global__ void __launch_bounds__(256) k_b_residual(int n, const int *__restrict
 
 // y = M x for a CSR transfer matrix (empty rows give 0)
 template <class T, int Q>
-__global__ void __launch_bounds__(256) k_b_restrict(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(kRowThreads, 2) k_b_restrict(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                     const T *__restrict__ w, const T *__restrict__ x,
-                                                    T *__restrict__ y, int B)
+                                                    T *__restrict__ y, int B, int rpc)
 {
     const int lane = threadIdx.x & 31;
     MGM_CTA_ROWS(i, n) {
         T acc[Q];
-        row_dot_b<T, Q, T>(col, w, rp[i], rp[i + 1] - rp[i], x, B, lane, acc);
+        row_dot_b<T, Q, T>(col, w, rp[i], rp[i + 1] - rp[i], x, lane, acc);
         stq<T, Q>(y + (long)i * B + lane * Q, acc);
     }
 }
 
 // ef += P ec - (P ec)[row 0]
 template <class T, int Q>
-__global__ void __launch_bounds__(256) k_b_prolong(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(kRowThreads, 2) k_b_prolong(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                    const T *__restrict__ w, const T *__restrict__ ec,
-                                                   T *__restrict__ ef, int B)
+                                                   T *__restrict__ ef, int B, int rpc)
 {
     __shared__ T shift[64];
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 32) {
         T acc[Q];
-        row_dot_b<T, Q, T>(col, w, rp[0], rp[1] - rp[0], ec, B, lane, acc);
+        row_dot_b<T, Q, T>(col, w, rp[0], rp[1] - rp[0], ec, lane, acc);
 #pragma unroll
         for (int q = 0; q < Q; q++) shift[lane * Q + q] = acc[q];
     }
     __syncthreads();
     MGM_CTA_ROWS(i, n) {
         T acc[Q], ev[Q];
-        row_dot_b<T, Q, T>(col, w, rp[i], rp[i + 1] - rp[i], ec, B, lane, acc);
+        row_dot_b<T, Q, T>(col, w, rp[i], rp[i + 1] - rp[i], ec, lane, acc);
         const long o = (long)i * B + lane * Q;
         ldq<T, Q>(ef + o, ev);
 #pragma unroll
@@ -215,41 +305,65 @@ __global__ void __launch_bounds__(256) k_b_prolong(int n, const int *__restrict_
     }
 }
 
-// E[n][B] = inv[n][n] R[n][B]; block: 32 rows x B columns, K tiles of 32
+// E[n][B] = inv[n][n] R[n][B], each element's products added in column order.
+// A CTA of 128 threads owns 16 rows x 32 columns (2 x 2 per thread) and takes K
+// in tiles of 32, the next tile's loads in flight during the current one: 196
+// CTAs for 1560 rows x 64 columns, where 32 rows x 64 columns per CTA gave 49
+// and 234 us.
 template <class T, int B>
-__global__ void __launch_bounds__(256) k_b_dense(int n, const T *__restrict__ inv, const T *__restrict__ R,
+__global__ void __launch_bounds__(128) k_b_dense(int n, const T *__restrict__ inv, const T *__restrict__ R,
                                                  T *__restrict__ E)
 {
-    constexpr int RPT = B / 8;  // rows per thread
-    __shared__ T a[32][33];
-    __shared__ T rt[32][B];
-    const int tid = threadIdx.x, b = tid % B, rg = tid / B;
-    const int row0 = blockIdx.x * 32;
-    T acc[RPT];
+    constexpr int BM = 16, BN = 32, BK = 32;
+    __shared__ T a[2][BK][BM + 2];
+    __shared__ T rt[2][BK][BN];
+    const int tid = threadIdx.x, cx = (tid & 15) * 2, ry = (tid >> 4) * 2;
+    const int row0 = blockIdx.x * BM, col0 = blockIdx.y * BN;
+    T av[BM * BK / 128], rv[BK * BN / 128];
+    auto load = [&](int k0) {
 #pragma unroll
-    for (int u = 0; u < RPT; u++) acc[u] = T(0);
-    for (int k0 = 0; k0 < n; k0 += 32) {
-        for (int e = tid; e < 32 * 32; e += 256) {
-            const int rr = e / 32, kk = e % 32;
-            a[rr][kk] = (row0 + rr < n && k0 + kk < n) ? inv[(long)(row0 + rr) * n + k0 + kk] : T(0);
+        for (int u = 0; u < BM * BK / 128; u++) {
+            const int e = tid + u * 128, rr = e / BK, kk = e % BK;
+            av[u] = row0 + rr < n && k0 + kk < n ? __ldg(inv + (long)(row0 + rr) * n + k0 + kk) : T(0);
         }
-        for (int e = tid; e < 32 * B; e += 256) {
-            const int kk = e / B, bb = e % B;
-            rt[kk][bb] = k0 + kk < n ? R[(long)(k0 + kk) * B + bb] : T(0);
+#pragma unroll
+        for (int u = 0; u < BK * BN / 128; u++) {
+            const int e = tid + u * 128, kk = e / BN, cc = e % BN;
+            rv[u] = k0 + kk < n ? __ldg(R + (long)(k0 + kk) * B + col0 + cc) : T(0);
+        }
+    };
+    T acc[2][2] = {};
+    load(0);
+    for (int k0 = 0, st = 0; k0 < n; k0 += BK, st ^= 1) {
+#pragma unroll
+        for (int u = 0; u < BM * BK / 128; u++) {
+            const int e = tid + u * 128;
+            a[st][e % BK][e / BK] = av[u];
+        }
+#pragma unroll
+        for (int u = 0; u < BK * BN / 128; u++) {
+            const int e = tid + u * 128;
+            rt[st][e / BN][e % BN] = rv[u];
         }
         __syncthreads();
+        if (k0 + BK < n) load(k0 + BK);
 #pragma unroll 8
-        for (int kk = 0; kk < 32; kk++) {
-            const T rv = rt[kk][b];
-#pragma unroll
-            for (int u = 0; u < RPT; u++) acc[u] += a[rg * RPT + u][kk] * rv;
+        for (int kk = 0; kk < BK; kk++) {
+            const T r0 = rt[st][kk][cx], r1 = rt[st][kk][cx + 1];
+            const T a0 = a[st][kk][ry], a1 = a[st][kk][ry + 1];
+            acc[0][0] += a0 * r0;
+            acc[0][1] += a0 * r1;
+            acc[1][0] += a1 * r0;
+            acc[1][1] += a1 * r1;
         }
-        __syncthreads();
     }
 #pragma unroll
-    for (int u = 0; u < RPT; u++) {
-        const int row = row0 + rg * RPT + u;
-        if (row < n) E[(long)row * B + b] = acc[u];
+    for (int u = 0; u < 2; u++) {
+        const int row = row0 + ry + u;
+        if (row < n) {
+            E[(long)row * B + col0 + cx] = acc[u][0];
+            E[(long)row * B + col0 + cx + 1] = acc[u][1];
+        }
     }
 }
 
@@ -270,7 +384,7 @@ __global__ void __launch_bounds__(256) k_b_resid64(int n, const int *__restrict_
     for (int q = 0; q < Q; q++) rr[q] = bb[q] = 0.0;
     for (int i = blockIdx.x * 8 + wib; i < n; i += gridDim.x * 8) {
         double acc[Q], bq[Q];
-        row_dot_b<double, Q, X>(col, A, rp[i], rp[i + 1] - rp[i], x, B, lane, acc);
+        row_dot_b<double, Q, X>(col, A, rp[i], rp[i + 1] - rp[i], x, lane, acc);
         const long o = (long)i * B + lane * Q;
         ldq<double, Q>(bv + o, bq);
 #pragma unroll
@@ -289,14 +403,14 @@ __global__ void __launch_bounds__(256) k_b_resid64(int n, const int *__restrict_
 }
 
 template <class X, int Q>
-__global__ void __launch_bounds__(256) k_b_apply64(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(kRowThreads, 2) k_b_apply64(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                    const double *__restrict__ A, const X *__restrict__ z,
-                                                   double *__restrict__ w, int B)
+                                                   double *__restrict__ w, int B, int rpc)
 {
     const int lane = threadIdx.x & 31;
     MGM_CTA_ROWS(i, n) {
         double acc[Q];
-        row_dot_b<double, Q, X>(col, A, rp[i], rp[i + 1] - rp[i], z, B, lane, acc);
+        row_dot_b<double, Q, X>(col, A, rp[i], rp[i + 1] - rp[i], z, lane, acc);
         stq<double, Q>(w + (long)i * B + lane * Q, acc);
     }
 }
@@ -341,8 +455,18 @@ __global__ void __launch_bounds__(256) k_b_reduce(const double *__restrict__ par
     const int chunks = (B + 31) / 32;
     const int c = blockIdx.x / chunks, b = (blockIdx.x % chunks) * 32 + (threadIdx.x & 31), w = threadIdx.x >> 5;
     double s = 0;
-    if (b < B)
-        for (int k = w; k < nblk; k += 8) s += part[((long)k * cnt + c) * B + b];
+    if (b < B) {
+        // 32 loads in flight, added in order (one at a time: 55 us for 1184 blocks)
+        int k = w;
+        for (; k + 8 * 31 < nblk; k += 8 * 32) {
+            double v[32];
+#pragma unroll
+            for (int u = 0; u < 32; u++) v[u] = part[((long)(k + 8 * u) * cnt + c) * B + b];
+#pragma unroll
+            for (int u = 0; u < 32; u++) s += v[u];
+        }
+        for (; k < nblk; k += 8) s += part[((long)k * cnt + c) * B + b];
+    }
     sm[w][threadIdx.x & 31] = s;
     __syncthreads();
     if (w == 0 && b < B) {
@@ -455,6 +579,17 @@ __global__ void k_b_pin(int n, const int *__restrict__ rp, const int *__restrict
     dinv32[i] = (float)dinv64[i];
 }
 
+// near[i]: row i has a boundary neighbour
+__global__ void k_b_near(int n, const int *__restrict__ rp, const int *__restrict__ col,
+                         const uint8_t *__restrict__ btag, uint8_t *__restrict__ near)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint8_t v = 0;
+    for (int j = rp[i]; j < rp[i + 1]; j++) v |= btag[col[j]] != 0;
+    near[i] = v;
+}
+
 __global__ void k_b_pow(int n, const int *__restrict__ rp, const int *__restrict__ col, const double *__restrict__ A,
                         const double *__restrict__ dinv, const uint8_t *__restrict__ btag,
                         const double *__restrict__ v, double *__restrict__ w, double *__restrict__ part)
@@ -516,6 +651,9 @@ void batch_prepare_solver(mgm_batch *b)
         L.A64.alloc(nz); L.A32.alloc(nz); L.dinv64.alloc(L.n); L.dinv32.alloc(L.n);
         k_b_pin<<<blocks_for(L.n, 256), 256, 0, s>>>(L.n, L.rp.p, L.col.p, L.lapP.p, L.A64.p, L.A32.p, L.dinv64.p,
                                                      L.dinv32.p, flag.p);
+        MGM_LAUNCHED();
+        L.near.alloc(L.n);
+        k_b_near<<<blocks_for(L.n, 256), 256, 0, s>>>(L.n, L.rp.p, L.col.p, L.btag.p, L.near.p);
         MGM_LAUNCHED();
         if (L.r_nnz > 0) { L.r_w32.alloc((size_t)L.r_nnz); convert_d2f(L.r_w64.p, L.r_w32.p, L.r_nnz, s); }
         if (L.p_nnz > 0) { L.p_w32.alloc((size_t)L.p_nnz); convert_d2f(L.p_w64.p, L.p_w32.p, L.p_nnz, s); }
@@ -586,7 +724,7 @@ struct BLev {
     int n, nbl;
     const int *rp, *col, *bnd_list;
     const T *A, *dinv;
-    const uint8_t *btag;
+    const uint8_t *btag, *near;
     const int *r_rp, *r_col, *p_rp, *p_col;
     const T *r_w, *p_w;
     T *r, *e, *e2, *d, *q;
@@ -609,6 +747,7 @@ std::vector<BLev<T>> blevels(mgm_batch *b)
         BVecs<T> &V = vecs<T>(b, l);
         BLev<T> o{};
         o.n = L.n; o.nbl = L.nbl; o.rp = L.rp.p; o.col = L.col.p; o.bnd_list = L.bnd_list.p; o.btag = L.btag.p;
+        o.near = L.near.p;
         if constexpr (sizeof(T) == 8) { o.A = L.A64.p; o.dinv = L.dinv64.p; o.r_w = L.r_w64.p; o.p_w = L.p_w64.p; }
         else { o.A = L.A32.p; o.dinv = L.dinv32.p; o.r_w = L.r_w32.p; o.p_w = L.p_w32.p; }
         o.r_rp = L.r_rp.p; o.r_col = L.r_col.p; o.p_rp = L.p_rp.p; o.p_col = L.p_col.p;
@@ -628,9 +767,14 @@ void bsmooth(mgm_batch *b, BLev<T> &L, bool zero_start)
     const double lM = 1.05 * L.lmax, lm = L.lmax / b->cheb_ratio;
     const double th = 0.5 * (lM + lm), de = 0.5 * (lM - lm), sig = th / de;
     double rho = 1.0 / sig;
-    k_b_bnd<T, Q><<<rows_grid(L.nbl), 256, 0, s>>>(L.nbl, L.bnd_list, L.rp, L.col, L.A, L.dinv, L.r, L.e, B,
-                                                    zero_start ? 1 : 0);
-    MGM_LAUNCHED();
+    const RowShape sl = row_shape(L.n), sb = row_shape(L.nbl);
+    auto bnd = [&] {
+        if (L.nbl == 0) return;
+        k_b_bnd<T, Q><<<sb.grid, sb.threads, 0, s>>>(L.nbl, L.bnd_list, L.rp, L.col, L.A, L.dinv, L.r, L.e, B,
+                                                        sb.rpc);
+        MGM_LAUNCHED();
+    };
+    if (!zero_start) bnd();
     for (int step = 0; step < b->cheb_deg; step++) {
         double c1 = 0, c2;
         if (step == 0) c2 = 1.0 / th;
@@ -640,12 +784,15 @@ void bsmooth(mgm_batch *b, BLev<T> &L, bool zero_start)
             c2 = 2.0 * rn / de;
             rho = rn;
         }
-        k_b_cheb<T, Q><<<rows_grid(L.n), 256, 0, s>>>(L.n, L.rp, L.col, L.A, L.dinv, L.btag, L.r, L.e, L.e2, L.d,
-                                                       B, (T)c1, (T)c2, step == 0 ? 1 : 0);
+        if (step == 0 && zero_start)
+            k_b_first<T, Q><<<sl.grid, sl.threads, 0, s>>>(L.n, L.rp, L.col, L.A, L.dinv, L.btag, L.near, L.r, L.e2,
+                                                           L.d, B, (T)c2, sl.rpc);
+        else
+            k_b_cheb<T, Q><<<sl.grid, sl.threads, 0, s>>>(L.n, L.rp, L.col, L.A, L.dinv, L.btag, L.r, L.e, L.e2, L.d,
+                                                           B, (T)c1, (T)c2, step == 0 ? 1 : 0, sl.rpc);
         MGM_LAUNCHED();
         std::swap(L.e, L.e2);
-        k_b_bnd<T, Q><<<rows_grid(L.nbl), 256, 0, s>>>(L.nbl, L.bnd_list, L.rp, L.col, L.A, L.dinv, L.r, L.e, B, 0);
-        MGM_LAUNCHED();
+        bnd();
     }
 }
 
@@ -658,19 +805,22 @@ void bvcycle(mgm_batch *b, std::vector<BLev<T>> &Ls, int l)
     if (l == b->nl - 1) {
         const T *inv;
         if constexpr (sizeof(T) == 8) inv = b->cinv64.p; else inv = b->cinv32.p;
-        k_b_dense<T, B><<<blocks_for(L.n, 32), 256, 0, s>>>(L.n, inv, L.r, L.e);
+        k_b_dense<T, B><<<dim3(blocks_for(L.n, 16), B / 32), 128, 0, s>>>(L.n, inv, L.r, L.e);
         MGM_LAUNCHED();
         return;
     }
-    MGM_CUDA(cudaMemsetAsync(L.e, 0, sizeof(T) * (size_t)L.n * B, s));
-    bsmooth<T, Q>(b, L, true);
+    bsmooth<T, Q>(b, L, true);  // from e = 0
     BLev<T> &C = Ls[l + 1];
-    k_b_residual<T, Q><<<rows_grid(L.n), 256, 0, s>>>(L.n, L.rp, L.col, L.A, L.btag, L.r, L.e, L.q, B);
+    const RowShape sl = row_shape(L.n), sc = row_shape(C.n);
+    k_b_residual<T, Q><<<sl.grid, sl.threads, 0, s>>>(L.n, L.rp, L.col, L.A, L.btag, L.r, L.e, L.q, B,
+                                                       sl.rpc);
     MGM_LAUNCHED();
-    k_b_restrict<T, Q><<<rows_grid(C.n), 256, 0, s>>>(C.n, C.r_rp, C.r_col, C.r_w, L.q, C.r, B);
+    k_b_restrict<T, Q><<<sc.grid, sc.threads, 0, s>>>(C.n, C.r_rp, C.r_col, C.r_w, L.q, C.r, B,
+                                                       sc.rpc);
     MGM_LAUNCHED();
     bvcycle<T, Q>(b, Ls, l + 1);
-    k_b_prolong<T, Q><<<rows_grid(L.n), 256, 0, s>>>(L.n, L.p_rp, L.p_col, L.p_w, C.e, L.e, B);
+    k_b_prolong<T, Q><<<sl.grid, sl.threads, 0, s>>>(L.n, L.p_rp, L.p_col, L.p_w, C.e, L.e, B,
+                                                      sl.rpc);
     MGM_LAUNCHED();
     bsmooth<T, Q>(b, L, false);
 }
@@ -716,6 +866,7 @@ void bfgmres(mgm_batch *b, int nrhs, int *vcycles, double *rel_res)
     if constexpr (sizeof(T) == 8) Z = b->Z64.p; else Z = b->Z32.p;
     double *V = b->V.p, *X = b->X.p, *hp = b->h_pinned, *dsc = b->hsc.p;
     const int gres = dot_grid(n);
+    const RowShape sl = row_shape(n);
     const int gdot = (int)std::max(1L, std::min<long>((n + (256 / B) - 1) / (256 / B), 148L * 8));
     const size_t part_need = std::max({(size_t)gres * 2 * B, (size_t)gdot * 8 * B, (size_t)148 * 16 * B});
     if (b->part.n < part_need) b->part.alloc(part_need);
@@ -770,7 +921,8 @@ void bfgmres(mgm_batch *b, int nrhs, int *vcycles, double *rel_res)
             // cancelled more than 1 - 1/sqrt(2) of |w| for some right-hand side
             // (the Daniel-Gragg-Kaufman-Stewart test)
             double *Wn = V + (long)(j + 1) * nB;
-            k_b_apply64<T, Q><<<rows_grid(n), 256, 0, s>>>(n, L0.rp.p, L0.col.p, L0.A64.p, Z + (long)j * nB, Wn, B);
+            k_b_apply64<T, Q><<<sl.grid, sl.threads, 0, s>>>(n, L0.rp.p, L0.col.p, L0.A64.p, Z + (long)j * nB, Wn, B,
+                                                              sl.rpc);
             MGM_LAUNCHED();
             const int h1 = 0, h2 = (kBatchMaxRestart + 2) * B, h3 = 2 * (kBatchMaxRestart + 2) * B;
             multidot(j + 2, V, Wn, h1);  // dots with V_0..V_j, then |w|^2
