@@ -959,7 +959,8 @@ void poisson(mgm_ctx *c, int mode, bool timple = false, bool captured = false, l
         MGM_REQUIRE(c->have_ref_transfer || c->nl == 1, "reference mode needs mgm_setup(..., MGM_SETUP_REFERENCE_TRANSFER)");
         auto R = ref_levels(c);
         const double w1 = (double)c->omega, w2 = (double)(1 - c->omega);
-        ref_multigrid(R, w1, w2, c->num_relax, c->num_vcycles, c->s, timple ? REF_TIMPLE : REF_FS);
+        ref_multigrid(R, w1, w2, c->num_relax, c->num_vcycles, c->s, timple ? REF_TIMPLE : REF_FS,
+                      c->chain_launches);
         return;
     }
     if (mode != MGM_MODE_FP64 && mode != MGM_MODE_FP32_IR) throw Error{MGM_ERR_ARG, "unknown Poisson mode"};
@@ -1153,7 +1154,7 @@ void ref_cycles(mgm_ctx *c, RefVariant v, int num_cycles)
     MGM_REQUIRE(c->have_ref_transfer || c->nl == 1, "reference mode needs mgm_setup(..., MGM_SETUP_REFERENCE_TRANSFER)");
     auto R = ref_levels(c);
     const double w1 = (double)c->omega, w2 = (double)(1 - c->omega);
-    ref_multigrid(R, w1, w2, c->num_relax, num_cycles, c->s, v);
+    ref_multigrid(R, w1, w2, c->num_relax, num_cycles, c->s, v, c->chain_launches);
 }
 }  // namespace mgm
 

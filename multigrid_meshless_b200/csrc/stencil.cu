@@ -9,6 +9,8 @@
 // the reference's C loops on the same operator values.
 #include "stencil.cuh"
 
+#include "rows.cuh"
+
 namespace mgm {
 
 template <int BS>
@@ -311,164 +313,284 @@ void launch_mass_diag(const StepArgs &a, int dim, double *partial, double *d_out
 
 // ---------------------------------------------------------------------------
 // reference-semantics multigrid (fractional_step_solver.h:150-246)
+//
+// A level's rows are a few per scheduler and each a chain of dependent loads
+// (index, then gather), so the kernels are chained launches that hold the first
+// slots' indices and weights before they wait for their predecessor, and fetch
+// the next slots' while the current gathers are in flight (one slot at a time
+// and unchained a sweep of 65k rows of 30 slots took 18 us, now 12).  SMALL:
+// levels below kRefSmallRows rows, which fit the chip with 32 slots in registers
+// per thread, gather from L2 and release their successor before the wait
+// (rows.cuh); 65k rows gather 68 MB of sectors that way against L1's reuse
+// (10 cycles of 4 levels: 1.57 ms with the level as SMALL, 1.52 without).
+constexpr int kRefSmallRows = 32768;
+template <bool SMALL>
+struct RefRow {
+    static constexpr int C = SMALL ? 32 : 8;
+    int c[C];
+    double w[C];
+    __device__ __forceinline__ void fetch(int n, int k, long i, const int *idx, const double *W, int j)
+    {
+        const int *pi = idx + (long)j * n + i;
+        const double *pw = W + (long)j * n + i;
+#pragma unroll
+        for (int q = 0; q < C; q++) {
+            c[q] = ldk(pi);
+            w[q] = ldk(pw);
+            const int st = j + q + 1 < k ? n : 0;  // past the row: its last slot again
+            pi += st;
+            pw += st;
+        }
+    }
+    // slots j0.. in order: op(weight, x[index] (- shift with SHIFT)), after
+    // fetch(j0) and the wait
+    template <bool SHIFT, class Op>
+    __device__ __forceinline__ void run(int n, int k, long i, const int *idx, const double *W, int j0, const double *x,
+                                        double shift, Op op)
+    {
+        for (int j = j0; j < k; j += C) {
+            double v[C];
+#pragma unroll
+            for (int q = 0; q < C; q++) v[q] = gather<SMALL>(x + c[q]);
+            if constexpr (SMALL) {
+#pragma unroll
+                for (int q = 0; q < C; q++)
+                    if (j + q < k) op(w[q], SHIFT ? MGM_SUB(v[q], shift) : v[q]);
+                if (j + C < k) fetch(n, k, i, idx, W, j + C);
+            } else {
+                double wc[C];
+#pragma unroll
+                for (int q = 0; q < C; q++) wc[q] = w[q];
+                if (j + C < k) fetch(n, k, i, idx, W, j + C);
+#pragma unroll
+                for (int q = 0; q < C; q++)
+                    if (j + q < k) op(wc[q], SHIFT ? MGM_SUB(v[q], shift) : v[q]);
+            }
+        }
+    }
+};
+
 // relaxation sweep (:171-179) in data-parallel (Jacobi) order: every node is
-// updated from the previous sweep's values.
-__global__ void __launch_bounds__(256) k_ref_sweep(int n, int k, const int *__restrict__ idx,
+// updated from the previous sweep's values.  SHIFT: pin is the previous sweep
+// before its re-pin p -= p[0] (:180-183), which is applied on the way in, so
+// that a relaxation needs no pass of its own for it between two sweeps.
+template <bool SHIFT, bool SMALL>
+__global__ void __launch_bounds__(128) k_ref_sweep(int n, int k, const int *__restrict__ idx,
                                                    const double *__restrict__ lapP, const double *__restrict__ src,
                                                    const double *__restrict__ pin, double *__restrict__ pout, double w1,
                                                    double w2)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double sum = 0.0;
-    for (int j = 1; j < k; j++) {
-        const long o = (long)j * n + i;
-        sum = MGM_ADD(sum, MGM_MUL(lapP[o], pin[idx[o]]));
-    }
-    pout[i] = MGM_ADD(MGM_MUL(w1, MGM_DIV(MGM_SUB(src[i], sum), lapP[i])), MGM_MUL(w2, pin[i]));
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, i = min(i0, n - 1);
+    RefRow<SMALL> R;
+    R.fetch(n, k, i, idx, lapP, 1);
+    const double di = ldk(lapP + i);
+    pdl_wait<SMALL>();
+    const double pref = SHIFT ? gather<SMALL>(pin) : 0.0, si = gather<SMALL>(src + i);
+    double pi = gather<SMALL>(pin + i), sum = 0.0;
+    R.template run<SHIFT>(n, k, i, idx, lapP, 1, pin, pref, [&](double w, double v) { sum = MGM_ADD(sum, MGM_MUL(w, v)); });
+    if (SHIFT) pi = MGM_SUB(pi, pref);
+    if (i0 < n) pout[i] = MGM_ADD(MGM_MUL(w1, MGM_DIV(MGM_SUB(si, sum), di)), MGM_MUL(w2, pi));
 }
 
-// p -= p[0] (:180-183) fused with the all-node residual (:185-191).  TIMPLE
-// form (timple_solver.h:265-281): the residual uses lap_Poison (passed as lap)
-// on interior rows and is 0 on boundary rows (btag non-null).
-__global__ void __launch_bounds__(256) k_ref_shift_residual(int n, int k, const int *__restrict__ idx,
+// What follows a relaxation's last sweep: p -= p[0] (:180-183) with the
+// all-node residual (:185-191), r = src - l_0 p - l_1 p ...; TIMPLE form
+// (timple_solver.h:265-281): lap_Poison (passed as lap), 0 on boundary rows
+// (zero_boundary).  With `interior` also calculate_residuals (:236-246, TIMPLE
+// timple_solver.h:285-301), which overwrites the interior rows with
+// src - (sum of the products).
+template <bool SMALL>
+__global__ void __launch_bounds__(128) k_ref_shift_residual(int n, int k, const int *__restrict__ idx,
                                                             const double *__restrict__ lap,
                                                             const double *__restrict__ src,
                                                             const double *__restrict__ pin, double *__restrict__ pout,
-                                                            double *__restrict__ res, const uint8_t *__restrict__ btag)
+                                                            double *__restrict__ res, const uint8_t *__restrict__ btag,
+                                                            int zero_boundary, int interior)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double pref = pin[0];
-    pout[i] = MGM_SUB(pin[i], pref);
-    if (btag && btag[i]) { res[i] = 0.0; return; }
-    double r = src[i];
-    for (int j = 0; j < k; j++) {
-        const long o = (long)j * n + i;
-        r = MGM_SUB(r, MGM_MUL(lap[o], MGM_SUB(pin[idx[o]], pref)));
-    }
-    res[i] = r;
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, i = min(i0, n - 1);
+    RefRow<SMALL> R;
+    R.fetch(n, k, i, idx, lap, 0);
+    const bool bnd = ldk(btag + i) != 0;
+    pdl_wait<SMALL>();
+    const double pref = gather<SMALL>(pin), pi = gather<SMALL>(pin + i), si = gather<SMALL>(src + i);
+    double sum = 0.0, r = si;
+    R.template run<true>(n, k, i, idx, lap, 0, pin, pref, [&](double w, double v) {
+        const double t = MGM_MUL(w, v);
+        sum = MGM_ADD(sum, t);
+        r = MGM_SUB(r, t);
+    });
+    if (i0 >= n) return;
+    pout[i] = MGM_SUB(pi, pref);
+    res[i] = bnd && zero_boundary ? 0.0 : interior && !bnd ? MGM_SUB(si, sum) : r;
 }
 
 // calculate_residuals (:236-246): interior rows only.  TIMPLE form
 // (timple_solver.h:285-301, zero_boundary): lap_Poison, boundary rows set to 0.
-__global__ void __launch_bounds__(256) k_ref_residual_interior(int n, int k, const int *__restrict__ idx,
+template <bool SMALL>
+__global__ void __launch_bounds__(128) k_ref_residual_interior(int n, int k, const int *__restrict__ idx,
                                                                const double *__restrict__ lap,
                                                                const uint8_t *__restrict__ btag,
                                                                const double *__restrict__ src,
                                                                const double *__restrict__ p, double *__restrict__ res,
                                                                int zero_boundary)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (btag[i]) {
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, i = min(i0, n - 1);
+    RefRow<SMALL> R;
+    R.fetch(n, k, i, idx, lap, 0);
+    const bool bnd = ldk(btag + i) != 0;
+    pdl_wait<SMALL>();
+    if (i0 >= n) return;
+    if (bnd) {
         if (zero_boundary) res[i] = 0.0;
         return;
     }
+    const double si = gather<SMALL>(src + i);
     double sum = 0;
-    for (int j = 0; j < k; j++) {
-        const long o = (long)j * n + i;
-        sum = MGM_ADD(sum, MGM_MUL(lap[o], p[idx[o]]));
-    }
-    res[i] = MGM_SUB(src[i], sum);
+    R.template run<false>(n, k, i, idx, lap, 0, p, 0.0, [&](double w, double v) { sum = MGM_ADD(sum, MGM_MUL(w, v)); });
+    res[i] = MGM_SUB(si, sum);
 }
 
 // restrict_residuals (:198-212) / the sum of prolongate_corrections (:216-227):
 // out[i] (+)= sum_j W[j][i] * in[gidx[j][i]] on rows whose tag is 0; rows
 // with a tag are left alone, or set to 0 with zero_tagged (the TIMPLE
 // restriction writes every coarse row, timple_solver.h:303-317).
-__global__ void __launch_bounds__(256) k_ref_transfer(int n, int k, const int *__restrict__ gidx,
+template <bool SMALL>
+__global__ void __launch_bounds__(128) k_ref_transfer(int n, int k, const int *__restrict__ gidx,
                                                       const double *__restrict__ W, const uint8_t *__restrict__ btag,
                                                       const double *__restrict__ in, double *__restrict__ out,
                                                       int accumulate, int zero_tagged)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (btag[i]) {
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, i = min(i0, n - 1);
+    RefRow<SMALL> R;
+    R.fetch(n, k, i, gidx, W, 0);
+    const bool tag = ldk(btag + i) != 0;
+    pdl_wait<SMALL>();
+    if (i0 >= n) return;
+    if (tag) {
         if (zero_tagged) out[i] = 0.0;
         return;
     }
+    const double o = accumulate ? out[i] : 0.0;
     double r = 0.0;
-    for (int j = 0; j < k; j++) {
-        const long o = (long)j * n + i;
-        r = MGM_ADD(r, MGM_MUL(W[o], in[gidx[o]]));
-    }
-    out[i] = accumulate ? MGM_ADD(out[i], r) : r;
+    R.template run<false>(n, k, i, gidx, W, 0, in, 0.0, [&](double w, double v) { r = MGM_ADD(r, MGM_MUL(w, v)); });
+    out[i] = accumulate ? MGM_ADD(o, r) : r;
 }
 
-__global__ void k_zero_interior(int n, const uint8_t *__restrict__ btag, double *__restrict__ p)
+// p = 0, on rows with a tag only with `all`
+template <bool SMALL>
+__global__ void __launch_bounds__(128) k_ref_zero(int n, const uint8_t *__restrict__ btag, double *__restrict__ p,
+                                                  int all)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !btag[i]) p[i] = 0.0;
+    const bool tag = i < n && ldk(btag + i) != 0;
+    pdl_wait<SMALL>();
+    if (i < n && (all || !tag)) p[i] = 0.0;
 }
 
-void ref_relaxation(const RefLevel &L, double w1, double w2, int num_relax, cudaStream_t s, RefVariant v)
+// The sweeps of one relaxation.  Their residuals between sweeps (:185-191) are
+// overwritten unread, so only the last one is taken, and L.res serves as the
+// third buffer of an even number of sweeps; the last sweep lands in L.ptmp.
+// interior: followed by calculate_residuals.
+static void ref_relax(const RefLevel &L, double w1, double w2, int num_relax, cudaStream_t s, RefVariant v,
+                      bool interior, Chain &launch)
 {
-    const int nb = blocks_for(L.n, 256);
+    const int nb = blocks_for(L.n, 128);
+    const bool small = L.n < kRefSmallRows;
+    double *in = L.p;
     for (int it = 0; it < num_relax; it++) {
-        k_ref_sweep<<<nb, 256, 0, s>>>(L.n, L.k, L.idx, L.lapP, L.src, L.p, L.ptmp, w1, w2);
-        MGM_LAUNCHED();
-        if (v == REF_HEAT) {
-            // heat_conduction.h:27-35: the sweep alone (no re-pin, no residual)
-            MGM_CUDA(cudaMemcpyAsync(L.p, L.ptmp, sizeof(double) * L.n, cudaMemcpyDeviceToDevice, s));
-            continue;
-        }
-        const bool t = v == REF_TIMPLE;
-        k_ref_shift_residual<<<nb, 256, 0, s>>>(L.n, L.k, L.idx, t ? L.lapP : L.lap, L.src, L.ptmp, L.p, L.res,
-                                                t ? L.btag : nullptr);
-        MGM_LAUNCHED();
+        const bool heat = v == REF_HEAT;
+        double *out = in == L.ptmp ? L.p : L.ptmp;
+        if (!heat && it == 0 && num_relax % 2 == 0) out = L.res;
+        const bool first = heat || it == 0;
+        launch(small ? (first ? k_ref_sweep<false, true> : k_ref_sweep<true, true>)
+                     : (first ? k_ref_sweep<false, false> : k_ref_sweep<true, false>), nb, 128, 0, s, L.n, L.k, L.idx, L.lapP,
+               (const double *)L.src, (const double *)in, out, w1, w2);
+        in = out;
     }
+    if (num_relax <= 0) return;
+    if (v == REF_HEAT) {
+        // heat_conduction.h:27-35: the sweeps alone (no re-pin, no residual)
+        if (in != L.p) {
+            MGM_CUDA(cudaMemcpyAsync(L.p, in, sizeof(double) * L.n, cudaMemcpyDeviceToDevice, s));
+            launch.broken();
+        }
+        return;
+    }
+    const bool t = v == REF_TIMPLE;
+    launch(small ? k_ref_shift_residual<true> : k_ref_shift_residual<false>, nb, 128, 0, s, L.n, L.k, L.idx,
+           t ? L.lapP : L.lap, (const double *)L.src, (const double *)in, L.p, L.res, L.btag, t ? 1 : 0,
+           interior ? 1 : 0);
 }
 
 // the TIMPLE and heat residuals are the same: lap_Poison on interior rows, 0 on
 // boundary rows (timple_solver.h:285-301, heat_conduction.h:100-113)
-void ref_residual_interior(const RefLevel &L, cudaStream_t s, RefVariant v)
+static void ref_residual(const RefLevel &L, cudaStream_t s, RefVariant v, Chain &launch)
 {
     const bool t = v != REF_FS;
-    k_ref_residual_interior<<<blocks_for(L.n, 256), 256, 0, s>>>(L.n, L.k, L.idx, t ? L.lapP : L.lap, L.btag,
-                                                                 L.src, L.p, L.res, t ? 1 : 0);
-    MGM_LAUNCHED();
+    const auto kern = L.n < kRefSmallRows ? k_ref_residual_interior<true> : k_ref_residual_interior<false>;
+    launch(kern, blocks_for(L.n, 128), 128, 0, s, L.n, L.k, L.idx, t ? L.lapP : L.lap, L.btag,
+           (const double *)L.src, (const double *)L.p, L.res, t ? 1 : 0);
 }
 
 // the TIMPLE and heat restrictions write every coarse row (timple_solver.h:303-317,
 // heat_conduction.h:57-75)
-void ref_restrict(const RefLevel &F, const RefLevel &C, cudaStream_t s, RefVariant v)
+static void ref_restrict_k(const RefLevel &F, const RefLevel &C, cudaStream_t s, RefVariant v, Chain &launch)
 {
-    k_ref_transfer<<<blocks_for(C.n, 256), 256, 0, s>>>(C.n, F.k, C.r_idx, C.restr, C.btag, F.res, C.src, 0,
-                                                        v != REF_FS ? 1 : 0);
-    MGM_LAUNCHED();
+    const auto kern = C.n < kRefSmallRows ? k_ref_transfer<true> : k_ref_transfer<false>;
+    launch(kern, blocks_for(C.n, 128), 128, 0, s, C.n, F.k, C.r_idx, C.restr, C.btag, (const double *)F.res,
+           C.src, 0, v != REF_FS ? 1 : 0);
 }
 
+static void ref_prolongate_k(const RefLevel &F, const RefLevel &C, cudaStream_t s, RefVariant v, Chain &launch)
+{
+    const auto kern = F.n < kRefSmallRows ? k_ref_transfer<true> : k_ref_transfer<false>;
+    launch(kern, blocks_for(F.n, 128), 128, 0, s, F.n, C.k, F.p_idx, F.prol, F.btag, (const double *)C.p,
+           F.p, 1, 0);
+    // coarse interior corrections reset (fractional_step_solver.h:228-233,
+    // heat_conduction.h:92-97); every coarse correction in TIMPLE (timple_solver.h:333-338)
+    const auto zero = C.n < kRefSmallRows ? k_ref_zero<true> : k_ref_zero<false>;
+    launch(zero, blocks_for(C.n, 128), 128, 0, s, C.n, C.btag, C.p, v == REF_TIMPLE ? 1 : 0);
+}
+
+void ref_relaxation(const RefLevel &L, double w1, double w2, int num_relax, cudaStream_t s, RefVariant v)
+{
+    Chain launch;
+    ref_relax(L, w1, w2, num_relax, s, v, false, launch);
+}
+void ref_residual_interior(const RefLevel &L, cudaStream_t s, RefVariant v)
+{
+    Chain launch;
+    ref_residual(L, s, v, launch);
+}
+void ref_restrict(const RefLevel &F, const RefLevel &C, cudaStream_t s, RefVariant v)
+{
+    Chain launch;
+    ref_restrict_k(F, C, s, v, launch);
+}
 void ref_prolongate(const RefLevel &F, const RefLevel &C, cudaStream_t s, RefVariant v)
 {
-    k_ref_transfer<<<blocks_for(F.n, 256), 256, 0, s>>>(F.n, C.k, F.p_idx, F.prol, F.btag, C.p, F.p, 1, 0);
-    MGM_LAUNCHED();
-    if (v == REF_TIMPLE) {
-        // every coarse correction reset (timple_solver.h:333-338)
-        MGM_CUDA(cudaMemsetAsync(C.p, 0, sizeof(double) * C.n, s));
-    } else {
-        // coarse interior corrections reset (fractional_step_solver.h:228-233, heat_conduction.h:92-97)
-        k_zero_interior<<<blocks_for(C.n, 256), 256, 0, s>>>(C.n, C.btag, C.p);
-        MGM_LAUNCHED();
-    }
+    Chain launch;
+    ref_prolongate_k(F, C, s, v, launch);
 }
 
 // multigrid_Poisson_solver (fractional_step_solver.h:150-166); the TIMPLE
 // variant (timple_solver.h:203-220) and the heat-conduction program's cycle
 // (mg_heat_conduction.c:57-71) have the same shape over their own routines
 void ref_multigrid(std::vector<RefLevel> &Ls, double w1, double w2, int num_relax, int num_vcycles, cudaStream_t s,
-                   RefVariant v)
+                   RefVariant v, bool chain)
 {
     const int nl = (int)Ls.size();
+    Chain launch;
+    launch.enabled = chain;
     for (int cyc = 0; cyc < num_vcycles; cyc++) {
         for (int l = 0; l < nl; l++) {
-            ref_relaxation(Ls[l], w1, w2, num_relax, s, v);
-            ref_residual_interior(Ls[l], s, v);
-            if (l != nl - 1) ref_restrict(Ls[l], Ls[l + 1], s, v);
+            const bool with_residual = v != REF_HEAT && num_relax > 0;
+            ref_relax(Ls[l], w1, w2, num_relax, s, v, with_residual, launch);
+            if (!with_residual) ref_residual(Ls[l], s, v, launch);
+            if (l != nl - 1) ref_restrict_k(Ls[l], Ls[l + 1], s, v, launch);
         }
         for (int l = nl - 1; l > 0; l--) {
-            ref_prolongate(Ls[l - 1], Ls[l], s, v);
-            if (l != 1) ref_relaxation(Ls[l - 1], w1, w2, num_relax, s, v);
+            ref_prolongate_k(Ls[l - 1], Ls[l], s, v, launch);
+            if (l != 1) ref_relax(Ls[l - 1], w1, w2, num_relax, s, v, false, launch);
         }
     }
 }

@@ -50,7 +50,7 @@ void ref_residual_interior(const RefLevel &L, cudaStream_t s, RefVariant v = REF
 void ref_restrict(const RefLevel &F, const RefLevel &C, cudaStream_t s, RefVariant v = REF_FS);
 void ref_prolongate(const RefLevel &F, const RefLevel &C, cudaStream_t s, RefVariant v = REF_FS);
 void ref_multigrid(std::vector<RefLevel> &Ls, double w1, double w2, int num_relax, int num_vcycles, cudaStream_t s,
-                   RefVariant v = REF_FS);
+                   RefVariant v, bool chain);
 
 // ---------------------------------------------------------------------------
 // convergent solver (solver.cu)
