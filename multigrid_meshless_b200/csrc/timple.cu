@@ -44,102 +44,181 @@ __global__ void k_t_iter(TimpleArgs a)
     a.pprime[i] = 0;
 }
 
+// A thread's row, slots j0.. in order, of NW operators over the shared gather
+// index: 4 slots at a time, the next 4 slots' indices and weights in flight
+// while the current gathers are.  A level has a few such rows per scheduler
+// and one slot at a time is a chain of two memory latencies.
+template <int NW>
+struct TimpleRow {
+    static constexpr int C = 4;
+    int c[C];
+    double w[NW][C];
+    const double *W[NW];
+    __device__ __forceinline__ void fetch(const TimpleArgs &a, int i, int j)
+    {
+#pragma unroll
+        for (int q = 0; q < C; q++) {
+            const long o = (long)min(j + q, a.k - 1) * a.n + i;
+            c[q] = __ldg(a.idx + o);
+#pragma unroll
+            for (int m = 0; m < NW; m++) w[m][q] = __ldg(W[m] + o);
+        }
+    }
+    // op(weights, values) with the values of the NX fields x at the slot's index
+    template <int NX, class Op>
+    __device__ __forceinline__ void run(const TimpleArgs &a, int i, int j0, const double *const (&x)[NX], Op op)
+    {
+        fetch(a, i, j0);
+        for (int j = j0; j < a.k; j += C) {
+            double v[C][NX], wc[C][NW];
+#pragma unroll
+            for (int q = 0; q < C; q++) {
+#pragma unroll
+                for (int m = 0; m < NX; m++) v[q][m] = x[m][c[q]];
+#pragma unroll
+                for (int m = 0; m < NW; m++) wc[q][m] = w[m][q];
+            }
+            if (j + C < a.k) fetch(a, i, j + C);
+#pragma unroll
+            for (int q = 0; q < C; q++)
+                if (j + q < a.k) op(wc[q], v[q]);
+        }
+    }
+};
+
 // One momentum sweep of calculate_intermediate_velocity_implicit (:88-173) in
 // data-parallel order: interior rows from the previous sweep's values (in*),
-// boundary rows copied.
+// boundary rows copied.  The operators are read once for all components (once
+// per component and slot by slot a sweep of the 250k-row annulus took 115 us,
+// now 50).
 template <int DIM>
-__global__ void __launch_bounds__(256) k_t_momentum(TimpleArgs a, const double *__restrict__ iu,
+__global__ void __launch_bounds__(128) k_t_momentum(TimpleArgs a, const double *__restrict__ iu,
                                                     const double *__restrict__ iv, const double *__restrict__ iw,
                                                     double *__restrict__ ou, double *__restrict__ ov,
                                                     double *__restrict__ ow)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = a.n, k = a.k;
-    if (i >= n) return;
+    if (i >= a.n) return;
     if (a.btag[i]) {
         ou[i] = iu[i]; ov[i] = iv[i];
         if (DIM == 3) ow[i] = iw[i];
         return;
     }
-    const double *comp_in[3] = {iu, iv, iw};
     double *comp_out[3] = {ou, ov, ow};
     const double *comp_old[3] = {a.u_old, a.v_old, a.w_old};
     const double *grad[3] = {a.dpdx, a.dpdy, a.dpdz};
     const double lap0 = a.lap[i], dx0 = a.Dx[i], dy0 = a.Dy[i];
     const double dz0 = DIM == 3 ? a.Dz[i] : 0.0;
     const double ui = a.u[i], vi = a.v[i], wi = a.w[i];
+    double t1[DIM] = {}, t2[DIM] = {}, t3[DIM] = {}, t4[DIM] = {}, own[DIM], old[DIM], gr[DIM];
+    const double *xs[DIM];
+    xs[0] = iu;
+    xs[1] = iv;
+    if constexpr (DIM == 3) xs[2] = iw;
 #pragma unroll
-    for (int cidx = 0; cidx < DIM; cidx++) {
-        const double *x = comp_in[cidx];
-        double temp1 = 0, temp2 = 0, temp3 = 0, temp4 = 0;
-        const double advection_x = MGM_MUL(ui, dx0);
-        const double advection_y = MGM_MUL(vi, dy0);
-        const double diffusion = MGM_MUL(MGM_MUL(-a.facRe, a.mu), lap0);
-        double unsteady = MGM_DIV(1., MGM_MUL(a.dt, a.facdt));
+    for (int q = 0; q < DIM; q++) { own[q] = xs[q][i]; old[q] = comp_old[q][i]; gr[q] = grad[q][i]; }
+    TimpleRow<DIM + 1> R;
+    R.W[0] = a.Dx;
+    R.W[1] = a.Dy;
+    R.W[2] = a.lap;
+    if constexpr (DIM == 3) R.W[3] = a.Dz;
+    R.template run<DIM>(a, i, 1, xs, [&](const double (&w)[DIM + 1], const double (&x)[DIM]) {
+#pragma unroll
+        for (int q = 0; q < DIM; q++) {
+            t1[q] = MGM_ADD(t1[q], MGM_MUL(w[0], x[q]));
+            t2[q] = MGM_ADD(t2[q], MGM_MUL(w[1], x[q]));
+            t4[q] = MGM_ADD(t4[q], MGM_MUL(w[2], x[q]));
+            if constexpr (DIM == 3) t3[q] = MGM_ADD(t3[q], MGM_MUL(w[3], x[q]));
+        }
+    });
+    const double advection_x = MGM_MUL(ui, dx0), advection_y = MGM_MUL(vi, dy0);
+    const double diffusion = MGM_MUL(MGM_MUL(-a.facRe, a.mu), lap0);
+    const double unsteady0 = MGM_DIV(1., MGM_MUL(a.dt, a.facdt));
+#pragma unroll
+    for (int q = 0; q < DIM; q++) {
         double denom;
-        if (cidx < 2) {
-            denom = MGM_ADD(MGM_MUL(a.rho, MGM_ADD(MGM_ADD(advection_x, advection_y), unsteady)), diffusion);
-            for (int j = 1; j < k; j++) {
-                const long o = (long)j * n + i;
-                const double xv = x[a.idx[o]];
-                temp1 = MGM_ADD(temp1, MGM_MUL(a.Dx[o], xv));
-                temp2 = MGM_ADD(temp2, MGM_MUL(a.Dy[o], xv));
-                temp4 = MGM_ADD(temp4, MGM_MUL(a.lap[o], xv));
-            }
-            if (DIM == 3) {
-                denom = MGM_ADD(denom, MGM_MUL(MGM_MUL(a.rho, wi), dz0));
-                for (int j = 1; j < k; j++) {
-                    const long o = (long)j * n + i;
-                    temp3 = MGM_ADD(temp3, MGM_MUL(a.Dz[o], x[a.idx[o]]));
-                }
-            }
+        if (q < 2) {
+            denom = MGM_ADD(MGM_MUL(a.rho, MGM_ADD(MGM_ADD(advection_x, advection_y), unsteady0)), diffusion);
+            if (DIM == 3) denom = MGM_ADD(denom, MGM_MUL(MGM_MUL(a.rho, wi), dz0));
         } else {
             const double advection_z = MGM_MUL(wi, dz0);
-            denom = MGM_ADD(MGM_MUL(a.rho, MGM_ADD(MGM_ADD(MGM_ADD(advection_x, advection_y), advection_z), unsteady)),
+            denom = MGM_ADD(MGM_MUL(a.rho, MGM_ADD(MGM_ADD(MGM_ADD(advection_x, advection_y), advection_z), unsteady0)),
                             diffusion);
-            for (int j = 1; j < k; j++) {
-                const long o = (long)j * n + i;
-                const double xv = x[a.idx[o]];
-                temp1 = MGM_ADD(temp1, MGM_MUL(a.Dx[o], xv));
-                temp2 = MGM_ADD(temp2, MGM_MUL(a.Dy[o], xv));
-                temp3 = MGM_ADD(temp3, MGM_MUL(a.Dz[o], xv));
-                temp4 = MGM_ADD(temp4, MGM_MUL(a.lap[o], xv));
-            }
         }
-        const double advection = MGM_ADD(MGM_ADD(MGM_MUL(ui, temp1), MGM_MUL(vi, temp2)), MGM_MUL(wi, temp3));
-        unsteady = MGM_DIV(comp_old[cidx][i], MGM_MUL(a.dt, a.facdt));
+        const double advection = MGM_ADD(MGM_ADD(MGM_MUL(ui, t1[q]), MGM_MUL(vi, t2[q])), MGM_MUL(wi, t3[q]));
+        const double unsteady = MGM_DIV(old[q], MGM_MUL(a.dt, a.facdt));
         double num = MGM_MUL(a.rho, MGM_SUB(unsteady, advection));
-        num = MGM_SUB(num, MGM_MUL(MGM_MUL(MGM_MUL(MGM_SUB(a.facRe, 1.0), a.mu), lap0), x[i]));
-        num = MGM_ADD(num, MGM_MUL(a.mu, temp4));
-        num = MGM_SUB(num, grad[cidx][i]);
-        comp_out[cidx][i] = MGM_DIV(num, denom);
+        num = MGM_SUB(num, MGM_MUL(MGM_MUL(MGM_MUL(MGM_SUB(a.facRe, 1.0), a.mu), lap0), own[q]));
+        num = MGM_ADD(num, MGM_MUL(a.mu, t4[q]));
+        num = MGM_SUB(num, gr[q]);
+        comp_out[q][i] = MGM_DIV(num, denom);
     }
 }
 
-// calculate_mass_residual_implicit (:186-197): source from the divergence
-// (dpdz is 0 in 2D: never written there, as in the reference)
-__global__ void k_t_source(TimpleArgs a)
+// dpdx, dpdy(, dpdz) = the gradient of one field.  UPDATE: of p', followed by
+// update_velocity_implicit (:351-363): interior velocities and pressure; pref
+// gets the new p_old[0].
+template <int DIM, bool UPDATE>
+__global__ void __launch_bounds__(128) k_t_gradient(TimpleArgs a, const double *__restrict__ f,
+                                                    double *__restrict__ pref)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
-    a.source[i] = a.btag[i] ? 0.0
-                            : MGM_DIV(MGM_MUL(a.rho, MGM_ADD(MGM_ADD(a.dpdx[i], a.dpdy[i]), a.dpdz[i])), a.dt);
+    double g[DIM] = {};
+    TimpleRow<DIM> R;
+    R.W[0] = a.Dx;
+    R.W[1] = a.Dy;
+    if constexpr (DIM == 3) R.W[2] = a.Dz;
+    const double *const xs[1] = {f};
+    R.template run<1>(a, i, 0, xs, [&](const double (&w)[DIM], const double (&x)[1]) {
+#pragma unroll
+        for (int q = 0; q < DIM; q++) g[q] = MGM_ADD(g[q], MGM_MUL(w[q], x[0]));
+    });
+    a.dpdx[i] = g[0];
+    a.dpdy[i] = g[1];
+    if constexpr (DIM == 3) a.dpdz[i] = g[2];
+    if constexpr (UPDATE) {
+        double p = a.p_old[i];
+        if (!a.btag[i]) {
+            a.u_new[i] = MGM_SUB(a.u_new[i], MGM_DIV(MGM_MUL(a.dt, g[0]), a.rho));
+            a.v_new[i] = MGM_SUB(a.v_new[i], MGM_DIV(MGM_MUL(a.dt, g[1]), a.rho));
+            if constexpr (DIM == 3) a.w_new[i] = MGM_SUB(a.w_new[i], MGM_DIV(MGM_MUL(a.dt, g[2]), a.rho));
+            p = MGM_ADD(p, MGM_MUL(1.0, f[i]));
+            a.p_old[i] = p;
+        }
+        if (i == 0) *pref = p;
+    }
 }
 
-// update_velocity_implicit (:351-363): interior velocities and pressure
+// calculate_mass_residual_implicit (:177-201): the components' own derivatives,
+// then the source from the divergence (dpdz is 0 in 2D: never written there, as
+// in the reference)
 template <int DIM>
-__global__ void k_t_update(TimpleArgs a)
+__global__ void __launch_bounds__(128) k_t_mass(TimpleArgs a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n || a.btag[i]) return;
-    a.u_new[i] = MGM_SUB(a.u_new[i], MGM_DIV(MGM_MUL(a.dt, a.dpdx[i]), a.rho));
-    a.v_new[i] = MGM_SUB(a.v_new[i], MGM_DIV(MGM_MUL(a.dt, a.dpdy[i]), a.rho));
-    if (DIM == 3) a.w_new[i] = MGM_SUB(a.w_new[i], MGM_DIV(MGM_MUL(a.dt, a.dpdz[i]), a.rho));
-    a.p_old[i] = MGM_ADD(a.p_old[i], MGM_MUL(1.0, a.pprime[i]));
+    if (i >= a.n) return;
+    double g[DIM] = {};
+    TimpleRow<DIM> R;
+    R.W[0] = a.Dx;
+    R.W[1] = a.Dy;
+    const double *xs[DIM];
+    xs[0] = a.u_new;
+    xs[1] = a.v_new;
+    if constexpr (DIM == 3) { R.W[2] = a.Dz; xs[2] = a.w_new; }
+    R.template run<DIM>(a, i, 0, xs, [&](const double (&w)[DIM], const double (&x)[DIM]) {
+#pragma unroll
+        for (int q = 0; q < DIM; q++) g[q] = MGM_ADD(g[q], MGM_MUL(w[q], x[q]));
+    });
+    a.dpdx[i] = g[0];
+    a.dpdy[i] = g[1];
+    double gz;
+    if constexpr (DIM == 3) a.dpdz[i] = gz = g[2];
+    else gz = a.dpdz[i];
+    a.source[i] = a.btag[i] ? 0.0 : MGM_DIV(MGM_MUL(a.rho, MGM_ADD(MGM_ADD(g[0], g[1]), gz)), a.dt);
 }
 
-// p_old -= p_old[0] (:364-368): the reference value is taken first
-__global__ void k_t_take(const double *p, double *out) { *out = p[0]; }
+// p_old -= p_old[0] (:364-368), the reference value as k_t_gradient left it
 __global__ void k_t_shift(int n, double *p, const double *pref)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -184,13 +263,16 @@ __global__ void k_t_bnd_pressure(TimpleArgs a)
         MGM_MUL(a.rho, MGM_ADD(MGM_ADD(MGM_MUL(temp1, nxi), MGM_MUL(temp2, nyi)), MGM_MUL(temp3, nzi)));
     a.dpdn[i] = dpdn;
     double sumx = 0, sumy = 0, sumz = 0, Ap = 0.0;
-    for (int j = 1; j < k; j++) {
-        const long o = (long)j * n + i;
-        const double pc = a.p_old[a.idx[o]];
-        sumx = MGM_ADD(sumx, MGM_MUL(a.Dx[o], pc));
-        sumy = MGM_ADD(sumy, MGM_MUL(a.Dy[o], pc));
-        if (DIM == 3) sumz = MGM_ADD(sumz, MGM_MUL(a.Dz[o], pc));
-    }
+    TimpleRow<DIM> R;
+    R.W[0] = a.Dx;
+    R.W[1] = a.Dy;
+    if constexpr (DIM == 3) R.W[2] = a.Dz;
+    const double *const xs[1] = {a.p_old};
+    R.template run<1>(a, i, 1, xs, [&](const double (&w)[DIM], const double (&x)[1]) {
+        sumx = MGM_ADD(sumx, MGM_MUL(w[0], x[0]));
+        sumy = MGM_ADD(sumy, MGM_MUL(w[1], x[0]));
+        if constexpr (DIM == 3) sumz = MGM_ADD(sumz, MGM_MUL(w[2], x[0]));
+    });
     Ap = MGM_ADD(Ap, MGM_MUL(a.Dx[i], nxi));
     Ap = MGM_ADD(Ap, MGM_MUL(a.Dy[i], nyi));
     if (DIM == 3) Ap = MGM_ADD(Ap, MGM_MUL(a.Dz[i], nzi));
@@ -222,11 +304,21 @@ __global__ void k_t_steady(TimpleArgs a, double *partial)
     if (threadIdx.x == 0) partial[blockIdx.x] = sm[0];
 }
 
-__global__ void k_t_steady_finish(const double *partial, int nparts, int n, double *out)
+// the partials through shared memory, added in order by one thread (straight
+// from global memory 1000 of them took 38 us)
+__global__ void __launch_bounds__(256) k_t_steady_finish(const double *partial, int nparts, int n, double *out)
 {
+    __shared__ double sm[2048];
     double s = 0.0;
-    for (int t = 0; t < nparts; t++) s += partial[t];
-    *out = sqrt(s / n);
+    for (int t0 = 0; t0 < nparts; t0 += 2048) {
+        const int m = min(2048, nparts - t0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < m; t += 256) sm[t] = partial[t0 + t];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int t = 0; t < m; t++) s += sm[t];
+    }
+    if (threadIdx.x == 0) *out = sqrt(s / n);
 }
 
 TimpleArgs timple_args(mgm_ctx *c)
@@ -251,16 +343,15 @@ TimpleArgs timple_args(mgm_ctx *c)
 static void timple_momentum(mgm_ctx *c)
 {
     cudaStream_t s = c->s;
-    Level &L = c->L[0];
-    const int n = L.n, k = L.k, dim = c->dim, nb = blocks_for(n, 256);
+    const int n = c->L[0].n, dim = c->dim, nb = blocks_for(n, 128);
     TimpleArgs a = timple_args(c);
-    spmv_parity(n, k, L.Dx.p, L.idx.p, c->p_old.p, c->dpdx.p, s);
-    spmv_parity(n, k, L.Dy.p, L.idx.p, c->p_old.p, c->dpdy.p, s);
-    if (dim == 3) spmv_parity(n, k, L.Dz.p, L.idx.p, c->p_old.p, c->dpdz.p, s);
+    if (dim == 3) k_t_gradient<3, false><<<nb, 128, 0, s>>>(a, c->p_old.p, nullptr);
+    else k_t_gradient<2, false><<<nb, 128, 0, s>>>(a, c->p_old.p, nullptr);
+    MGM_LAUNCHED();
     double *in[3] = {c->u_new.p, c->v_new.p, c->w_new.p}, *out[3] = {c->tu.p, c->tv.p, c->tw.p};
     for (int sw = 0; sw < c->iter_momentum; sw++) {
-        if (dim == 3) k_t_momentum<3><<<nb, 256, 0, s>>>(a, in[0], in[1], in[2], out[0], out[1], out[2]);
-        else k_t_momentum<2><<<nb, 256, 0, s>>>(a, in[0], in[1], in[2], out[0], out[1], out[2]);
+        if (dim == 3) k_t_momentum<3><<<nb, 128, 0, s>>>(a, in[0], in[1], in[2], out[0], out[1], out[2]);
+        else k_t_momentum<2><<<nb, 128, 0, s>>>(a, in[0], in[1], in[2], out[0], out[1], out[2]);
         MGM_LAUNCHED();
         for (int q = 0; q < 3; q++) std::swap(in[q], out[q]);
     }
@@ -274,13 +365,9 @@ static void timple_momentum(mgm_ctx *c)
 // calculate_mass_residual_implicit (:177-201)
 static void timple_mass(mgm_ctx *c)
 {
-    cudaStream_t s = c->s;
-    Level &L = c->L[0];
-    const int n = L.n, k = L.k;
-    spmv_parity(n, k, L.Dx.p, L.idx.p, c->u_new.p, c->dpdx.p, s);
-    spmv_parity(n, k, L.Dy.p, L.idx.p, c->v_new.p, c->dpdy.p, s);
-    if (c->dim == 3) spmv_parity(n, k, L.Dz.p, L.idx.p, c->w_new.p, c->dpdz.p, s);
-    k_t_source<<<blocks_for(n, 256), 256, 0, s>>>(timple_args(c));
+    const int nb = blocks_for(c->L[0].n, 128);
+    if (c->dim == 3) k_t_mass<3><<<nb, 128, 0, c->s>>>(timple_args(c));
+    else k_t_mass<2><<<nb, 128, 0, c->s>>>(timple_args(c));
     MGM_LAUNCHED();
 }
 
@@ -289,14 +376,9 @@ static void timple_update(mgm_ctx *c)
 {
     cudaStream_t s = c->s;
     Level &L = c->L[0];
-    const int n = L.n, k = L.k, nb = blocks_for(n, 256);
-    spmv_parity(n, k, L.Dx.p, L.idx.p, L.p.p, c->dpdx.p, s);
-    spmv_parity(n, k, L.Dy.p, L.idx.p, L.p.p, c->dpdy.p, s);
-    if (c->dim == 3) spmv_parity(n, k, L.Dz.p, L.idx.p, L.p.p, c->dpdz.p, s);
-    if (c->dim == 3) k_t_update<3><<<nb, 256, 0, s>>>(timple_args(c));
-    else k_t_update<2><<<nb, 256, 0, s>>>(timple_args(c));
-    MGM_LAUNCHED();
-    k_t_take<<<1, 1, 0, s>>>(c->p_old.p, c->scal.p);
+    const int n = L.n, nb = blocks_for(n, 256), nr = blocks_for(n, 128);
+    if (c->dim == 3) k_t_gradient<3, true><<<nr, 128, 0, s>>>(timple_args(c), L.p.p, c->scal.p);
+    else k_t_gradient<2, true><<<nr, 128, 0, s>>>(timple_args(c), L.p.p, c->scal.p);
     MGM_LAUNCHED();
     k_t_shift<<<nb, 256, 0, s>>>(n, c->p_old.p, c->scal.p);
     MGM_LAUNCHED();
@@ -320,8 +402,10 @@ double timple_step(mgm_ctx *c, int mode)
     k_t_begin<<<nb, 256, 0, s>>>(a);
     MGM_LAUNCHED();
     for (int it = 0; it < c->iter_timple; it++) {
-        k_t_iter<<<nb, 256, 0, s>>>(a);
-        MGM_LAUNCHED();
+        if (it > 0) {  // the first iteration's state is k_t_begin's
+            k_t_iter<<<nb, 256, 0, s>>>(a);
+            MGM_LAUNCHED();
+        }
         timple_momentum(c);
         timple_mass(c);
         poisson_solve(c, mode, true);  // the pressure-correction equation, on p' (L.p)
@@ -332,7 +416,7 @@ double timple_step(mgm_ctx *c, int mode)
     if (c->dim == 3) k_t_steady<3><<<nb, 256, 0, s>>>(a, c->partial.p);
     else k_t_steady<2><<<nb, 256, 0, s>>>(a, c->partial.p);
     MGM_LAUNCHED();
-    k_t_steady_finish<<<1, 1, 0, s>>>(c->partial.p, nb, n, c->scal.p + 1);
+    k_t_steady_finish<<<1, 256, 0, s>>>(c->partial.p, nb, n, c->scal.p + 1);
     MGM_LAUNCHED();
     double e = 0;
     MGM_CUDA(cudaMemcpyAsync(&e, c->scal.p + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
