@@ -21,6 +21,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "ctx.cuh"
 
@@ -48,7 +49,7 @@ struct MpnnState {
     DBuf<bf16> h[kLayers + 1];
     DBuf<bf16> cat[kLayers];
     DBuf<float> z[kLayers + 1];
-    DBuf<float> y, dy, dH, dHin, dz, dm;
+    DBuf<float> y, dy, dH, dz;
     DBuf<double> scal;       // device scalars: [0..1] sum of squares of b, p; [2] loss; [5] of dp
     DBuf<float> ds;          // dataset: cap samples x kSlot x n (b_hat, p_hat, dp_hat, target)
     DBuf<double> dp;         // p_prev - p_prev2 of the sample being recorded
@@ -394,145 +395,353 @@ __global__ void k_loss(int n, const float *y, const float *t, float *dy, double 
     if (threadIdx.x == 0) atomicAdd(loss, s / n);
 }
 
-// dH4 = dy w_d ; grads of w_d, c_d (warp per node, grid-stride, one atomic per lane at the end)
-__global__ void __launch_bounds__(256) k_decode_bwd(int n, const bf16 *h, const float *dy, const float *P, float *dH,
-                                                    float *G)
+// The sum of NV values per lane over the CTA's 8 warps, one atomic per value:
+// out[v] of lane l to dst(v, l).  (One atomic per warp put 4700 on each address:
+// 83 us of k_encode_bwd at 90k nodes, now 24.)
+template <int NV, class D>
+__device__ __forceinline__ void cta_atomic(const float (&v)[NV], D dst)
+{
+    __shared__ float sm[8][NV][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NV; q++) sm[w][q][lane] = v[q];
+    __syncthreads();
+    for (int e = threadIdx.x; e < NV * 32; e += 256) {
+        float s = 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u++) s += sm[u][e / 32][e % 32];
+        atomicAdd(dst(e / 32, e % 32), s);
+    }
+}
+
+// dH4 = dy w_d ; grads of w_d, c_d (warp per node, grid-stride)
+__global__ void __launch_bounds__(256) k_decode_bwd(int n, const bf16 *__restrict__ h, const float *__restrict__ dy,
+                                                    const float *__restrict__ P, float *__restrict__ dH, float *G)
 {
     const int lane = threadIdx.x & 31;
     const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-    float gw0 = 0, gw1 = 0, gc = 0;
+    float g[3] = {};
     const float w0 = P[P_WD + 2 * lane], w1 = P[P_WD + 2 * lane + 1];
+#pragma unroll 4
     for (long i = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += nw) {
         const float d = dy[i];
         const float2 v = ld_bf2(h + i * kH + 2 * lane);
-        gw0 += v.x * d; gw1 += v.y * d;
-        gc += d;
-        dH[i * kH + 2 * lane] = d * w0;
-        dH[i * kH + 2 * lane + 1] = d * w1;
+        g[0] += v.x * d;
+        g[1] += v.y * d;
+        g[2] += d;
+        *reinterpret_cast<float2 *>(dH + i * kH + 2 * lane) = make_float2(d * w0, d * w1);
     }
-    atomicAdd(&G[P_WD + 2 * lane], gw0);
-    atomicAdd(&G[P_WD + 2 * lane + 1], gw1);
-    if (lane == 0) atomicAdd(&G[P_CD], gc);
+    if (lane > 0) g[2] = 0.f;  // every lane has the node's d
+    cta_atomic<3>(g, [&](int q, int l) { return q < 2 ? &G[P_WD + 2 * l + q] : &G[P_CD]; });
 }
 
-// dz = dH * [z > 0] ; dHin = dH (residual path) ; bias grads
-__global__ void __launch_bounds__(256) k_relu_bwd(int n, const float *dH, const float *z, float *dz, float *dHin,
-                                                  float *gbias)
+// Backward pass of a layer on the tensor cores.  The activations and weights
+// are BF16; the FP32 gradients dz enter as three BF16 parts whose sum is the
+// FP32 value (8 significand bits each), so every product is exact and the
+// FP32 accumulation is the only rounding, as it was with FP32 multiply-adds on
+// the CUDA cores.  The small parts are accumulated before the large one, and a
+// tile's sums start from zero and are added to the running FP32 sums, which
+// keeps the tensor cores' truncating accumulation to 4 steps at full size.
+__device__ __forceinline__ void split3(float2 v, uint32_t (&p)[3])
 {
-    const int lane = threadIdx.x & 31;
-    const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-    float g0 = 0, g1 = 0;
-    for (long i = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += nw) {
-        const long o = i * kH + 2 * lane;
-        const float d0 = z[o] > 0.f ? dH[o] : 0.f, d1 = z[o + 1] > 0.f ? dH[o + 1] : 0.f;
-        dz[o] = d0; dz[o + 1] = d1;
-        if (dHin) { dHin[o] = dH[o]; dHin[o + 1] = dH[o + 1]; }
-        g0 += d0; g1 += d1;
-    }
-    atomicAdd(&gbias[2 * lane], g0);
-    atomicAdd(&gbias[2 * lane + 1], g1);
-}
-
-// gW[kk][f] += sum_i cat[i][kk] dz[i][f]  (thread kk, 64 accumulators; node chunks per CTA)
-__global__ void __launch_bounds__(192) k_dW(int n, int chunk, const bf16 *cat, const float *dz, float *gW)
-{
-    __shared__ float dzs[16][kH];
-    const int kk = threadIdx.x;
-    const long i0 = (long)blockIdx.x * chunk, i1 = min((long)n, i0 + chunk);
-    float acc[kH];
 #pragma unroll
-    for (int f = 0; f < kH; f++) acc[f] = 0.f;
-    for (long ib = i0; ib < i1; ib += 16) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < 16 * kH; e += blockDim.x) {
-            const long i = ib + e / kH;
-            dzs[e / kH][e % kH] = i < i1 ? dz[i * kH + e % kH] : 0.f;
-        }
-        __syncthreads();
-        const int m = (int)min(16L, i1 - ib);
-        for (int q = 0; q < m; q++) {
-            const float a = __bfloat162float(cat[(ib + q) * kCat + kk]);
-#pragma unroll
-            for (int f = 0; f < kH; f++) acc[f] += a * dzs[q][f];
-        }
-    }
-#pragma unroll
-    for (int f = 0; f < kH; f++) atomicAdd(&gW[kk * kH + f], acc[f]);
-}
-
-// dcat = dz W^T: self part added to dHin, mean/lap parts into dm [n][128]
-__global__ void __launch_bounds__(192) k_dcat(int n, const float *dz, const bf16 *WT, float *dHin, float *dm)
-{
-    __shared__ bf16 Wsh[kCat][kH + 2];
-    __shared__ float dzs[16][kH];
-    const int kk = threadIdx.x;
-    for (int e = threadIdx.x; e < kCat * kH; e += blockDim.x) {
-        const int f = e / kCat, c = e % kCat;  // WT is [64][192]
-        Wsh[c][f] = WT[e];
-    }
-    for (long ib = (long)blockIdx.x * 16; ib < n; ib += (long)gridDim.x * 16) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < 16 * kH; e += blockDim.x) {
-            const long i = ib + e / kH;
-            dzs[e / kH][e % kH] = i < n ? dz[i * kH + e % kH] : 0.f;
-        }
-        __syncthreads();
-        for (int q = 0; q < 16; q++) {
-            const long i = ib + q;
-            if (i >= n) break;
-            float s = 0.f;
-#pragma unroll 16
-            for (int f = 0; f < kH; f++) s += dzs[q][f] * __bfloat162float(Wsh[kk][f]);
-            if (kk < kH) dHin[i * kH + kk] += s;
-            else dm[i * 128 + (kk - kH)] = s;
-        }
+    for (int q = 0; q < 3; q++) {
+        const __nv_bfloat162 b = __floats2bfloat162_rn(v.x, v.y);
+        const float2 f = __bfloat1622float2(b);
+        p[q] = *reinterpret_cast<const uint32_t *>(&b);
+        v.x -= f.x;
+        v.y -= f.y;
     }
 }
 
-// dHin[j] += sum over in-edges (i, l_ij): dm_mean[i] / k + l_ij dm_lap[i]
-__global__ void __launch_bounds__(256) k_scatter_T(int n, int k, float inv_k, const int *tptr, const int *tpos,
-                                                   const float *lapS, const float *dm, float *dHin)
+__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3)
 {
-    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (j >= n) return;
-    float a0 = 0, a1 = 0;
-    for (int e = tptr[j]; e < tptr[j + 1]; e++) {
-        const int pos = tpos[e];
-        const long i = pos / k;
-        const float w = lapS[pos];
-        const float *r = dm + i * 128;
-        a0 += inv_k * r[2 * lane] + w * r[kH + 2 * lane];
-        a1 += inv_k * r[2 * lane + 1] + w * r[kH + 2 * lane + 1];
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"(addr));
+}
+
+constexpr int kPadH = kH + 8;  // padded row (bf16) of a 64-column tile: 144 bytes, no bank conflicts in ldmatrix
+constexpr int kDwThreads = 512;
+constexpr size_t kDwSmem = sizeof(bf16) * (size_t)kTile * (kPad + 3 * kPadH);
+
+// dz = dH * [z > 0], its bias sums, and gW[kk][f] += sum_i cat[i][kk] dz[i][f].
+// One CTA per SM over tiles of 64 nodes, the next tile's loads in flight during
+// the products; a warp owns 48 x 16 of the 192 x 64 sums.  Bound by the reads
+// of dH, z and cat and the write of dz: 104 MB in 30 us at 90k nodes (on the CUDA
+// cores, with a pass of its own for dz, 350 us).  Against 64-bit sums its error is
+// half that of the FP32 multiply-adds (2.4e-7 against 4.7e-7).
+__global__ void __launch_bounds__(kDwThreads, 1) k_dW(int n, const float *__restrict__ dH, const float *__restrict__ z,
+                                                      const bf16 *__restrict__ cat, float *__restrict__ dz,
+                                                      float *__restrict__ gbias, float *__restrict__ gW)
+{
+    extern __shared__ __align__(16) unsigned char dw_smem[];
+    bf16 *const Cs = reinterpret_cast<bf16 *>(dw_smem);  // [64][kPad]
+    bf16 *const Ds = Cs + kTile * kPad;                  // [3][64][kPadH]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane >> 3, rq = lane & 7;
+    const int row0 = tid >> 4, c4 = (tid & 15) * 4;  // dH, z: rows row0, row0 + 32, columns c4..c4+3
+    float4 h[2], zz[2];
+    uint4 ct[3];
+    auto fetch = [&](long base) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const long i = base + row0 + 32 * u;
+            h[u] = zz[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < n) {
+                h[u] = __ldg(reinterpret_cast<const float4 *>(dH + i * kH + c4));
+                zz[u] = __ldg(reinterpret_cast<const float4 *>(z + i * kH + c4));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+            const int e = tid + u * kDwThreads;
+            const long i = base + e / (kCat / 8);
+            ct[u] = i < n ? __ldg(reinterpret_cast<const uint4 *>(cat + i * kCat) + e % (kCat / 8))
+                          : make_uint4(0, 0, 0, 0);
+        }
+    };
+    float sum[3][2][4] = {}, gb[4] = {};
+    const int m0 = (warp >> 2) * 48, n0 = (warp & 3) * 16;
+    // A = cat^T, B = dz, both stored [node][...]: transposing loads
+    const uint32_t a_addr =
+        (uint32_t)__cvta_generic_to_shared(Cs + (rq + 8 * (q >> 1)) * kPad + m0 + 8 * (q & 1));
+    const uint32_t b_addr =
+        (uint32_t)__cvta_generic_to_shared(Ds + (rq + 8 * (q & 1)) * kPadH + n0 + 8 * (q >> 1));
+    fetch((long)blockIdx.x * kTile);
+    for (long base = (long)blockIdx.x * kTile; base < n; base += (long)gridDim.x * kTile) {
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int row = row0 + 32 * u;
+            const float4 d = make_float4(zz[u].x > 0.f ? h[u].x : 0.f, zz[u].y > 0.f ? h[u].y : 0.f,
+                                         zz[u].z > 0.f ? h[u].z : 0.f, zz[u].w > 0.f ? h[u].w : 0.f);
+            gb[0] += d.x; gb[1] += d.y; gb[2] += d.z; gb[3] += d.w;
+            if (base + row < n) *reinterpret_cast<float4 *>(dz + (base + row) * kH + c4) = d;
+            uint32_t lo[3], hi[3];
+            split3(make_float2(d.x, d.y), lo);
+            split3(make_float2(d.z, d.w), hi);
+#pragma unroll
+            for (int p = 0; p < 3; p++)
+                *reinterpret_cast<uint2 *>(Ds + (p * kTile + row) * kPadH + c4) = make_uint2(lo[p], hi[p]);
+        }
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+            const int e = tid + u * kDwThreads;
+            *reinterpret_cast<uint4 *>(Cs + (e / (kCat / 8)) * kPad + 8 * (e % (kCat / 8))) = ct[u];
+        }
+        __syncthreads();
+        const long next = base + (long)gridDim.x * kTile;
+        if (next < n) fetch(next);
+        float acc[3][2][4] = {};
+        auto products = [&](int ks, auto FIRST, auto LAST) {  // parts FIRST, FIRST - 1, .. LAST
+            uint32_t a[3][4];
+#pragma unroll
+            for (int m = 0; m < 3; m++)
+                ldsm_x4_t(a_addr + (ks * 16 * kPad + m * 16) * (uint32_t)sizeof(bf16), a[m][0], a[m][1], a[m][2],
+                          a[m][3]);
+#pragma unroll
+            for (int p = decltype(FIRST)::value; p >= decltype(LAST)::value; p--) {
+                uint32_t b[4];
+                ldsm_x4_t(b_addr + (p * kTile + ks * 16) * kPadH * (uint32_t)sizeof(bf16), b[0], b[1], b[2], b[3]);
+#pragma unroll
+                for (int m = 0; m < 3; m++) {
+                    mma_bf16(acc[m][0], a[m][0], a[m][1], a[m][2], a[m][3], b[0], b[1]);
+                    mma_bf16(acc[m][1], a[m][0], a[m][1], a[m][2], a[m][3], b[2], b[3]);
+                }
+            }
+        };
+        // the two small parts, then the large one
+#pragma unroll 1
+        for (int ks = 0; ks < kTile / 16; ks++)
+            products(ks, std::integral_constant<int, 2>{}, std::integral_constant<int, 1>{});
+#pragma unroll 1
+        for (int ks = 0; ks < kTile / 16; ks++)
+            products(ks, std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{});
+#pragma unroll
+        for (int m = 0; m < 3; m++)
+#pragma unroll
+            for (int t = 0; t < 2; t++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) sum[m][t][e] += acc[m][t][e];
     }
-    dHin[(long)j * kH + 2 * lane] += a0;
-    dHin[(long)j * kH + 2 * lane + 1] += a1;
+    const int g = lane >> 2, t2 = 2 * (lane & 3);
+#pragma unroll
+    for (int m = 0; m < 3; m++)
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+#pragma unroll
+            for (int hh = 0; hh < 2; hh++)
+                atomicAdd(reinterpret_cast<float2 *>(gW + (m0 + m * 16 + g + 8 * hh) * kH + n0 + t * 8 + t2),
+                          make_float2(sum[m][t][2 * hh], sum[m][t][2 * hh + 1]));
+    // bias: the 32 threads of a column group through shared memory
+    __syncthreads();
+    float *const gs = reinterpret_cast<float *>(dw_smem);
+#pragma unroll
+    for (int e = 0; e < 4; e++) gs[row0 * kH + c4 + e] = gb[e];
+    __syncthreads();
+    if (tid < kH) {
+        float v = 0.f;
+        for (int r = 0; r < 32; r++) v += gs[r * kH + tid];
+        atomicAdd(&gbias[tid], v);
+    }
+}
+
+constexpr size_t kBackSmem = sizeof(bf16) * (size_t)(3 * kTile * kPadH + kH * kPad);
+
+// dH[j] += dz[j] W_self^T + (sum_e dz[i] / k) W_mean^T + (sum_e l_ij dz[i]) W_lap^T
+// over the in-edges e = (i, l_ij) of node j.  The sums are taken over dz (64
+// features a node) before the products: after them the edges would gather the
+// 128 products of a node, twice the bytes (products 245 us, scatter 130 at 90k
+// nodes of 30 slots; now 98 together, 7 TB/s of gathers).  64 nodes per CTA; a warp
+// gathers two at a time, four features a lane, 8 rows each in flight, and owns 16 x 32 of
+// the 64 x 64 outputs.
+__global__ void __launch_bounds__(256, 2) k_back(int n, int k, float inv_k, const int *__restrict__ tptr,
+                                                 const int *__restrict__ tpos, const float *__restrict__ lapS,
+                                                 const float *__restrict__ dz, const bf16 *__restrict__ WT,
+                                                 float *__restrict__ dH)
+{
+    extern __shared__ __align__(16) unsigned char back_smem[];
+    bf16 *const Xs = reinterpret_cast<bf16 *>(back_smem);  // [3][64][kPadH]: dz, mean or lap in three parts
+    bf16 *const Ws = Xs + 3 * kTile * kPadH;               // [64][kPad]: W^T
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane >> 3, rq = lane & 7;
+    const long base = (long)blockIdx.x * kTile;
+    const unsigned full = 0xffffffffu;
+    for (int e = tid; e < kH * (kCat / 8); e += 256)
+        *reinterpret_cast<uint4 *>(Ws + (e / (kCat / 8)) * kPad + 8 * (e % (kCat / 8))) =
+            __ldg(reinterpret_cast<const uint4 *>(WT) + e);
+    const int half = lane >> 4, hl = lane & 15;
+    float4 S[kTile / 16][3];
+#pragma unroll
+    for (int rr = 0; rr < kTile / 16; rr++) {
+        const int row = warp * (kTile / 8) + rr * 2 + half;
+        const long j = base + row;
+        float4 own = make_float4(0.f, 0.f, 0.f, 0.f), s1 = own, s2 = own;
+        int e0 = 0, e1 = 0;
+        if (j < n) {
+            own = __ldg(reinterpret_cast<const float4 *>(dz + j * kH) + hl);
+            e0 = __ldg(tptr + j);
+            e1 = __ldg(tptr + j + 1);
+        }
+        for (int left = __reduce_max_sync(full, e1 - e0); left > 0; left -= 16, e0 += 16) {
+            int src = 0;
+            float w = 0.f;
+            if (e0 + hl < e1) {
+                const int pos = __ldg(tpos + e0 + hl);
+                src = pos / k;
+                w = __ldg(lapS + pos);
+            }
+#pragma unroll
+            for (int t = 0; t < 16; t += 8) {
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const int c = __shfl_sync(full, src, t + u, 16);
+                    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (e0 + t + u < e1) v[u] = __ldg(reinterpret_cast<const float4 *>(dz + (long)c * kH) + hl);
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const float wu = __shfl_sync(full, w, t + u, 16);
+                    s1.x += v[u].x;
+                    s1.y += v[u].y;
+                    s1.z += v[u].z;
+                    s1.w += v[u].w;
+                    s2.x += wu * v[u].x;
+                    s2.y += wu * v[u].y;
+                    s2.z += wu * v[u].z;
+                    s2.w += wu * v[u].w;
+                }
+            }
+        }
+        S[rr][0] = own;
+        S[rr][1] = make_float4(s1.x * inv_k, s1.y * inv_k, s1.z * inv_k, s1.w * inv_k);
+        S[rr][2] = s2;
+    }
+    const int r0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
+    const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(Xs + (r0 + rq + 8 * (q & 1)) * kPadH + 8 * (q >> 1));
+    const uint32_t b_addr = (uint32_t)__cvta_generic_to_shared(Ws + (rq + 8 * (q & 1)) * kPad + n0 + 8 * (q >> 1));
+    float sum[4][4] = {};
+#pragma unroll
+    for (int part = 0; part < 3; part++) {  // self, mean, lap
+        __syncthreads();
+#pragma unroll
+        for (int rr = 0; rr < kTile / 16; rr++) {
+            const int row = warp * (kTile / 8) + rr * 2 + half;
+            const float4 f = S[rr][part];
+            uint32_t a[3], b[3];
+            split3(make_float2(f.x, f.y), a);
+            split3(make_float2(f.z, f.w), b);
+#pragma unroll
+            for (int p = 0; p < 3; p++)
+                *reinterpret_cast<uint2 *>(Xs + (p * kTile + row) * kPadH + 4 * hl) = make_uint2(a[p], b[p]);
+        }
+        __syncthreads();
+        float acc[4][4] = {};
+#pragma unroll
+        for (int big = 0; big < 2; big++)
+#pragma unroll
+            for (int ks = 0; ks < kH / 16; ks++) {
+                uint32_t b[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    ldsm_x4_t(b_addr + (ks * 16 * kPad + part * kH + h * 16) * (uint32_t)sizeof(bf16), b[h][0], b[h][1],
+                              b[h][2], b[h][3]);
+#pragma unroll
+                for (int p = big ? 0 : 2; p >= (big ? 0 : 1); p--) {
+                    uint32_t a0, a1, a2, a3;
+                    ldsm_x4(a_addr + (p * kTile * kPadH + ks * 16) * (uint32_t)sizeof(bf16), a0, a1, a2, a3);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        mma_bf16(acc[2 * h], a0, a1, a2, a3, b[h][0], b[h][1]);
+                        mma_bf16(acc[2 * h + 1], a0, a1, a2, a3, b[h][2], b[h][3]);
+                    }
+                }
+            }
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) sum[t][e] += acc[t][e];
+    }
+    const int g = lane >> 2, t2 = 2 * (lane & 3);
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+            const long i = base + r0 + g + 8 * hh;
+            if (i >= n) continue;
+            float2 *const o = reinterpret_cast<float2 *>(dH + i * kH + n0 + t * 8 + t2);
+            float2 v = *o;
+            v.x += sum[t][2 * hh];
+            v.y += sum[t][2 * hh + 1];
+            *o = v;
+        }
 }
 
 // encoder grads
-__global__ void __launch_bounds__(256) k_encode_bwd(int n, const float *feat, const float *z0, const float *dH,
+__global__ void __launch_bounds__(256) k_encode_bwd(int n, const float *__restrict__ feat,
+                                                    const float *__restrict__ z0, const float *__restrict__ dH,
                                                     float *G)
 {
     const int lane = threadIdx.x & 31;
     const long nw = ((long)gridDim.x * blockDim.x) >> 5;
-    float gw[kFin][2] = {}, gc0 = 0, gc1 = 0;
+    float g[2 * kFin + 2] = {};
+#pragma unroll 4
     for (long i = (((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += nw) {
-        const long o = i * kH + 2 * lane;
-        const float d0 = z0[o] > 0.f ? dH[o] : 0.f, d1 = z0[o + 1] > 0.f ? dH[o + 1] : 0.f;
+        const float2 zv = __ldg(reinterpret_cast<const float2 *>(z0 + i * kH) + lane);
+        const float2 hv = __ldg(reinterpret_cast<const float2 *>(dH + i * kH) + lane);
+        const float d0 = zv.x > 0.f ? hv.x : 0.f, d1 = zv.y > 0.f ? hv.y : 0.f;
 #pragma unroll
         for (int q = 0; q < kFin; q++) {
-            const float xv = feat[i * kFin + q];
-            gw[q][0] += xv * d0;
-            gw[q][1] += xv * d1;
+            const float xv = __ldg(feat + i * kFin + q);
+            g[2 * q] += xv * d0;
+            g[2 * q + 1] += xv * d1;
         }
-        gc0 += d0; gc1 += d1;
+        g[2 * kFin] += d0;
+        g[2 * kFin + 1] += d1;
     }
-#pragma unroll
-    for (int q = 0; q < kFin; q++) {
-        atomicAdd(&G[P_WE + q * kH + 2 * lane], gw[q][0]);
-        atomicAdd(&G[P_WE + q * kH + 2 * lane + 1], gw[q][1]);
-    }
-    atomicAdd(&G[P_CE + 2 * lane], gc0);
-    atomicAdd(&G[P_CE + 2 * lane + 1], gc1);
+    cta_atomic<2 * kFin + 2>(g, [&](int q, int l) {
+        return q < 2 * kFin ? &G[P_WE + (q / 2) * kH + 2 * l + (q & 1)] : &G[P_CE + 2 * l + (q & 1)];
+    });
 }
 
 __global__ void k_adam(int np, float *P, const float *G, float *m, float *v, float lr, float b1, float b2, float eps,
@@ -771,22 +980,21 @@ static void loss_and_grad(MpnnState &M, const float *t, cudaStream_t s)
     forward(M, true, s);
     loss_head(M, t, s);
     float *G = M.grads.p;
-    k_decode_bwd<<<red_blocks(n), 256, 0, s>>>(n, M.h[kLayers].p, M.dy.p, M.params.p, M.dH.p, G);
+    k_decode_bwd<<<std::min(blocks_for(n, 8), 148 * 4), 256, 0, s>>>(n, M.h[kLayers].p, M.dy.p, M.params.p, M.dH.p, G);
     MGM_LAUNCHED();
-    const int chunk = std::max(64, blocks_for(n, 148 * 4));
+    MGM_CUDA(cudaFuncSetAttribute(k_dW, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem));
+    MGM_CUDA(cudaFuncSetAttribute(k_back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBackSmem));
+    const int tiles = blocks_for(n, kTile);
     for (int l = kLayers - 1; l >= 0; l--) {
         float *gl = G + P_L0 + l * kLayerParams;
-        k_relu_bwd<<<red_blocks(n), 256, 0, s>>>(n, M.dH.p, M.z[l + 1].p, M.dz.p, M.dHin.p, gl + kCat * kH);
+        k_dW<<<std::min(tiles, 148), kDwThreads, kDwSmem, s>>>(n, M.dH.p, M.z[l + 1].p, M.cat[l].p, M.dz.p,
+                                                              gl + kCat * kH, gl);
         MGM_LAUNCHED();
-        k_dW<<<blocks_for(n, chunk), 192, 0, s>>>(n, chunk, M.cat[l].p, M.dz.p, gl);
+        k_back<<<tiles, 256, kBackSmem, s>>>(n, M.k, 1.f / M.k, M.tptr.p, M.tpos.p, M.lapS.p, M.dz.p, M.WT[l].p,
+                                             M.dH.p);
         MGM_LAUNCHED();
-        k_dcat<<<std::min(blocks_for(n, 16), 148 * 8), 192, 0, s>>>(n, M.dz.p, M.WT[l].p, M.dHin.p, M.dm.p);
-        MGM_LAUNCHED();
-        k_scatter_T<<<warp_blocks(n), 256, 0, s>>>(n, M.k, 1.f / M.k, M.tptr.p, M.tpos.p, M.lapS.p, M.dm.p, M.dHin.p);
-        MGM_LAUNCHED();
-        std::swap(M.dH.p, M.dHin.p);
     }
-    k_encode_bwd<<<red_blocks(n), 256, 0, s>>>(n, M.feat.p, M.z[0].p, M.dH.p, G);
+    k_encode_bwd<<<std::min(blocks_for(n, 8), 148 * 4), 256, 0, s>>>(n, M.feat.p, M.z[0].p, M.dH.p, G);
     MGM_LAUNCHED();
 }
 
@@ -942,8 +1150,7 @@ int mgm_mpnn_init(mgm_ctx *c, unsigned long long seed, int dataset_capacity)
         for (auto &h : M.h) h.alloc(n * kH);
         for (auto &ct : M.cat) ct.alloc(n * kCat);
         for (auto &z : M.z) z.alloc(n * kH);
-        M.y.alloc(n); M.dy.alloc(n); M.dH.alloc(n * kH); M.dHin.alloc(n * kH); M.dz.alloc(n * kH);
-        M.dm.alloc(n * 128);
+        M.y.alloc(n); M.dy.alloc(n); M.dH.alloc(n * kH); M.dz.alloc(n * kH);
         M.scal.alloc(8);
         M.dp.alloc(n);
         M.ds_cap = dataset_capacity;
