@@ -72,7 +72,7 @@ extern "C" int mgm_avg_dx_noalloc(int n, int k, int dim, const double *d_x, cons
         // every entry len[0..n) is written before it is read: nothing to clear
         k_spacing<<<blocks_for(n, 256), 256, 0, s>>>(n, k, dim, d_x, d_y, d_z, d_btag, d_cloud, len);
         MGM_LAUNCHED();
-        k_ordered_sum<<<1, 1, 0, s>>>(n, len, d_avg);
+        k_ordered_sum<<<1, 256, 0, s>>>(n, len, d_avg);
         MGM_LAUNCHED();
         return MGM_OK;
     } catch (const Error &e) {

@@ -17,6 +17,7 @@
 #include <cmath>
 
 #include "krylov.cuh"
+#include "coop.cuh"
 #include "rows.cuh"
 #include "stencil.cuh"
 
@@ -1202,42 +1203,6 @@ struct FusedArgs {
     FusedLevel<T> L[kFusedMaxLevels];
 };
 
-// Grid barrier of a cooperative launch (all CTAs resident): thread 0 of each
-// CTA arrives on a counter; the last arrival resets it and advances the
-// generation the others wait on (polled without sleeping: the wait is a few
-// microseconds).  The wait is bounded (2^20 polls of L2, under a second);
-// when it runs out the CTA records the error and the kernel's CTAs
-// return at their next barrier.  Returns false once any CTA has given up.
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned &gen)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int good = 1;
-        __threadfence();
-        const unsigned arrived = atomicAdd(&bar[0], 1u) + 1u;
-        if (arrived == gridDim.x) {
-            atomicExch(&bar[0], 0u);
-            __threadfence();
-            atomicAdd(&bar[1], 1u);
-        } else {
-            long spins = 0;
-            while (*(volatile unsigned *)&bar[1] == gen) {
-                if (++spins > (1L << 20) || ((spins & 255) == 0 && *(volatile int *)err)) {
-                    atomicExch(err, 1);
-                    good = 0;
-                    break;
-                }
-            }
-        }
-        __threadfence();
-        gen++;
-        ok = good && *(volatile int *)err == 0;
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 template <class T>
 __global__ void __launch_bounds__(kFusedThreads) k_coarse_vcycle(const __grid_constant__ FusedArgs<T> a)
 {
@@ -1411,16 +1376,7 @@ __global__ void k_barrier_selftest(unsigned *bar, int *err)
 }
 cudaError_t launch_barrier_selftest(cudaStream_t s, unsigned *bar, int *err)
 {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2);
-    cfg.blockDim = dim3(32);
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_barrier_selftest, bar, err);
+    return launch_cooperative(k_barrier_selftest, 2, 32, 0, s, bar, err);
 }
 
 // a cooperative launch of one CTA that does nothing (capture probe)
@@ -1699,20 +1655,37 @@ template void vcycle<float>(std::vector<SolveLevel<float>> &, const CoarseSolve<
 // ---------------------------------------------------------------------------
 // spectral radius of D^-1 A restricted to interior rows (power iteration)
 // ---------------------------------------------------------------------------
+// w = D^-1 A (v scale) with scale the previous step's 1 / |w| (null: 1)
 template <class T>
 __global__ void __launch_bounds__(256) k_power_step(int n, int k, const int *__restrict__ idx, const T *__restrict__ A,
                                                     const T *__restrict__ dinv, const uint8_t *__restrict__ btag,
-                                                    const double *__restrict__ v, double *__restrict__ w,
-                                                    double *__restrict__ partial)
+                                                    const double *__restrict__ v, const double *__restrict__ scale,
+                                                    double *__restrict__ w, double *__restrict__ partial)
 {
     __shared__ double sm[32];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double f = scale ? *scale : 1.0;
     double val = 0.0;
     if (i < n && !btag[i]) {
         double s = 0.0;
-        for (int j = 0; j < k; j++) {
+        int j = 0;
+        for (; j + 8 <= k; j += 8) {  // 8 slots' loads in flight, summed in slot order
+            int c[8];
+            double a[8], x[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const long o = (long)(j + q) * n + i;
+                c[q] = __ldg(idx + o);
+                a[q] = (double)__ldg(A + o);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[q] = __ldg(v + c[q]);
+#pragma unroll
+            for (int q = 0; q < 8; q++) s = fma(a[q], __dmul_rn(x[q], f), s);
+        }
+        for (; j < k; j++) {
             const long o = (long)j * n + i;
-            s += (double)A[o] * v[idx[o]];
+            s = fma((double)A[o], __dmul_rn(v[idx[o]], f), s);
         }
         val = (double)dinv[i] * s;
     }
@@ -1731,46 +1704,52 @@ __global__ void k_seed_vector(int n, const uint8_t *btag, double *v)
     v[i] = btag[i] ? 0.0 : ((double)(h & 0xffffff) / 16777216.0 - 0.5);
 }
 
-__global__ void k_scale(int n, double *v, const double *partial, int nparts)
+// The partials' sum in block order (through shared memory, added by one
+// thread): out[0] = 1 / sqrt(sum), out[1] = sqrt(sum)
+__global__ void __launch_bounds__(256) k_power_norm(const double *__restrict__ partial, int nparts, double *out)
 {
-    __shared__ double tot;
-    if (threadIdx.x == 0) {
-        double s = 0;
-        for (int t = 0; t < nparts; t++) s += partial[t];
-        tot = s > 0 ? 1.0 / sqrt(s) : 0.0;
+    __shared__ double sm[2048];
+    double s = 0;
+    for (int t0 = 0; t0 < nparts; t0 += 2048) {
+        const int m = min(2048, nparts - t0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < m; t += 256) sm[t] = partial[t0 + t];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int t = 0; t < m; t++) s += sm[t];
     }
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] *= tot;
+    if (threadIdx.x == 0) {
+        out[0] = s > 0 ? 1.0 / sqrt(s) : 0.0;
+        out[1] = sqrt(s);
+    }
 }
 
+// 40 steps without the host: the norm stays on the device and the next step
+// applies it (with a read of each step's partials 160 steps of four levels of up
+// to 250k rows took 10 ms, now 2.1)
 template <class T>
 void estimate_lmax(SolveLevel<T> &L, cudaStream_t s)
 {
     const int nb = blocks_for(L.n, 256);
-    DBuf<double> v(L.n), w(L.n), part(nb);
-    std::vector<double> hp(nb);
+    DBuf<double> v(L.n), w(L.n), part(nb), norm(2);
     k_seed_vector<<<nb, 256, 0, s>>>(L.n, L.btag, v.p);
     MGM_LAUNCHED();
-    double lam = 0;
-    for (int it = 0; it < 40; it++) {
-        // normalise v, apply, measure |w|
-        k_power_step<T><<<nb, 256, 0, s>>>(L.n, L.k, L.idx, L.A, L.dinv, L.btag, v.p, w.p, part.p);
+    constexpr int kSteps = 40;
+    for (int it = 0; it < kSteps; it++) {
+        k_power_step<T><<<nb, 256, 0, s>>>(L.n, L.k, L.idx, L.A, L.dinv, L.btag, v.p, it > 0 ? norm.p : nullptr, w.p,
+                                           part.p);
         MGM_LAUNCHED();
-        part.download(hp.data(), nb, s);
-        MGM_CUDA(cudaStreamSynchronize(s));
-        double sq = 0;
-        for (double x : hp) sq += x;
-        // |v| is 1 after the first normalisation
-        if (it > 0) lam = sqrt(sq);
-        k_scale<<<nb, 256, 0, s>>>(L.n, w.p, part.p, nb);
+        k_power_norm<<<1, 256, 0, s>>>(part.p, nb, norm.p);
         MGM_LAUNCHED();
         std::swap(v.p, w.p);
     }
+    double h[2];
+    norm.download(h, 2, s);
+    MGM_CUDA(cudaStreamSynchronize(s));
+    const double lam = h[1];  // |v| was 1 before the last step
     L.lmax = lam > 0 && std::isfinite(lam) ? lam : 2.0;
 }
 
 template void estimate_lmax<double>(SolveLevel<double> &, cudaStream_t);
-template void estimate_lmax<float>(SolveLevel<float> &, cudaStream_t);
 
 }  // namespace mgm
