@@ -10,20 +10,24 @@
 // with t_i = 0, so both lanes run the same instructions.  After every second
 // step the registers rotate by one (row l's result goes to register l - 1), so
 // the two pivot rows of a pair of steps are always register 0 and the loop
-// over the steps is not unrolled.  t is computed by the warp that holds column
-// i -- a reciprocal of the pivot and five operations per row -- right after its
-// own update, and read by all after the step's one barrier.
+// over the steps is not unrolled.  t is a reciprocal of the pivot and five
+// operations per row, longer than the update itself: above order 32 (reg_ahead)
+// a warp of its own takes column i + 1 as it was before step i, applies step i
+// to it and divides while the other warps are still in step i; below, the warp
+// that holds the column divides after its own update.  Either way all read t
+// after the step's one barrier.
 //
 // Work left out without changing a bit: the identity columns beyond the
 // stencil (never read), an identity column before its own row becomes the
 // pivot row (its entry in the pivot row is zero), the duplicate halves of the
 // symmetric RBF block, the scaling of the left half.
 //
-// Bound: latency at 25 warps per SM, then the shared-memory words of t (12
+// Bound: latency at 24 warps per SM, then the shared-memory words of t (12
 // broadcast 16-byte loads per 48 FP64 instructions of a warp).  Measured, 30
-// nodes with 15 monomials: 94 ns per system against 209 in shared memory (20
-// nodes with 10: 33 against 92); a whole column per thread (12 warps per SM)
-// 101 (39), two warps per 32 columns with t computed by every warp 113 (50).
+// nodes with 15 monomials: 76.5 ns per system against 209 in shared memory (20
+// nodes with 10: 34 against 92), 94 with the division after the update; a whole
+// column per thread (12 warps per SM) 101, two warps per 32 columns with t
+// computed by every warp 113.
 #include <algorithm>
 
 #include "mgm_internal.cuh"
@@ -72,28 +76,34 @@ __device__ __forceinline__ double div_by(double a, double b, double y, bool usab
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
-constexpr int reg_threads(int cols) { return (cols + 15) / 16 * 32; }
+// Orders above 32 give the division its own warp, which works a step ahead: 8
+// CTAs per SM hide the division's chain at order 30 (33.9 ns per system, 35.2
+// with the warp), 4 or fewer do not (order 35 54.9 -> 53.2, 45 88.0 -> 76.5, 53
+// 184 -> 160, 62 228 -> 183).
+constexpr bool reg_ahead(int NT) { return NT > 32; }
+// a warp per 16 columns, and the warp that divides
+constexpr int reg_threads(int NT, int cols) { return (cols + 15) / 16 * 32 + (reg_ahead(NT) ? 32 : 0); }
 
-// bytes of shared memory: L[4][NT] | col[NT] | t[2][NT] | diag, rdiag[NT] | A[N][N] | sx,sy,sz[m] |
+// bytes of shared memory: L[4][NT] | col[2][NT] | t[2][NT] | diag, rdiag[NT] | A[N][N] | sx,sy,sz[m] |
 // res[4][m] | pw[3][kRegPow][m], then perm[NT], pos[NT], use[NT] ints (NT a multiple of 4)
 inline size_t reg_smem_bytes(int N, int m, int NT)
 {
-    return sizeof(double) * (4 * NT + NT + 2 * NT + 2 * NT + (size_t)N * N + (3 + 4 + 3 * kRegPow) * m) +
+    return sizeof(double) * (4 * NT + 2 * NT + 2 * NT + 2 * NT + (size_t)N * N + (3 + 4 + 3 * kRegPow) * m) +
            sizeof(int) * 3 * NT;
 }
 
 // CTAs per SM the register budget is set for
-constexpr int reg_min_blocks(int NT) { return NT <= 32 ? 8 : (NT <= 48 ? 4 : 2); }
+constexpr int reg_min_blocks(int NT) { return NT <= 32 ? 8 : (NT <= 48 ? 3 : 2); }
 
 template <int NT, bool TRANSFER>
-__global__ void __launch_bounds__(reg_threads(2 * NT), reg_min_blocks(NT)) k_weights_reg(const __grid_constant__ RegArgs g)
+__global__ void __launch_bounds__(reg_threads(NT, 2 * NT), reg_min_blocks(NT)) k_weights_reg(const __grid_constant__ RegArgs g)
 {
     constexpr int RH = NT / 2;
     extern __shared__ __align__(16) double sm[];
     const int m = g.m, np = g.mono.np, N = m + np;
     double *L = sm;                     // [4][NT]
-    double *col = L + 4 * NT;           // [2][RH]
-    double *tb = col + NT;              // [2][2][RH]
+    double *cb = L + 4 * NT;            // [2][2][RH]
+    double *tb = cb + 2 * NT;           // [2][2][RH]
     double *diag = tb + 2 * NT, *rdiag = diag + NT;
     double *A = rdiag + NT;             // [N][N]
     double *sx = A + (size_t)N * N, *sy = sx + m, *sz = sy + m;
@@ -206,15 +216,59 @@ __global__ void __launch_bounds__(reg_threads(2 * NT), reg_min_blocks(NT)) k_wei
 #pragma unroll
             for (int l = 0; l < RH; l++) a[l] = (mypos & 1) == h && l == at ? 1.0 : 0.0;
         }
-        // t of step i from its column, by the column's warp
-        auto divide = [&](int i) {
-            if (warp != (i >> 4)) return;
-            if ((lane & 15) == (i & 15)) {
+        // column c as it stands, for the dividing warp
+        auto post = [&](int c) {
+            if (warp != (c >> 4) || (lane & 15) != (c & 15)) return;
+            double *o = cb + (c & 1) * NT + h * RH;
 #pragma unroll
-                for (int l = 0; l < RH; l += 2)
-                    *reinterpret_cast<double2 *>(col + h * RH + l) = make_double2(a[l], a[l + 1]);
+            for (int l = 0; l < RH; l += 2) *reinterpret_cast<double2 *>(o + l) = make_double2(a[l], a[l + 1]);
+        };
+        // the entry in the pivot row, from the lane of its half
+        auto pivot_entry = [&](int half) {
+            return __shfl_sync(0xffffffffu, a[0], (lane & 15) + 16 * half);
+        };
+        constexpr bool AHEAD = reg_ahead(NT);
+        const bool divider = AHEAD && warp == (int)(blockDim.x >> 5) - 1;
+        constexpr int U = (NT + 31) / 32;
+        // t of step i + 1, by the dividing warp: column i + 1 through step i,
+        // divided by its pivot (update false: column 0, for step 0).  Positions
+        // e = half * RH + register, as they are before step i; after an odd step
+        // the registers have turned by one.
+        auto divide = [&](int i, bool update) {
+            const double *col = cb + ((i + 1) & 1) * NT, *t = tb + (i & 1) * NT;
+            const int odd = i & 1;                                // step i's half (position odd * RH)
+            const int at = !update ? 0 : odd ? 1 : RH;            // the row of step i + 1
+            double u[U];
+            const double pc = update ? col[odd * RH] : 0.0;
+#pragma unroll
+            for (int q = 0; q < U; q++) {
+                const int e = lane + 32 * q;
+                u[q] = e < NT ? col[e] : 0.0;
+                if (update && e < NT) u[q] = MGM_SUB(u[q], MGM_MUL(pc, t[e]));
             }
+            double piv = u[0];
+#pragma unroll
+            for (int q = 1; q < U; q++)
+                if (at >= 32 * q) piv = u[q];
+            piv = __shfl_sync(0xffffffffu, piv, at & 31);
+            const bool ok = rcp_usable(piv);
+            const double y = ok ? __drcp_rn(piv) : 0.0;
+            double *o = tb + ((i + 1) & 1) * NT;
+#pragma unroll
+            for (int q = 0; q < U; q++) {
+                const int e = lane + 32 * q;
+                if (e >= NT) continue;
+                int to = e;
+                if (update && odd) to = e == 0 ? RH - 1 : e == RH ? NT - 1 : e - 1;
+                o[to] = e == at ? 0.0 : div_by(u[q], piv, y, ok);
+            }
+        };
+        // without it: t of step i + 1 from its column, by the column's own warp
+        auto divide_own = [&](int i) {
+            if (warp != (i >> 4)) return;
+            post(i);
             __syncwarp();
+            const double *col = cb + (i & 1) * NT;
             double *t = tb + (i & 1) * NT;
             const int at = (i & 1) * RH;  // the pivot row: register 0 of its half
             const double piv = col[at];
@@ -226,46 +280,62 @@ __global__ void __launch_bounds__(reg_threads(2 * NT), reg_min_blocks(NT)) k_wei
                 if (j < NT) t[j] = j == at ? 0.0 : div_by(col[j], piv, y, ok);
             }
         };
-        // the entry in the pivot row, from the lane of its half
-        auto pivot_entry = [&](int half) {
-            return __shfl_sync(0xffffffffu, a[0], (lane & 15) + 16 * half);
-        };
-        divide(0);
+        if constexpr (AHEAD) {
+            post(0);
+            if (N > 1) post(1);
+            __syncthreads();
+            if (divider) divide(-1, false);
+        } else {
+            divide_own(0);
+        }
         __syncthreads();
-        int i = 0;
+        if (divider) {
 #pragma unroll 1
-        for (; i < N; i += 2) {
-            if (i >= start) {
-                const double pc = pivot_entry(0);
-                const double *t = tb + h * RH;
-#pragma unroll
-                for (int l = 0; l < RH; l += 2) {
-                    if (l % 8 == 0) __syncwarp();  // keeps the loads of t from all moving up (registers)
-                    const double2 tj = *reinterpret_cast<const double2 *>(t + l);
-                    a[l] = MGM_SUB(a[l], MGM_MUL(pc, tj.x));
-                    a[l + 1] = MGM_SUB(a[l + 1], MGM_MUL(pc, tj.y));
-                }
+            for (int i = 0; i < N; i++) {
+                if (i + 1 < N) divide(i, true);
+                __syncthreads();
             }
-            if (i + 1 >= N) break;
-            divide(i + 1);
-            __syncthreads();
-            if (i >= start) {
-                const double pc = pivot_entry(1);
-                const double *t = tb + NT + h * RH;
-                double first = 0.0;
+        } else {
+            int i = 0;
+#pragma unroll 1
+            for (; i < N; i += 2) {
+                if (i >= start) {
+                    const double pc = pivot_entry(0);
+                    const double *t = tb + h * RH;
 #pragma unroll
-                for (int l = 0; l < RH; l += 2) {
-                    if (l % 8 == 0) __syncwarp();
-                    const double2 tj = *reinterpret_cast<const double2 *>(t + l);
-                    const double u = MGM_SUB(a[l], MGM_MUL(pc, tj.x));
-                    if (l > 0) a[l - 1] = u;
-                    else first = u;
-                    a[l] = MGM_SUB(a[l + 1], MGM_MUL(pc, tj.y));
+                    for (int l = 0; l < RH; l += 2) {
+                        if (l % 8 == 0) __syncwarp();  // keeps the loads of t from all moving up (registers)
+                        const double2 tj = *reinterpret_cast<const double2 *>(t + l);
+                        a[l] = MGM_SUB(a[l], MGM_MUL(pc, tj.x));
+                        a[l + 1] = MGM_SUB(a[l + 1], MGM_MUL(pc, tj.y));
+                    }
                 }
-                a[RH - 1] = first;
+                if constexpr (!AHEAD) {
+                    if (i + 1 >= N) break;
+                    divide_own(i + 1);
+                } else if (i + 2 < N) post(i + 2);
+                __syncthreads();
+                if (i + 1 >= N) break;
+                if (i >= start) {
+                    const double pc = pivot_entry(1);
+                    const double *t = tb + NT + h * RH;
+                    double first = 0.0;
+#pragma unroll
+                    for (int l = 0; l < RH; l += 2) {
+                        if (l % 8 == 0) __syncwarp();
+                        const double2 tj = *reinterpret_cast<const double2 *>(t + l);
+                        const double u = MGM_SUB(a[l], MGM_MUL(pc, tj.x));
+                        if (l > 0) a[l - 1] = u;
+                        else first = u;
+                        a[l] = MGM_SUB(a[l + 1], MGM_MUL(pc, tj.y));
+                    }
+                    a[RH - 1] = first;
+                }
+                if constexpr (!AHEAD) {
+                    if (i + 2 < N) divide_own(i + 2);
+                } else if (i + 3 < N) post(i + 3);
+                __syncthreads();
             }
-            if (i + 2 < N) divide(i + 2);
-            __syncthreads();
         }
         // register l now holds row 2 (l + N / 2 mod RH) + h; the identity
         // columns go through shared memory (the matrix has been read), where
@@ -328,7 +398,7 @@ template <int NT, bool TRANSFER>
 static void launch_reg(const RegArgs &g, cudaStream_t s)
 {
     const int N = g.m + g.mono.np;
-    const int threads = reg_threads(N + g.m);
+    const int threads = reg_threads(NT, N + g.m);
     const size_t smem = reg_smem_bytes(N, g.m, NT);
     auto kern = k_weights_reg<NT, TRANSFER>;
     MGM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
