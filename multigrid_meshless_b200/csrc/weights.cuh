@@ -138,52 +138,55 @@ __device__ inline void gauss_jordan(const Team &tm, double *aug, int *perm, doub
 }
 
 // Row 0 of gradx/grady/gradz/laplacian_matrix (rbf.h:79-270) at the seed.
-// op: 0 d/dx, 1 d/dy, 2 d/dz, 3 Laplacian.
+// op: 0 d/dx, 1 d/dy, 2 d/dz, 3 Laplacian.  Entry c.
+__device__ inline double operator_row0_entry(int op, int c, int m, int dim, int phs, const MonoDev &mono,
+                                             const double *sx, const double *sy, const double *sz)
+{
+    const double p1[3] = {sx[0], sy[0], sz[0]};
+    double v = 0;
+    if (c < m) {
+        const double p2[3] = {sx[c], sy[c], sz[c]};
+        if (op <= 2) v = MGM_MUL(MGM_MUL((double)phs, MGM_SUB(p1[op], p2[op])), mgm_phs_rbf(p1, p2, phs - 2, dim));
+        else v = MGM_MUL((double)(phs * phs), mgm_phs_rbf(p1, p2, phs - 2, dim));
+        if ((op == 1 || op == 2) && c == 0) v = 0;  // rbf.h:141, :180 zero column 0
+    } else {
+        const int j = c - m;
+        const double d0 = MGM_SUB(p1[0], sx[0]), d1 = MGM_SUB(p1[1], sy[0]), d2 = MGM_SUB(p1[2], sz[0]);
+        const int ex = mono.px[j], ey = mono.py[j], ez = mono.pz[j];
+        if (op == 0) {
+            if (j == 0 || ex == 0) v = 0;
+            else { v = MGM_MUL((double)ex, mgm_pow_int(d0, ex - 1)); v = MGM_MUL(v, mgm_pow_int(d1, ey)); v = MGM_MUL(v, mgm_pow_int(d2, ez)); }
+        } else if (op == 1) {
+            if (j == 0 || ey == 0) v = 0;  // grad[i][m] is never written by grady_matrix: zero from create_matrix
+            else { v = MGM_MUL((double)ey, mgm_pow_int(d1, ey - 1)); v = MGM_MUL(v, mgm_pow_int(d0, ex)); v = MGM_MUL(v, mgm_pow_int(d2, ez)); }
+        } else if (op == 2) {
+            if (j == 0 || ez == 0) v = 0;
+            else { v = MGM_MUL((double)ez, mgm_pow_int(d2, ez - 1)); v = MGM_MUL(v, mgm_pow_int(d1, ey)); v = MGM_MUL(v, mgm_pow_int(d0, ex)); }
+        } else {
+            double tx = 0, ty = 0, tz = 0;
+            if (ex > 1) {
+                tx = MGM_MUL((double)(ex * (ex - 1)), mgm_pow_int(d0, ex - 2));
+                tx = MGM_MUL(tx, mgm_pow_int(d1, ey));
+                if (dim == 3) tx = MGM_MUL(tx, mgm_pow_int(d2, ez));
+            } else if (ey > 1) {
+                ty = MGM_MUL((double)(ey * (ey - 1)), mgm_pow_int(d1, ey - 2));
+                ty = MGM_MUL(ty, mgm_pow_int(d0, ex));
+                if (dim == 3) ty = MGM_MUL(ty, mgm_pow_int(d2, ez));
+            } else if (dim == 3 && ez > 1) {
+                tz = MGM_MUL((double)(ez * (ez - 1)), mgm_pow_int(d2, ez - 2));
+                tz = MGM_MUL(tz, mgm_pow_int(d0, ex));
+                tz = MGM_MUL(tz, mgm_pow_int(d1, ey));
+            }
+            v = dim == 3 ? MGM_ADD(MGM_ADD(tx, ty), tz) : MGM_ADD(tx, ty);
+        }
+    }
+    return v;
+}
+
 __device__ inline void operator_row0(const Team &tm, int op, int m, int np, int dim, int phs, const MonoDev &mono,
                                      const double *sx, const double *sy, const double *sz, double *L)
 {
-    const int N = m + np;
-    const double p1[3] = {sx[0], sy[0], sz[0]};
-    for (int c = tm.tid; c < N; c += tm.size) {
-        double v = 0;
-        if (c < m) {
-            const double p2[3] = {sx[c], sy[c], sz[c]};
-            if (op <= 2) v = MGM_MUL(MGM_MUL((double)phs, MGM_SUB(p1[op], p2[op])), mgm_phs_rbf(p1, p2, phs - 2, dim));
-            else v = MGM_MUL((double)(phs * phs), mgm_phs_rbf(p1, p2, phs - 2, dim));
-            if ((op == 1 || op == 2) && c == 0) v = 0;  // rbf.h:141, :180 zero column 0
-        } else {
-            const int j = c - m;
-            const double d0 = MGM_SUB(p1[0], sx[0]), d1 = MGM_SUB(p1[1], sy[0]), d2 = MGM_SUB(p1[2], sz[0]);
-            const int ex = mono.px[j], ey = mono.py[j], ez = mono.pz[j];
-            if (op == 0) {
-                if (j == 0 || ex == 0) v = 0;
-                else { v = MGM_MUL((double)ex, mgm_pow_int(d0, ex - 1)); v = MGM_MUL(v, mgm_pow_int(d1, ey)); v = MGM_MUL(v, mgm_pow_int(d2, ez)); }
-            } else if (op == 1) {
-                if (j == 0 || ey == 0) v = 0;  // grad[i][m] is never written by grady_matrix: zero from create_matrix
-                else { v = MGM_MUL((double)ey, mgm_pow_int(d1, ey - 1)); v = MGM_MUL(v, mgm_pow_int(d0, ex)); v = MGM_MUL(v, mgm_pow_int(d2, ez)); }
-            } else if (op == 2) {
-                if (j == 0 || ez == 0) v = 0;
-                else { v = MGM_MUL((double)ez, mgm_pow_int(d2, ez - 1)); v = MGM_MUL(v, mgm_pow_int(d1, ey)); v = MGM_MUL(v, mgm_pow_int(d0, ex)); }
-            } else {
-                double tx = 0, ty = 0, tz = 0;
-                if (ex > 1) {
-                    tx = MGM_MUL((double)(ex * (ex - 1)), mgm_pow_int(d0, ex - 2));
-                    tx = MGM_MUL(tx, mgm_pow_int(d1, ey));
-                    if (dim == 3) tx = MGM_MUL(tx, mgm_pow_int(d2, ez));
-                } else if (ey > 1) {
-                    ty = MGM_MUL((double)(ey * (ey - 1)), mgm_pow_int(d1, ey - 2));
-                    ty = MGM_MUL(ty, mgm_pow_int(d0, ex));
-                    if (dim == 3) ty = MGM_MUL(ty, mgm_pow_int(d2, ez));
-                } else if (dim == 3 && ez > 1) {
-                    tz = MGM_MUL((double)(ez * (ez - 1)), mgm_pow_int(d2, ez - 2));
-                    tz = MGM_MUL(tz, mgm_pow_int(d0, ex));
-                    tz = MGM_MUL(tz, mgm_pow_int(d1, ey));
-                }
-                v = dim == 3 ? MGM_ADD(MGM_ADD(tx, ty), tz) : MGM_ADD(tx, ty);
-            }
-        }
-        L[c] = v;
-    }
+    for (int c = tm.tid; c < m + np; c += tm.size) L[c] = operator_row0_entry(op, c, m, dim, phs, mono, sx, sy, sz);
 }
 
 // Interpolation row of create_restriction/prolongation_matrix (mesh_functions.h:533-670):

@@ -174,8 +174,11 @@ __global__ void __launch_bounds__(reg_threads(NT, 2 * NT), reg_min_blocks(NT)) k
             const double s0[3] = {g.x[seed], g.y[seed], g.z[seed]};
             transfer_row(tm, m, np, g.dim, g.phs, g.mono, sx, sy, sz, p1, s0, L);
         } else {
-            for (int o = 0; o < nops; o++)
-                operator_row0(tm, o == nops - 1 ? 3 : o, m, np, g.dim, g.phs, g.mono, sx, sy, sz, L + o * NT);
+            // all operators' rows in one pass, a thread per entry
+            for (int e = tid; e < nops * N; e += blockDim.x) {
+                const int o = e / N, c = e - o * N;
+                L[o * NT + c] = operator_row0_entry(o == nops - 1 ? 3 : o, c, m, g.dim, g.phs, g.mono, sx, sy, sz);
+            }
         }
         __syncthreads();
         // the bubble pass on column 0 from the last row up: the carried row
