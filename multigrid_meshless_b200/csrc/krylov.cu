@@ -455,7 +455,8 @@ struct FgRow {
     RowChunk<double, KC ? KC : 8, IDX> R;
     __device__ __forceinline__ void fetch(const FgOperator &op, int i)
     {
-        if (KC || op.k >= 8) R.fetch(op.gi, op.A, op.n, i, i, 0);
+        if constexpr (KC > 0) R.fetch(op.gi, op.A, op.n, i, i, 0);
+        else R.fetch_to(op.gi, op.A, op.n, i, i, 0, op.k);
     }
     template <class X>
     __device__ __forceinline__ double dot(const FgOperator &op, const X *x, int i)

@@ -88,6 +88,24 @@ struct RowChunk {
             a[q] = ldk(pa + q * ld);
         }
     }
+    // the same of a row of k slots; past its end the last slot again (not summed)
+    __device__ __forceinline__ void fetch_to(const void *__restrict__ gi, const T *__restrict__ A, long ld, long i,
+                                             int base, int j0, int k)
+    {
+        const T *pa = A + (long)j0 * ld + i;
+        const int *pi = static_cast<const int *>(gi) + (long)j0 * ld + i;
+        const short *po = static_cast<const short *>(gi) + (long)j0 * ld + i;
+#pragma unroll
+        for (int q = 0; q < KC; q++) {
+            if constexpr (IDX) c[q] = ldk(pi);
+            else c[q] = base + ldk(po);
+            a[q] = ldk(pa);
+            const long st = j0 + q + 1 < k ? ld : 0;
+            pa += st;
+            if constexpr (IDX) pi += st;
+            else po += st;
+        }
+    }
     template <bool EARLY, class X>
     __device__ __forceinline__ T dot(const X *x, T s) const
     {
@@ -112,27 +130,27 @@ __device__ __forceinline__ T row_rest(const void *gi, const T *A, const X *x, lo
     return s;
 }
 
-// a whole row of k slots, 8 at a time, none beyond k read (the large levels);
-// R: the first chunk, already fetched (k >= 8)
+// a whole row of k slots, 8 at a time, none beyond k read (the large levels),
+// the next 8 slots' operator in flight during the current gathers; R: the first
+// chunk, by fetch_to (prolongation to 1M rows of 30 slots: 63 us with each
+// chunk's loads after the last one's gathers and the last k mod 8 slots one by
+// one, now 45)
 template <class T, bool IDX, class X>
 __device__ __forceinline__ T row_big(RowChunk<T, 8, IDX> &R, const void *gi, const T *A, const X *x, long ld, int k,
                                      long i, int base)
 {
     T s = T(0);
-    int j = 0;
-    if (k >= 8) {
-        s = R.template dot<false>(x, s);
-        for (j = 8; j + 8 <= k; j += 8) {
-            R.fetch(gi, A, ld, i, base, j);
-            s = R.template dot<false>(x, s);
-        }
-    }
-    for (; j < k; j++) {
-        const long o = (long)j * ld + i;
-        int c;
-        if constexpr (IDX) c = __ldg(static_cast<const int *>(gi) + o);
-        else c = base + (int)__ldg(static_cast<const short *>(gi) + o);
-        s = fma_rn(__ldg(A + o), (T)__ldg(x + c), s);
+    for (int j = 0; j < k; j += 8) {
+        RowChunk<T, 8, IDX> N;
+        X v[8];
+        if (j + 8 < k) N.fetch_to(gi, A, ld, i, base, j + 8, k);
+        else N = R;
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = __ldg(x + R.c[q]);
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (j + q < k) s = fma_rn(R.a[q], (T)v[q], s);
+        R = N;
     }
     return s;
 }

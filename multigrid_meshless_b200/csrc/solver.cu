@@ -713,7 +713,8 @@ struct TransferRow {
     __device__ __forceinline__ void fetch(const TransferArgs<T> &a, int i)
     {
         if constexpr (!IDX) base = ldk(a.base + i);
-        if (EARLY || a.k >= KC) R.fetch(a.gi, a.w, a.n, i, base, 0);
+        if constexpr (EARLY) R.fetch(a.gi, a.w, a.n, i, base, 0);
+        else R.fetch_to(a.gi, a.w, a.n, i, base, 0, a.k);
     }
     __device__ __forceinline__ T dot(const TransferArgs<T> &a, int i)
     {
