@@ -77,50 +77,6 @@ __global__ void k_reduce_parts(const double *__restrict__ part, int nblk, int cn
     if (threadIdx.x == 0) out[c] = s;
 }
 
-// w -= sum_c h[c] V_c, and per-block partial |w|^2 of the result (grid-stride)
-__global__ void __launch_bounds__(256) k_orth_norm(int n, int cnt, const double *__restrict__ V, long ldv,
-                                                   const double *__restrict__ h, double *__restrict__ w,
-                                                   double *__restrict__ part)
-{
-    __shared__ double hs[kMaxKrylov + 1];
-    __shared__ double sm[32];
-    for (int c = threadIdx.x; c < cnt; c += blockDim.x) hs[c] = h[c];
-    __syncthreads();
-    double acc = 0.0;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        double s = w[i];
-        for (int c = 0; c < cnt; c++) s = fma(-hs[c], V[c * ldv + i], s);
-        w[i] = s;
-        acc = fma(s, s, acc);
-    }
-    acc = bsum<256>(acc, sm);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc;
-}
-
-// w -= sum_c h[c] V_c
-__global__ void __launch_bounds__(256) k_orth_update(int n, int cnt, const double *__restrict__ V, long ldv,
-                                                     const double *__restrict__ h, double *__restrict__ w)
-{
-    __shared__ double hs[kMaxKrylov + 1];
-    for (int c = threadIdx.x; c < cnt; c += blockDim.x) hs[c] = h[c];
-    __syncthreads();
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = w[i];
-    for (int c = 0; c < cnt; c++) s = fma(-hs[c], V[c * ldv + i], s);
-    w[i] = s;
-}
-
-// out = in * (1 / *nrm) where nrm holds |.|^2 or |.| (is_sq)
-__global__ void k_scale_by(int n, const double *__restrict__ in, double *__restrict__ out, const double *__restrict__ nrm,
-                           int is_sq)
-{
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double d = is_sq ? sqrt(*nrm) : *nrm;
-    out[i] = d > 0 ? in[i] / d : 0.0;
-}
-
 // x += sum_c y[c] Z_c  (Z in precision T)
 template <class T>
 __global__ void __launch_bounds__(256) k_combine(int n, int cnt, const T *__restrict__ Z, long ldz,
@@ -173,30 +129,6 @@ void multidot(int n, int cnt, const double *V, long ldv, const double *w, double
     k_multidot<<<nb, 256, 0, s>>>(n, cnt, V, ldv, w, part);
     MGM_LAUNCHED();
     k_reduce_parts<<<cnt, 256, 0, s>>>(part, nb, cnt, out);
-    MGM_LAUNCHED();
-}
-void reduce_parts(const double *part, int nblk, int cnt, double *out, cudaStream_t s)
-{
-    k_reduce_parts<<<cnt, 256, 0, s>>>(part, nblk, cnt, out);
-    MGM_LAUNCHED();
-}
-void orth_norm(int n, int cnt, const double *V, long ldv, const double *h, double *w, double *part, double *norm2,
-               cudaStream_t s)
-{
-    const int nb = dot_blocks(n);
-    k_orth_norm<<<nb, 256, 0, s>>>(n, cnt, V, ldv, h, w, part);
-    MGM_LAUNCHED();
-    k_reduce_parts<<<1, 256, 0, s>>>(part, nb, 1, norm2);
-    MGM_LAUNCHED();
-}
-void orth_update(int n, int cnt, const double *V, long ldv, const double *h, double *w, cudaStream_t s)
-{
-    k_orth_update<<<blocks_for(n, 256), 256, 0, s>>>(n, cnt, V, ldv, h, w);
-    MGM_LAUNCHED();
-}
-void scale_by(int n, const double *in, double *out, const double *nrm, int is_sq, cudaStream_t s)
-{
-    k_scale_by<<<blocks_for(n, 256), 256, 0, s>>>(n, in, out, nrm, is_sq);
     MGM_LAUNCHED();
 }
 template <class T>
@@ -925,8 +857,9 @@ void set_scalar(double *dst, double v, cudaStream_t s)
 // grid barrier all take the same winner, scale its row and update their own
 // rows.  The operations on an entry, and their order, are those of elimination
 // on [M | I] with row swaps, whose other entries are zeros and ones.  A step is
-// the barrier and two dependent L2 reads: 7.5 us at 957 rows, against 15 us as
-// four launches over the matrix of twice the width (1024 threads 8.2; 74 CTAs 9.2).
+// the barrier and two dependent L2 reads: 6.9 us at 896 rows (7.4 with the
+// candidates read by one warp), against 15 us as four launches over the matrix
+// of twice the width (1024 threads 8.2; 74 CTAs 9.2).
 constexpr int kInvThreads = 512;
 
 struct InvCand {
@@ -989,11 +922,14 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_dense_inverse(int n, int k, 
                 const InvCand x{v >= 0.0 ? v : -1.0, pos[q], b + q * G};  // a NaN after every number
                 if (better(x, best)) best = x;
             }
-        best = warp_best(best);
-        if (lane == 0) wcand[warp] = best;
-        __syncthreads();
+        if (mine > 32) {  // else warp 0 has them all
+            best = warp_best(best);
+            if (lane == 0) wcand[warp] = best;
+            __syncthreads();
+            if (warp == 0) best = lane < kInvThreads / 32 ? wcand[lane] : InvCand{-2.0, n, -1};
+        }
         if (warp == 0) {
-            best = warp_best(lane < kInvThreads / 32 ? wcand[lane] : InvCand{-2.0, n, -1});
+            best = warp_best(best);
             if (lane == 0) {
                 win = best;
                 __stcg(reinterpret_cast<int4 *>(cand + (c & 1) * G + b), *reinterpret_cast<const int4 *>(&best));
@@ -1009,21 +945,20 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_dense_inverse(int n, int k, 
     offer(0);
     for (int c = 0; c < n; c++) {
         if (!grid_barrier(bar, err, gen)) return;
-        if (warp == 0) {
-            InvCand best{-2.0, n, -1};
-            for (int t = lane; t < G; t += 32) {
-                const int4 raw = __ldcg(reinterpret_cast<const int4 *>(cand + (c & 1) * G + t));
-                const InvCand x = *reinterpret_cast<const InvCand *>(&raw);
-                if (better(x, best)) best = x;
-            }
+        // the winner: a candidate per thread, then every warp over the warps' best
+        InvCand best{-2.0, n, -1};
+        if (tid < G) {
+            const int4 raw = __ldcg(reinterpret_cast<const int4 *>(cand + (c & 1) * G + tid));
+            best = *reinterpret_cast<const InvCand *>(&raw);
+        }
+        if (warp < (G + 31) / 32) {
             best = warp_best(best);
-            if (lane == 0) {
-                win = best;
-                piv[c] = best.row;
-            }
+            if (lane == 0) wcand[warp] = best;
         }
         __syncthreads();
-        const int P = win.row, pp = win.pos, owner = P % G;
+        best = warp_best(lane < (G + 31) / 32 ? wcand[lane] : InvCand{-2.0, n, -1});
+        if (tid == 0) piv[c] = best.row;
+        const int P = best.row, pp = best.pos, owner = P % G;
         const double *src = cand_row + (long)((c & 1) * G + owner) * n;
         const double p = __ldcg(src + c);
         for (int t = tid; t < n; t += kInvThreads) sc[t] = (t == c ? 1.0 : __ldcg(src + t)) / p;

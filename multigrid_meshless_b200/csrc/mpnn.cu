@@ -65,10 +65,6 @@ __device__ __forceinline__ float2 ld_bf2(const bf16 *p)
     const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162 *>(p);
     return __bfloat1622float2(v);
 }
-__device__ __forceinline__ void st_bf2(bf16 *p, float a, float b)
-{
-    *reinterpret_cast<__nv_bfloat162 *>(p) = __floats2bfloat162_rn(a, b);
-}
 
 template <int BS>
 __device__ __forceinline__ double bsum_d(double v, double *sm)
@@ -189,8 +185,6 @@ __device__ __forceinline__ void mma_bf16(float *c, uint32_t a0, uint32_t a1, uin
 }
 
 constexpr int kTile = 64, kPad = 200;  // rows per CTA, padded row length (bf16) of the smem tile
-
-struct bf4 { __nv_bfloat162 a, b; };
 
 // One message-passing layer for 64 nodes: gather [h_i | mean h_j | sum l_ij h_j]
 // into shared memory (BF16), multiply by W (tensor cores, FP32 accumulate),
