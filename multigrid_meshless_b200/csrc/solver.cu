@@ -16,6 +16,8 @@
 // Outer: flexible GMRES in FP64 (residuals, Krylov basis, solution updates).
 #include <cmath>
 
+#include <type_traits>
+
 #include "krylov.cuh"
 #include "coop.cuh"
 #include "rows.cuh"
@@ -92,18 +94,76 @@ struct BndRow {
     }
 };
 
-// Exact solve of the boundary rows, one warp per row.
+// The same by 8 lanes, g = lane & 7, for the levels of kVecMinRows rows and
+// more, where a warp per row is several waves of CTAs: 23k boundary rows of the
+// 64^3 cube take 7.1 us a launch, 9.3 with a warp per row; on the small levels
+// it is the longer chain (5.4k rows: 5.0 us against 4.2).  Lane g stands for
+// lanes g, g + 8, g + 16 and g + 24 of the warp, so the sum has the same bits.
+template <class T>
+struct BndRow8 {
+    int i = 0, w = 0, c[2][4];
+    T a[2][4], di;
+    __device__ __forceinline__ void fetch(int row, int g, int nbl, const int *__restrict__ list, int k,
+                                          const int *__restrict__ bidx, const T *__restrict__ bA,
+                                          const T *__restrict__ dinv)
+    {
+        w = min(row, nbl - 1);
+        i = ldk(list + w);
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            if (32 * q < k) {
+#pragma unroll
+                for (int v = 0; v < 4; v++) {
+                    const long o = (long)w * k + min(g + 8 * v + 32 * q, k - 1);
+                    c[q][v] = ldk(bidx + o);
+                    a[q][v] = ldk(bA + o);
+                }
+            }
+        di = ldk(dinv + i);
+    }
+    __device__ __forceinline__ T value(int g, int k, const int *__restrict__ bidx, const T *__restrict__ bA,
+                                       const T *r, const T *e) const
+    {
+        T x[2][4], s[4] = {T(0), T(0), T(0), T(0)};
+        const T ri = __ldcg(r + i), ei = __ldcg(e + i);
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            if (32 * q < k) {
+#pragma unroll
+                for (int v = 0; v < 4; v++) x[q][v] = __ldcg(e + c[q][v]);
+            }
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int v = 0; v < 4; v++)
+                if (g + 8 * v + 32 * q < k) s[v] = fma_rn(a[q][v], x[q][v], s[v]);
+        for (int j0 = 64; j0 < k; j0 += 32)
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const int j = j0 + g + 8 * v;
+                if (j < k) s[v] = fma_rn(__ldg(bA + (long)w * k + j), __ldcg(e + __ldg(bidx + (long)w * k + j)), s[v]);
+            }
+        T t = (s[0] + s[2]) + (s[1] + s[3]);
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o, 8);
+        return fma_rn(ri - t, di, ei);
+    }
+};
+inline int bnd_blocks(int nbl, bool big) { return blocks_for((long)nbl * (big ? 8 : 32), 256); }
+
+// Exact solve of the boundary rows: a warp per row (EARLY, the small levels) or
+// 8 lanes per row.
 template <class T, bool EARLY>
 __global__ void __launch_bounds__(256) k_bnd_exact(int nbl, const int *__restrict__ list, int k,
                                                    const int *__restrict__ bidx, const T *__restrict__ bA,
                                                    const T *__restrict__ dinv, const T *r, T *e)
 {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    BndRow<T> B;
-    B.fetch(w, lane, nbl, list, k, bidx, bA, dinv);
+    constexpr int LANES = EARLY ? 32 : 8;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) / LANES, g = threadIdx.x % LANES;
+    std::conditional_t<EARLY, BndRow<T>, BndRow8<T>> B;
+    B.fetch(w, g, nbl, list, k, bidx, bA, dinv);
     pdl_wait<EARLY>();
-    const T v = B.value(lane, k, bidx, bA, r, e);
-    if (lane == 0 && w < nbl) e[B.i] = v;
+    const T v = B.value(g, k, bidx, bA, r, e);
+    if (g == 0 && w < nbl) e[B.i] = v;
 }
 
 // The first step of a smoothing pass from e = 0.  There e is zero but on the
@@ -347,12 +407,12 @@ __device__ __forceinline__ void step_out(const StepArgsL<T> &a, int i, T ri, T e
 template <int MODE, class T>
 __device__ __forceinline__ void step_bnd_part(const StepArgsL<T> &a, int blk)
 {
-    const int w = (blk * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    BndRow<T> B;
-    B.fetch(w, lane, a.nbl, a.bnd_list, a.k, a.bnd_idx, a.bnd_A, a.dinv);
+    const int w = (blk * blockDim.x + threadIdx.x) >> 3, g = threadIdx.x & 7;
+    BndRow8<T> B;
+    B.fetch(w, g, a.nbl, a.bnd_list, a.k, a.bnd_idx, a.bnd_A, a.dinv);
     pdl_wait<false>();
-    const T v = B.value(lane, a.k, a.bnd_idx, a.bnd_A, a.r, a.e);
-    if (lane == 0 && w < a.nbl) {
+    const T v = B.value(g, a.k, a.bnd_idx, a.bnd_A, a.r, a.e);
+    if (g == 0 && w < a.nbl) {
         a.e[B.i] = v;
         a.out[B.i] = MODE == 0 ? v : T(0);
     }
@@ -637,7 +697,7 @@ static StepArgsL<T> step_args_of(const SolveLevel<T> &L, T *e, T *out, T c1, T c
 template <class T>
 static void launch_bnd(const SolveLevel<T> &L, T *e, cudaStream_t s, Chain &launch)
 {
-    const int nbb = blocks_for((long)L.nb_list * 32, 256);
+    const int nbb = bnd_blocks(L.nb_list, L.n >= kVecMinRows);
     if (nbb == 0) return;
     if (L.n < kVecMinRows)
         launch(k_bnd_exact<T, true>, nbb, 256, 0, s, L.nb_list, L.bnd_list, L.k, L.bnd_idx, L.bnd_A, L.dinv, L.r, e);
@@ -1500,10 +1560,10 @@ static void launch_step(const SolveLevel<T> &L, T *e, T *out, T c1, T c2, int fi
     }
     const bool big = L.off && L.n >= kVecMinRows;
     // One launch with the boundary part pays while that part is small beside
-    // the far part (the 500^2 cavity, 250 CTAs beside 245: 17.4 us against
-    // 16.0 + 4.2); in 3D it is not (the 64^3 cube, 2883 beside 245: 44 us
-    // against 19.6 + 6.3, the far part waits for slots).
-    const int nbc = blocks_for((long)L.nb_list * 32, 256), nfar = blocks_for(L.n, 1024);
+    // the far part (the 500^2 cavity, 63 CTAs beside 245: 17 us against
+    // 16.0 + 4.2); in 3D it is not (the 64^3 cube, 721 beside 256; with four
+    // times as many 44 us against 19.6 + 6.3, the far part waits for slots).
+    const int nbc = bnd_blocks(L.nb_list, true), nfar = blocks_for(L.n, 1024);
     const bool one = big && nbc <= 2 * nfar;
     if (!one) launch_bnd(L, e, s, launch);
     mark();
