@@ -862,7 +862,7 @@ void set_scalar(double *dst, double v, cudaStream_t s)
 // of twice the width (1024 threads 8.2; 74 CTAs 9.2).
 constexpr int kInvThreads = 512;
 
-struct InvCand {
+struct alignas(16) InvCand {  // read and written as one int4
     double v;
     int pos, row;
 };
