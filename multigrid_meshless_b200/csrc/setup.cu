@@ -600,6 +600,10 @@ static int weights_grid(long rows)
     return (int)std::min<long>(rows, 148L * 64);
 }
 
+// Opt-in shared memory of the two kernels for orders above the register
+// kernels'.  The limit holds for all threads of the process: one value for all.
+constexpr size_t kWeightsSmem = 227 * 1024;
+
 void derivative_weights(int n, int k, int dim, int phs, const Monomials &mono, const double *x, const double *y,
                         const double *z, const double *nx, const double *ny, const double *nz, const uint8_t *btag,
                         const int *cloud, double *Dx, double *Dy, double *Dz, double *lap, double *lapP, cudaStream_t s)
@@ -608,8 +612,8 @@ void derivative_weights(int n, int k, int dim, int phs, const Monomials &mono, c
     if (n <= 0) return;
     if (derivative_weights_reg(n, k, dim, phs, mono, x, y, z, nx, ny, nz, btag, cloud, Dx, Dy, Dz, lap, lapP, s)) return;
     size_t smem = weights_smem(k, mono.np);
-    MGM_REQUIRE(smem <= 227 * 1024, "weights: system does not fit in shared memory");
-    MGM_CUDA(cudaFuncSetAttribute(k_derivative_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MGM_REQUIRE(smem <= kWeightsSmem, "weights: system does not fit in shared memory");
+    MGM_CUDA(cudaFuncSetAttribute(k_derivative_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWeightsSmem));
     k_derivative_weights<<<weights_grid(n), 128, smem, s>>>(n, k, dim, phs, to_dev(mono), x, y, z, nx, ny, nz, btag,
                                                            cloud, Dx, Dy, Dz, lap, lapP);
     MGM_LAUNCHED();
@@ -664,8 +668,8 @@ void transfer_weights(int nt, const double *tx, const double *ty, const double *
         return;
     const int N = ks + mono.np;
     size_t smem = sizeof(double) * ((size_t)N * 2 * N + 3 * ks + 2 * N) + sizeof(int) * N;
-    MGM_REQUIRE(smem <= 227 * 1024, "transfer weights: system does not fit in shared memory");
-    MGM_CUDA(cudaFuncSetAttribute(k_transfer_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MGM_REQUIRE(smem <= kWeightsSmem, "transfer weights: system does not fit in shared memory");
+    MGM_CUDA(cudaFuncSetAttribute(k_transfer_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWeightsSmem));
     k_transfer_weights<<<weights_grid(nt), 128, smem, s>>>(nt, tx, ty, tz, tbtag, src_pt, rows_from, only_interior, ks,
                                                           dim, phs, to_dev(mono), sx, sy, sz, scloud, W);
     MGM_LAUNCHED();

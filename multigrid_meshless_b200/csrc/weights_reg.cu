@@ -404,7 +404,9 @@ static void launch_reg(const RegArgs &g, cudaStream_t s)
     const int threads = reg_threads(NT, N + g.m);
     const size_t smem = reg_smem_bytes(N, g.m, NT);
     auto kern = k_weights_reg<NT, TRANSFER>;
-    MGM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the kernel's limit holds for all threads of the process: one value for all the orders it takes
+    MGM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)reg_smem_bytes(NT, NT, NT)));
     int per_sm = 0;
     MGM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     const int grid = (int)std::min<long>(g.n, 148L * std::max(1, per_sm));
