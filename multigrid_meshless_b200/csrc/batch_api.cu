@@ -10,6 +10,7 @@ namespace {
 template <class F>
 int bguard(F &&f)
 {
+    const TrimScope trim;
     try {
         f();
         return MGM_OK;

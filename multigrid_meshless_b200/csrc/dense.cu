@@ -53,6 +53,7 @@ __global__ void k_lap_poisson(int n, int k, int dim, const double *__restrict__ 
 template <class F>
 int dguard(F &&f)
 {
+    const TrimScope trim;
     try {
         f();
         return MGM_OK;
@@ -78,22 +79,15 @@ int mgm_gauss_jordan(int order, const double *A, double *inverse)
         MGM_REQUIRE(order >= 1 && order <= 1024, "mgm_gauss_jordan: order must be in [1, 1024]");
         MGM_REQUIRE(A != nullptr && inverse != nullptr, "mgm_gauss_jordan: null pointer");
         const size_t nn = (size_t)order * order;
-        cudaStream_t s = nullptr;
-        MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        const AllocScope scope(s);
-        try {
-            DBuf<double> dA(nn), aug(2 * nn), t(order), dinv(nn);
-            DBuf<int> perm(order);
-            dA.upload(A, nn, s);
-            k_gj_inverse<<<1, 256, 0, s>>>(order, dA.p, aug.p, perm.p, t.p, dinv.p);
-            MGM_LAUNCHED();
-            dinv.download(inverse, nn, s);
-            MGM_CUDA(cudaStreamSynchronize(s));
-        } catch (...) {
-            cudaStreamDestroy(s);
-            throw;
-        }
-        MGM_CUDA(cudaStreamDestroy(s));
+        const CallStream call;
+        const cudaStream_t s = call.s;
+        DBuf<double> dA(nn), aug(2 * nn), t(order), dinv(nn);
+        DBuf<int> perm(order);
+        dA.upload(A, nn, s);
+        k_gj_inverse<<<1, 256, 0, s>>>(order, dA.p, aug.p, perm.p, t.p, dinv.p);
+        MGM_LAUNCHED();
+        dinv.download(inverse, nn, s);
+        MGM_CUDA(cudaStreamSynchronize(s));
     });
 }
 
@@ -106,25 +100,18 @@ int mgm_laplacian_for_poisson(int n, int k, int dim, const double *Dx, const dou
         MGM_REQUIRE(Dx && Dy && lap && nx && ny && btag && lapP && (dim == 2 || (Dz && nz)),
                     "mgm_laplacian_for_poisson: null pointer");
         const size_t nk = (size_t)n * k;
-        cudaStream_t s = nullptr;
-        MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        const AllocScope scope(s);
-        try {
-            DBuf<double> dx(nk), dy(nk), dz(dim == 3 ? nk : 1), dl(nk), vx(n), vy(n), vz(n), out(nk);
-            DBuf<unsigned char> bt(n);
-            dx.upload(Dx, nk, s); dy.upload(Dy, nk, s); dl.upload(lap, nk, s);
-            vx.upload(nx, n, s); vy.upload(ny, n, s); bt.upload(btag, n, s);
-            if (dim == 3) { dz.upload(Dz, nk, s); vz.upload(nz, n, s); }
-            k_lap_poisson<<<blocks_for((long)nk, 256), 256, 0, s>>>(n, k, dim, dx.p, dy.p, dz.p, dl.p, vx.p, vy.p, vz.p,
-                                                                   bt.p, out.p);
-            MGM_LAUNCHED();
-            out.download(lapP, nk, s);
-            MGM_CUDA(cudaStreamSynchronize(s));
-        } catch (...) {
-            cudaStreamDestroy(s);
-            throw;
-        }
-        MGM_CUDA(cudaStreamDestroy(s));
+        const CallStream call;
+        const cudaStream_t s = call.s;
+        DBuf<double> dx(nk), dy(nk), dz(dim == 3 ? nk : 1), dl(nk), vx(n), vy(n), vz(n), out(nk);
+        DBuf<unsigned char> bt(n);
+        dx.upload(Dx, nk, s); dy.upload(Dy, nk, s); dl.upload(lap, nk, s);
+        vx.upload(nx, n, s); vy.upload(ny, n, s); bt.upload(btag, n, s);
+        if (dim == 3) { dz.upload(Dz, nk, s); vz.upload(nz, n, s); }
+        k_lap_poisson<<<blocks_for((long)nk, 256), 256, 0, s>>>(n, k, dim, dx.p, dy.p, dz.p, dl.p, vx.p, vy.p, vz.p,
+                                                               bt.p, out.p);
+        MGM_LAUNCHED();
+        out.download(lapP, nk, s);
+        MGM_CUDA(cudaStreamSynchronize(s));
     });
 }
 

@@ -224,26 +224,19 @@ mgm_mesh *read_mesh(const char *path, int dim)
     }
     std::vector<double> NX(nn), NY(nn), NZ(nn);
     {
-        cudaStream_t s;
-        MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        const AllocScope scope(s);
-        try {
-            DBuf<double> dx(nn), dy(nn), dz(nn), dnx(nn), dny(nn), dnz(nn);
-            DBuf<int4> dev(std::max<size_t>(be.size(), 1));
-            DBuf<int> det(std::max<size_t>(be.size(), 1)), drp(nn + 1), del(std::max<size_t>(elist.size(), 1));
-            dx.upload(X.data(), nn, s); dy.upload(Y.data(), nn, s); dz.upload(Z.data(), nn, s);
-            dev.upload(ev.data(), ev.size(), s); det.upload(et.data(), et.size(), s);
-            drp.upload(rowptr.data(), nn + 1, s); del.upload(elist.data(), elist.size(), s);
-            k_mesh_normals<<<blocks_for(nn, 256), 256, 0, s>>>((int)nn, dx.p, dy.p, dz.p, dev.p, det.p, drp.p, del.p,
-                                                               dnx.p, dny.p, dnz.p);
-            MGM_LAUNCHED();
-            dnx.download(NX.data(), nn, s); dny.download(NY.data(), nn, s); dnz.download(NZ.data(), nn, s);
-            MGM_CUDA(cudaStreamSynchronize(s));
-        } catch (...) {
-            cudaStreamDestroy(s);
-            throw;
-        }
-        MGM_CUDA(cudaStreamDestroy(s));
+        const CallStream call;
+        const cudaStream_t s = call.s;
+        DBuf<double> dx(nn), dy(nn), dz(nn), dnx(nn), dny(nn), dnz(nn);
+        DBuf<int4> dev(std::max<size_t>(be.size(), 1));
+        DBuf<int> det(std::max<size_t>(be.size(), 1)), drp(nn + 1), del(std::max<size_t>(elist.size(), 1));
+        dx.upload(X.data(), nn, s); dy.upload(Y.data(), nn, s); dz.upload(Z.data(), nn, s);
+        dev.upload(ev.data(), ev.size(), s); det.upload(et.data(), et.size(), s);
+        drp.upload(rowptr.data(), nn + 1, s); del.upload(elist.data(), elist.size(), s);
+        k_mesh_normals<<<blocks_for(nn, 256), 256, 0, s>>>((int)nn, dx.p, dy.p, dz.p, dev.p, det.p, drp.p, del.p,
+                                                           dnx.p, dny.p, dnz.p);
+        MGM_LAUNCHED();
+        dnx.download(NX.data(), nn, s); dny.download(NY.data(), nn, s); dnz.download(NZ.data(), nn, s);
+        MGM_CUDA(cudaStreamSynchronize(s));
     }
     long nbnd = 0, ncorner = 0;
     for (long i = 0; i < nn; i++) { nbnd += BT[i] != 0; ncorner += CT[i] != 0; }
@@ -264,6 +257,7 @@ mgm_mesh *read_mesh(const char *path, int dim)
 template <class F>
 int gguard(F &&f)
 {
+    const TrimScope trim;
     try {
         f();
         return MGM_OK;

@@ -132,6 +132,7 @@ double heat_step(mgm_ctx *c)
 template <class F>
 int hguard(F &&f)
 {
+    const TrimScope trim;
     try {
         f();
         return MGM_OK;

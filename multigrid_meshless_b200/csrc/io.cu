@@ -176,6 +176,7 @@ void write_solution(mgm_ctx *c, const char *path, int pressure_field)
 template <class F>
 int ioguard(F &&f)
 {
+    const TrimScope trim;
     try {
         f();
         return MGM_OK;

@@ -10,8 +10,9 @@
 // stream of the pool's own is used.
 //
 // What the pool keeps beyond the buffers in use is bounded: kIdleBytes after
-// each set-up and each destroyed object (trim_memory), nothing when an
-// allocation fails (it is given back and the allocation tried again).
+// each call that freed some, whether it succeeded or not (trim_memory at the
+// end of every entry point), nothing when an allocation fails (it is given
+// back and the allocation tried again).
 #include <mutex>
 
 #include "mgm_internal.cuh"
@@ -30,6 +31,7 @@ struct DevicePool {
 std::mutex g_mutex;
 DevicePool g_pools[kMaxDevices];
 thread_local cudaStream_t t_stream = nullptr;
+thread_local bool t_freed = false;  // a buffer since this thread's last trim
 
 void check(cudaError_t e, const char *what)
 {
@@ -86,6 +88,7 @@ void *dev_alloc(size_t bytes)
 void dev_free(void *ptr) noexcept
 {
     if (!ptr) return;
+    t_freed = true;
     cudaStream_t s = t_stream;
     if (!s) {
         cudaPointerAttributes at;
@@ -100,15 +103,19 @@ void dev_free(void *ptr) noexcept
 
 void trim_memory() noexcept
 {
+    if (!t_freed) return;
+    t_freed = false;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
     cudaMemPool_t pool;
+    cudaStream_t s;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         pool = g_pools[dev].pool;
         if (!pool) return;
-        if (!t_stream) cudaStreamSynchronize(g_pools[dev].idle);
+        s = t_stream ? t_stream : g_pools[dev].idle;
     }
+    cudaStreamSynchronize(s);  // memory is given back once the work before its free is done
     unsigned long long used = 0;
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
         cudaMemPoolTrimTo(pool, (size_t)used + kIdleBytes);

@@ -30,6 +30,7 @@ namespace {
 template <class F>
 int guard(F &&f)
 {
+    const TrimScope trim;
     try {
         f();
         return MGM_OK;
@@ -1692,7 +1693,6 @@ int mgm_setup(mgm_ctx *c, int flags)
         pipeline_transfer(c, c->have_ref_transfer);
         pipeline_derivatives(c);
         prepare_solver(c);
-        trim_memory();
     });
 }
 

@@ -88,13 +88,31 @@ void *dev_alloc(size_t bytes);
 void dev_free(void *p) noexcept;
 void trim_memory() noexcept;  // gives back what the pool holds beyond its bound
 
-// names a stream for a scope
-struct AllocScope {
-    cudaStream_t before;
-    explicit AllocScope(cudaStream_t s) : before(alloc_stream()) { alloc_stream(s); }
-    ~AllocScope() { alloc_stream(before); }
-    AllocScope(const AllocScope &) = delete;
-    AllocScope &operator=(const AllocScope &) = delete;
+// at the top of every entry point: the bound holds again when the call returns,
+// with an error too
+struct TrimScope {
+    TrimScope() = default;
+    ~TrimScope() { trim_memory(); }
+    TrimScope(const TrimScope &) = delete;
+    TrimScope &operator=(const TrimScope &) = delete;
+};
+
+// a call's own stream, named for the buffers declared after it
+struct CallStream {
+    cudaStream_t s = nullptr, before;
+    CallStream() : before(alloc_stream())
+    {
+        MGM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        alloc_stream(s);
+    }
+    ~CallStream()
+    {
+        alloc_stream(before);
+        cudaStreamSynchronize(s);  // the buffers' frees
+        cudaStreamDestroy(s);
+    }
+    CallStream(const CallStream &) = delete;
+    CallStream &operator=(const CallStream &) = delete;
 };
 
 // device buffer with RAII

@@ -1101,6 +1101,7 @@ extern "C" {
 
 int mgm_mpnn_init(mgm_ctx *c, unsigned long long seed, int dataset_capacity)
 {
+    const TrimScope trim;
     try {
         MGM_REQUIRE(c && c->setup_done, "mgm_mpnn_init: call mgm_setup first");
         MGM_REQUIRE(dataset_capacity >= 0, "mgm_mpnn_init: negative capacity");
@@ -1164,6 +1165,7 @@ int mgm_mpnn_num_params(void) { return kNumParams; }
 
 int mgm_mpnn_params(mgm_ctx *c, float *get, const float *set)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         cudaStream_t s = c->s;
@@ -1184,6 +1186,7 @@ int mgm_mpnn_params(mgm_ctx *c, float *get, const float *set)
 int mgm_mpnn_loss_grad(mgm_ctx *c, const float *b_hat, const float *p_hat, const float *dp_hat, const float *target,
                        double *loss, float *grads, float *prediction)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         cudaStream_t s = c->s;
@@ -1214,6 +1217,7 @@ int mgm_mpnn_loss_grad(mgm_ctx *c, const float *b_hat, const float *p_hat, const
 // the network's inference pass (the one a step runs) on normalised inputs
 int mgm_mpnn_predict(mgm_ctx *c, const float *b_hat, const float *p_hat, const float *dp_hat, float *prediction)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         MGM_REQUIRE(b_hat && p_hat && dp_hat && prediction, "mgm_mpnn_predict: null argument");
@@ -1238,6 +1242,7 @@ int mgm_mpnn_predict(mgm_ctx *c, const float *b_hat, const float *p_hat, const f
 // runs nsteps fractional steps with the given Poisson mode, recording (b, p_prev, p_new) samples
 int mgm_mpnn_collect(mgm_ctx *c, int mode, int nsteps)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         MGM_REQUIRE(M.ds_cap > 0, "mgm_mpnn_collect: dataset capacity is zero");
@@ -1261,6 +1266,7 @@ int mgm_mpnn_collect(mgm_ctx *c, int mode, int nsteps)
 
 int mgm_mpnn_dataset_size(mgm_ctx *c, int *count)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         *count = std::min(M.ds_count, M.ds_cap);
@@ -1275,6 +1281,7 @@ int mgm_mpnn_dataset_size(mgm_ctx *c, int *count)
 // seeded shuffled order; losses[it] (host, may be NULL) receives each iteration's loss.
 int mgm_mpnn_train(mgm_ctx *c, int first, int count, int iters, float lr, unsigned long long seed, double *losses)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         const int have = std::min(M.ds_count, M.ds_cap);
@@ -1307,6 +1314,7 @@ int mgm_mpnn_train(mgm_ctx *c, int first, int count, int iters, float lr, unsign
 // mean loss of the network on samples [first, first + count) (no update)
 int mgm_mpnn_eval(mgm_ctx *c, int first, int count, double *mean_loss)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         const int have = std::min(M.ds_count, M.ds_cap);
@@ -1336,6 +1344,7 @@ int mgm_mpnn_eval(mgm_ctx *c, int first, int count, double *mean_loss)
 
 int mgm_mpnn_set_loss(mgm_ctx *c, float w_mse, float w_res)
 {
+    const TrimScope trim;
     try {
         MpnnState &M = state(c);
         MGM_REQUIRE(w_mse >= 0 && w_res >= 0 && w_mse + w_res > 0, "mgm_mpnn_set_loss: weights must be >= 0, not both 0");
@@ -1350,6 +1359,7 @@ int mgm_mpnn_set_loss(mgm_ctx *c, float w_mse, float w_res)
 
 int mgm_set_warm_start(mgm_ctx *c, int enable)
 {
+    const TrimScope trim;
     try {
         MGM_REQUIRE(c, "null context");
         if (enable) {

@@ -445,6 +445,7 @@ namespace {
 template <class F>
 int tguard(F &&f)
 {
+    const TrimScope trim;
     try {
         f();
         return MGM_OK;
