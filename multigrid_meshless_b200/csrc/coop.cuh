@@ -1,5 +1,7 @@
 // coop.cuh -- cooperative launches and the bounded grid barrier of their kernels.
 #pragma once
+#include <algorithm>
+
 #include "mgm_internal.cuh"
 
 namespace mgm {
@@ -38,6 +40,18 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned &
     }
     __syncthreads();
     return ok != 0;
+}
+
+// CTAs of that size that the device (as much of it as the process may use)
+// holds at once: the most a cooperative launch may have
+template <class... P>
+inline int cooperative_ctas(void (*kern)(P...), int block, size_t smem)
+{
+    int dev = 0, sms = 0, per_sm = 0;
+    MGM_CUDA(cudaGetDevice(&dev));
+    MGM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MGM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
+    return std::max(1, sms * per_sm);
 }
 
 template <class... P, class... A>

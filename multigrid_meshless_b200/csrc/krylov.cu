@@ -990,9 +990,14 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_dense_inverse(int n, int k, 
         }
 }
 
-void dense_inverse(int n, int k, const int *idx, const double *A, double *inv64, float *inv32, cudaStream_t s)
+void dense_inverse(int n, int k, const int *idx, const double *A, double *inv64, float *inv32, cudaStream_t s,
+                   int most_ctas)
 {
-    const int grid = std::min(n, 148), maxr = (n + grid - 1) / grid;
+    constexpr size_t kMostSmem = 220 * 1024;
+    MGM_CUDA(cudaFuncSetAttribute(k_dense_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem));
+    // a candidate per thread: no more CTAs than threads
+    const int grid = std::min({n, most_ctas, kInvThreads, cooperative_ctas(k_dense_inverse, kInvThreads, kMostSmem)});
+    const int maxr = (n + grid - 1) / grid;
     // scaled pivot row, column entries, pivots, positions, and the rows where they fit
     const size_t head = sizeof(double) * (n + maxr) + sizeof(int) * ((size_t)n + (n & 1) + ((maxr + 1) & ~1));
     const size_t own = sizeof(double) * (size_t)maxr * n;
@@ -1003,7 +1008,6 @@ void dense_inverse(int n, int k, const int *idx, const double *A, double *inv64,
     DBuf<int> state(4);
     state.zero(s);
     const size_t smem = head + (fits ? own : 0);
-    MGM_CUDA(cudaFuncSetAttribute(k_dense_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     MGM_CUDA(launch_cooperative(k_dense_inverse, grid, kInvThreads, smem, s, n, k, idx, A, fits ? nullptr : M.p,
                                 cand_row.p, cand.p, state.p, inv64, inv32));
     MGM_LAUNCHED();

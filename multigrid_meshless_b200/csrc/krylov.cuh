@@ -21,7 +21,8 @@ template <class T>
 void copy_convert(long n, const double *in, T *out, cudaStream_t s);
 template <class T>
 void copy_out(long n, const T *in, T *out, cudaStream_t s);
-void dense_inverse(int n, int k, const int *idx, const double *A, double *inv64, float *inv32, cudaStream_t s);
+void dense_inverse(int n, int k, const int *idx, const double *A, double *inv64, float *inv32, cudaStream_t s,
+                   int most_ctas = kCoopCtas);
 
 // ---------------------------------------------------------------------------
 // Device-resident control of the outer flexible GMRES.  Every scalar of the

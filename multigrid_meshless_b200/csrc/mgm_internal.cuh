@@ -168,8 +168,11 @@ void knn_query(const GridIndex &g, const double *px, const double *py, const dou
                const double *qx, const double *qy, const double *qz, const int *self_id, int k, int mode,
                int *out, int ld, cudaStream_t s);
 
+// CTAs of the cooperative set-up kernels: one per SM, fewer where the process
+// sees fewer
+constexpr int kCoopCtas = 148;
 // breadth-first order (rcm_reordering_with_boundarynodes); returns reached count
-int bfs_order(int n, int k, const int *d_cloud_rowmajor, int *d_queue1, cudaStream_t s);
+int bfs_order(int n, int k, const int *d_cloud_rowmajor, int *d_queue1, cudaStream_t s, int most_ctas = kCoopCtas);
 void apply_order(int n, int k, const int *d_queue1, double *x, double *y, double *z, double *nx, double *ny,
                  double *nz, uint8_t *btag, int *cloud_rowmajor, cudaStream_t s);
 void correct_normals(int n, int k, const double *x, const double *y, const double *z, const uint8_t *btag,

@@ -373,13 +373,14 @@ __global__ void __launch_bounds__(kBfsThreads) k_bfs(int n, int k, const int *__
     if (blockIdx.x == 0 && tid == 0) state[3] = tail;
 }
 
-int bfs_order(int n, int k, const int *d_cloud, int *d_queue1, cudaStream_t s)
+int bfs_order(int n, int k, const int *d_cloud, int *d_queue1, cudaStream_t s, int most_ctas)
 {
     MGM_REQUIRE(n >= 1 && k >= 2, "bfs_order: bad sizes");
     DBuf<long long> key(n);
     k_bfs_init<<<blocks_for(n, 256), 256, 0, s>>>(n, key.p, d_queue1);
     MGM_LAUNCHED();
-    const int grid = std::max(1, std::min(148, n / 2048));  // a level's items, 4 or more a thread at most sizes
+    // a level's items, 4 or more a thread at most sizes
+    const int grid = std::max(1, std::min({most_ctas, n / 2048, cooperative_ctas(k_bfs, kBfsThreads, 0)}));
     DBuf<int> cnt(grid), state(5);
     state.zero(s);
     MGM_CUDA(launch_cooperative(k_bfs, grid, kBfsThreads, 0, s, n, k, d_cloud, d_queue1, key.p, cnt.p, state.p));
