@@ -6,10 +6,14 @@
 
 namespace mgm {
 
+#ifndef MGM_BARRIER_POLLS
+#define MGM_BARRIER_POLLS (1L << 20)
+#endif
+
 // Grid barrier of a cooperative launch (all CTAs resident): thread 0 of each
 // CTA arrives on a counter; the last arrival resets it and advances the
 // generation the others wait on (polled without sleeping: the wait is a few
-// microseconds).  The wait is bounded (2^20 polls of L2, under a second);
+// microseconds).  The wait is bounded (MGM_BARRIER_POLLS of L2, under a second);
 // when it runs out the CTA records the error and the kernel's CTAs
 // return at their next barrier.  Returns false once any CTA has given up.
 __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned &gen)
@@ -27,7 +31,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned &
         } else {
             long spins = 0;
             while (*(volatile unsigned *)&bar[1] == gen) {
-                if (++spins > (1L << 20) || ((spins & 255) == 0 && *(volatile int *)err)) {
+                if (++spins > MGM_BARRIER_POLLS || ((spins & 255) == 0 && *(volatile int *)err)) {
                     atomicExch(err, 1);
                     good = 0;
                     break;
@@ -68,6 +72,12 @@ inline cudaError_t launch_cooperative(void (*kern)(P...), int grid, int block, s
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+// after the launch: the error flag that its barriers set
+inline void check_barrier(int err, const char *what)
+{
+    if (err != 0) throw Error{4 /* MGM_ERR_TIMEOUT */, std::string(what) + ": a grid barrier's wait ran out"};
 }
 
 }  // namespace mgm

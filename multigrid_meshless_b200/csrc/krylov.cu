@@ -1014,7 +1014,7 @@ void dense_inverse(int n, int k, const int *idx, const double *A, double *inv64,
     int h[4];
     state.download(h, 4, s);
     MGM_CUDA(cudaStreamSynchronize(s));
-    if (h[2] != 0) throw Error{1, "dense inverse: a grid barrier's wait ran out"};
+    check_barrier(h[2], "dense inverse");
 }
 
 }  // namespace mgm

@@ -389,7 +389,7 @@ int bfs_order(int n, int k, const int *d_cloud, int *d_queue1, cudaStream_t s, i
     state.download(h, 5, s);
     MGM_CUDA(cudaStreamSynchronize(s));
     MGM_REQUIRE(h[4] == 0, "bfs_order: frontier too large");
-    if (h[2] != 0) throw Error{1, "bfs_order: a grid barrier's wait ran out"};
+    check_barrier(h[2], "bfs_order");
     MGM_REQUIRE(h[3] <= n, "bfs_order: queue overflow (corrupt cloud indices)");
     return h[3];
 }
