@@ -9,10 +9,12 @@
 // named (objects being destroyed, after their stream was synchronised) a
 // stream of the pool's own is used.
 //
-// What the pool keeps beyond the buffers in use is bounded: kIdleBytes after
-// each call that freed some, whether it succeeded or not (trim_memory at the
-// end of every entry point), nothing when an allocation fails (it is given
-// back and the allocation tried again).
+// What the pool keeps beyond the buffers in use is bounded by kIdleBytes (and
+// kTrimEvery for each further thread) when a call returns, whether it succeeded
+// or not: trim_memory, at the end of every entry point, gives back what is above
+// once its thread has freed kTrimEvery since the last time (a trim is a
+// synchronisation and two calls of the driver).  When an allocation fails all
+// of it is given back and the allocation tried again.
 #include <mutex>
 
 #include "mgm_internal.cuh"
@@ -21,7 +23,7 @@ namespace mgm {
 
 namespace {
 
-constexpr size_t kIdleBytes = size_t(2) << 30;
+constexpr size_t kIdleBytes = size_t(2) << 30, kTrimEvery = size_t(64) << 20;
 constexpr int kMaxDevices = 64;
 
 struct DevicePool {
@@ -31,7 +33,7 @@ struct DevicePool {
 std::mutex g_mutex;
 DevicePool g_pools[kMaxDevices];
 thread_local cudaStream_t t_stream = nullptr;
-thread_local bool t_freed = false;  // a buffer since this thread's last trim
+thread_local size_t t_freed = 0;  // bytes since this thread's last trim
 
 void check(cudaError_t e, const char *what)
 {
@@ -85,10 +87,10 @@ void *dev_alloc(size_t bytes)
     return ptr;
 }
 
-void dev_free(void *ptr) noexcept
+void dev_free(void *ptr, size_t bytes) noexcept
 {
     if (!ptr) return;
-    t_freed = true;
+    t_freed += bytes;
     cudaStream_t s = t_stream;
     if (!s) {
         cudaPointerAttributes at;
@@ -103,8 +105,8 @@ void dev_free(void *ptr) noexcept
 
 void trim_memory() noexcept
 {
-    if (!t_freed) return;
-    t_freed = false;
+    if (t_freed < kTrimEvery) return;
+    t_freed = 0;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
     cudaMemPool_t pool;
@@ -118,7 +120,7 @@ void trim_memory() noexcept
     cudaStreamSynchronize(s);  // memory is given back once the work before its free is done
     unsigned long long used = 0;
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
-        cudaMemPoolTrimTo(pool, (size_t)used + kIdleBytes);
+        cudaMemPoolTrimTo(pool, (size_t)used + kIdleBytes - kTrimEvery);
     cudaGetLastError();
 }
 

@@ -85,7 +85,7 @@ __device__ __forceinline__ T ell_row_dot(const int *__restrict__ idx, const T *_
 void alloc_stream(cudaStream_t s);
 cudaStream_t alloc_stream();
 void *dev_alloc(size_t bytes);
-void dev_free(void *p) noexcept;
+void dev_free(void *p, size_t bytes) noexcept;
 void trim_memory() noexcept;  // gives back what the pool holds beyond its bound
 
 // at the top of every entry point: the bound holds again when the call returns,
@@ -135,7 +135,7 @@ struct DBuf {
         if (count) p = static_cast<T *>(dev_alloc(count * sizeof(T)));
         n = count;
     }
-    void release() { dev_free(p); p = nullptr; n = 0; }
+    void release() { dev_free(p, n * sizeof(T)); p = nullptr; n = 0; }
     void zero(cudaStream_t s) { if (n) { cudaError_t e = cudaMemsetAsync(p, 0, n * sizeof(T), s); if (e != cudaSuccess) throw Error{1, cudaGetErrorString(e)}; } }
     void upload(const T *h, size_t count, cudaStream_t s) {
         if (count > n) alloc(count);
