@@ -436,16 +436,59 @@ __global__ void __launch_bounds__(256) k_decode_bwd(int n, const bf16 *__restric
 // the CUDA cores.  The small parts are accumulated before the large one, and a
 // tile's sums start from zero and are added to the running FP32 sums, which
 // keeps the tensor cores' truncating accumulation to 4 steps at full size.
-__device__ __forceinline__ void split3(float2 v, uint32_t (&p)[3])
+//
+// Values that BF16 would round to an infinity are cut instead of rounded (the
+// parts' sum is exact either way); an infinity or a NaN is in all three parts,
+// so that its products are what FP32 makes of them (a part of zero would turn
+// them into NaN, and so would the infinity's own remainder).
+__device__ __forceinline__ void split3_wide(float v, unsigned short (&p)[3])
 {
+    const bool finite = fabsf(v) < INFINITY;
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        const __nv_bfloat162 b = __floats2bfloat162_rn(v.x, v.y);
-        const float2 f = __bfloat1622float2(b);
-        p[q] = *reinterpret_cast<const uint32_t *>(&b);
-        v.x -= f.x;
-        v.y -= f.y;
+        const float f = finite ? __uint_as_float(__float_as_uint(v) & 0xffff0000u) : v;
+        p[q] = __bfloat16_as_ushort(__float2bfloat16_rn(f));
+        if (finite) v -= f;
     }
+}
+
+// values that need split3_wide
+__device__ __forceinline__ bool beyond_bf16(float4 v)
+{
+    constexpr float kMax = 0x1.fep127f;
+    return !(fabsf(v.x) <= kMax) | !(fabsf(v.y) <= kMax) | !(fabsf(v.z) <= kMax) | !(fabsf(v.w) <= kMax);
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void split3(float2 v, uint32_t (&p)[3])
+{
+    if constexpr (WIDE) {
+        unsigned short x[3], y[3];
+        split3_wide(v.x, x);
+        split3_wide(v.y, y);
+#pragma unroll
+        for (int q = 0; q < 3; q++) p[q] = x[q] | (uint32_t)y[q] << 16;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v.x, v.y);
+            const float2 f = __bfloat1622float2(b);
+            p[q] = *reinterpret_cast<const uint32_t *>(&b);
+            v.x -= f.x;
+            v.y -= f.y;
+        }
+    }
+}
+
+// the three parts of four columns of a row, into shared memory (parts `stride` apart)
+template <bool WIDE>
+__device__ __forceinline__ void store_parts(float4 v, bf16 *to, int stride)
+{
+    uint32_t lo[3], hi[3];
+    split3<WIDE>(make_float2(v.x, v.y), lo);
+    split3<WIDE>(make_float2(v.z, v.w), hi);
+#pragma unroll
+    for (int p = 0; p < 3; p++) *reinterpret_cast<uint2 *>(to + p * stride) = make_uint2(lo[p], hi[p]);
 }
 
 __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3)
@@ -504,20 +547,22 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW(int n, const float *__rest
     fetch((long)blockIdx.x * kTile);
     for (long base = (long)blockIdx.x * kTile; base < n; base += (long)gridDim.x * kTile) {
         __syncthreads();
+        float4 d[2];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int row = row0 + 32 * u;
-            const float4 d = make_float4(zz[u].x > 0.f ? h[u].x : 0.f, zz[u].y > 0.f ? h[u].y : 0.f,
-                                         zz[u].z > 0.f ? h[u].z : 0.f, zz[u].w > 0.f ? h[u].w : 0.f);
-            gb[0] += d.x; gb[1] += d.y; gb[2] += d.z; gb[3] += d.w;
-            if (base + row < n) *reinterpret_cast<float4 *>(dz + (base + row) * kH + c4) = d;
-            uint32_t lo[3], hi[3];
-            split3(make_float2(d.x, d.y), lo);
-            split3(make_float2(d.z, d.w), hi);
-#pragma unroll
-            for (int p = 0; p < 3; p++)
-                *reinterpret_cast<uint2 *>(Ds + (p * kTile + row) * kPadH + c4) = make_uint2(lo[p], hi[p]);
+            d[u] = make_float4(zz[u].x > 0.f ? h[u].x : 0.f, zz[u].y > 0.f ? h[u].y : 0.f,
+                               zz[u].z > 0.f ? h[u].z : 0.f, zz[u].w > 0.f ? h[u].w : 0.f);
+            gb[0] += d[u].x; gb[1] += d[u].y; gb[2] += d[u].z; gb[3] += d[u].w;
+            if (base + row < n) *reinterpret_cast<float4 *>(dz + (base + row) * kH + c4) = d[u];
         }
+        auto parts = [&](auto WIDE) {
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                store_parts<decltype(WIDE)::value>(d[u], Ds + (row0 + 32 * u) * kPadH + c4, kTile * kPadH);
+        };
+        if (beyond_bf16(d[0]) | beyond_bf16(d[1])) parts(std::true_type{});
+        else parts(std::false_type{});
 #pragma unroll
         for (int u = 0; u < 3; u++) {
             const int e = tid + u * kDwThreads;
@@ -658,17 +703,17 @@ __global__ void __launch_bounds__(256, 2) k_back(int n, int k, float inv_k, cons
 #pragma unroll
     for (int part = 0; part < 3; part++) {  // self, mean, lap
         __syncthreads();
+        bool wide = false;
 #pragma unroll
-        for (int rr = 0; rr < kTile / 16; rr++) {
-            const int row = warp * (kTile / 8) + rr * 2 + half;
-            const float4 f = S[rr][part];
-            uint32_t a[3], b[3];
-            split3(make_float2(f.x, f.y), a);
-            split3(make_float2(f.z, f.w), b);
+        for (int rr = 0; rr < kTile / 16; rr++) wide |= beyond_bf16(S[rr][part]);
+        auto parts = [&](auto WIDE) {
 #pragma unroll
-            for (int p = 0; p < 3; p++)
-                *reinterpret_cast<uint2 *>(Xs + (p * kTile + row) * kPadH + 4 * hl) = make_uint2(a[p], b[p]);
-        }
+            for (int rr = 0; rr < kTile / 16; rr++)
+                store_parts<decltype(WIDE)::value>(
+                    S[rr][part], Xs + (warp * (kTile / 8) + rr * 2 + half) * kPadH + 4 * hl, kTile * kPadH);
+        };
+        if (wide) parts(std::true_type{});
+        else parts(std::false_type{});
         __syncthreads();
         float acc[4][4] = {};
 #pragma unroll
