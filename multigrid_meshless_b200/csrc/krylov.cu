@@ -381,8 +381,9 @@ __global__ void __launch_bounds__(kFgThreads) k_fg_reduce(const double *part, in
 
 // a row of the operator in the level's own slot order: KC > 0 int16 offsets in
 // padded rows, the first KC slots before the wait; KC = 0 by chunks of 8
-// (IDX: 32-bit indices)
-template <int KC, bool IDX>
+// (IDX: 32-bit indices).  SMALL: in a kernel that releases its successor before
+// its own wait, which gathers from L2.
+template <int KC, bool IDX, bool SMALL>
 struct FgRow {
     RowChunk<double, KC ? KC : 8, IDX> R;
     __device__ __forceinline__ void fetch(const FgOperator &op, int i)
@@ -397,7 +398,7 @@ struct FgRow {
             const double s = R.template dot<true>(x, 0.0);
             return row_rest<true, double, KC, IDX>(op.gi, op.A, x, op.n, op.kp, i, i, s);
         } else {
-            return row_big<double, IDX>(R, op.gi, op.A, x, op.n, op.k, i, i);
+            return row_big<double, IDX, SMALL>(R, op.gi, op.A, x, op.n, op.k, i, i);
         }
     }
 };
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(kFgThreads) k_fg_apply(FgOperator op, const T 
 {
     __shared__ double sm[kFgChunk][kFgWarps];
     const int i0 = blockIdx.x * kFgThreads + threadIdx.x, i = min(i0, op.n - 1);
-    FgRow<KC, IDX> R;
+    FgRow<KC, IDX, SMALL> R;
     R.fetch(op, i);
     pdl_wait<SMALL>();
     const int j = __ldcg(&st->j_next);
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(256) k_fg_resid(FgOperator op, const double *_
 {
     __shared__ double sm[32];
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x, i = min(i0, op.n - 1);
-    FgRow<KC, IDX> R;
+    FgRow<KC, IDX, false> R;
     R.fetch(op, i);
     const double bi = b[i];
     asm volatile("" ::: "memory");  // the operator loads above stay ahead of the gathers

@@ -130,12 +130,13 @@ __device__ __forceinline__ T row_rest(const void *gi, const T *A, const X *x, lo
     return s;
 }
 
-// a whole row of k slots, 8 at a time, none beyond k read (the large levels),
+// a whole row of k slots, 8 at a time, none beyond k read (the large levels, and
+// level 0 with 32-bit indices at any size, where EARLY says how to gather),
 // the next 8 slots' operator in flight during the current gathers; R: the first
 // chunk, by fetch_to (prolongation to 1M rows of 30 slots: 63 us with each
 // chunk's loads after the last one's gathers and the last k mod 8 slots one by
 // one, now 45)
-template <class T, bool IDX, class X>
+template <class T, bool IDX, bool EARLY, class X>
 __device__ __forceinline__ T row_big(RowChunk<T, 8, IDX> &R, const void *gi, const T *A, const X *x, long ld, int k,
                                      long i, int base)
 {
@@ -146,7 +147,7 @@ __device__ __forceinline__ T row_big(RowChunk<T, 8, IDX> &R, const void *gi, con
         if (j + 8 < k) N.fetch_to(gi, A, ld, i, base, j + 8, k);
         else N = R;
 #pragma unroll
-        for (int q = 0; q < 8; q++) v[q] = __ldg(x + R.c[q]);
+        for (int q = 0; q < 8; q++) v[q] = gather<EARLY>(x + R.c[q]);
 #pragma unroll
         for (int q = 0; q < 8; q++)
             if (j + q < k) s = fma_rn(R.a[q], (T)v[q], s);

@@ -783,7 +783,7 @@ struct TransferRow {
             return row_rest<true, T, KC, IDX>(a.gi, a.w, a.in, a.n, a.kp, i, base, s);
         } else {
             static_assert(KC == 8, "row_big takes chunks of 8");
-            return row_big<T, IDX>(R, a.gi, a.w, a.in, a.n, a.k, i, base);
+            return row_big<T, IDX, false>(R, a.gi, a.w, a.in, a.n, a.k, i, base);
         }
     }
 };
