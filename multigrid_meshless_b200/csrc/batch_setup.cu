@@ -16,7 +16,6 @@
 // (weights.cuh), i.e. of rbf.h:42-421 and mesh_functions.h:533-670; the
 // stencil of node i is the first k_i entries of its nearest-node list.
 #include <algorithm>
-#include <cstring>
 #include <numeric>
 
 #include "batch.cuh"
@@ -34,8 +33,12 @@ struct BLevelDev {
     MonoDev mono;
 };
 
-__constant__ BLevelDev c_blev[kBatchMaxLevels];
-__constant__ int c_bdim, c_bphs;
+// a kernel argument (constant memory of its launch): set-ups of several threads
+// each have their own
+struct BatchTable {
+    BLevelDev lev[kBatchMaxLevels];
+    int dim, phs;
+};
 
 struct WTask {
     int code;  // level | kind << 4 ; kind 0 derivative row, 1 restriction row, 2 prolongation row
@@ -43,12 +46,12 @@ struct WTask {
 };
 
 // One system, solved by team tm in the shared-memory slot `slot`.
-__device__ void solve_system(const Team &tm, WTask task, double *slot)
+__device__ void solve_system(const BatchTable &tab, const Team &tm, WTask task, double *slot)
 {
-    const int dim = c_bdim, phs = c_bphs;
+    const int dim = tab.dim, phs = tab.phs;
     const int lev = task.code & 15, kind = task.code >> 4, i = task.row;
-    const BLevelDev &T = c_blev[lev];
-    const BLevelDev &S = c_blev[kind == 0 ? lev : (kind == 1 ? lev - 1 : lev + 1)];
+    const BLevelDev &T = tab.lev[lev];
+    const BLevelDev &S = tab.lev[kind == 0 ? lev : (kind == 1 ? lev - 1 : lev + 1)];
     const int ip = kind == 0 ? i : (kind == 1 ? T.rpts[i] : T.ppts[i]);
     const int m = S.kk[ip], np = S.mono.np, N = m + np;
     double *aug = slot;
@@ -102,7 +105,8 @@ __device__ void solve_system(const Team &tm, WTask task, double *slot)
 }
 
 // tiles[t] = {first task, systems in the tile, threads per system, slot bytes}
-__global__ void __launch_bounds__(kBatchCta) k_weights_persistent(const int4 *__restrict__ tiles, int ntiles,
+__global__ void __launch_bounds__(kBatchCta) k_weights_persistent(const __grid_constant__ BatchTable tab,
+                                                                  const int4 *__restrict__ tiles, int ntiles,
                                                                   const WTask *__restrict__ tasks, int *counter)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -116,7 +120,7 @@ __global__ void __launch_bounds__(kBatchCta) k_weights_persistent(const int4 *__
         const int team = tile.z, grp = threadIdx.x / team;
         if (grp < tile.y) {
             const Team tm{(int)threadIdx.x % team, team, team == kBatchCta ? 0 : 1 + grp};
-            solve_system(tm, tasks[tile.x + grp], (double *)(smraw + (size_t)grp * tile.w));
+            solve_system(tab, tm, tasks[tile.x + grp], (double *)(smraw + (size_t)grp * tile.w));
         }
         __syncthreads();
     }
@@ -143,13 +147,12 @@ int num_sms()
     return std::max(1, v);
 }
 
-void upload_level_table(mgm_batch *b)
+BatchTable level_table(mgm_batch *b)
 {
-    BLevelDev d[kBatchMaxLevels];
-    std::memset(d, 0, sizeof(d));
+    BatchTable t{};
     for (int l = 0; l < b->nl; l++) {
         BLevel &L = b->L[l];
-        BLevelDev &o = d[l];
+        BLevelDev &o = t.lev[l];
         o.n = L.n; o.kmax = L.kmax;
         o.x = L.x.p; o.y = L.y.p; o.z = L.z.p; o.nx = L.nx.p; o.ny = L.ny.p; o.nz = L.nz.p;
         o.btag = L.btag.p; o.kk = L.kk.p; o.cloud = L.cloud.p; o.rp = L.rp.p;
@@ -158,9 +161,9 @@ void upload_level_table(mgm_batch *b)
         o.r_w = L.r_w64.p; o.p_w = L.p_w64.p;
         o.mono = to_dev(monomials(b->dim, L.poly));
     }
-    MGM_CUDA(cudaMemcpyToSymbolAsync(c_blev, d, sizeof(d), 0, cudaMemcpyHostToDevice, b->s));
-    MGM_CUDA(cudaMemcpyToSymbolAsync(c_bdim, &b->dim, sizeof(int), 0, cudaMemcpyHostToDevice, b->s));
-    MGM_CUDA(cudaMemcpyToSymbolAsync(c_bphs, &b->phs, sizeof(int), 0, cudaMemcpyHostToDevice, b->s));
+    t.dim = b->dim;
+    t.phs = b->phs;
+    return t;
 }
 
 // kNN lists with k_max entries, breadth-first reorder, normals, CSR structure
@@ -268,7 +271,8 @@ void make_tiles(std::vector<int4> &tiles, long long first, long long count, int 
         tiles.push_back(make_int4((int)(first + q), (int)std::min<long long>(g, count - q), kBatchCta / g, slot));
 }
 
-double run_tiles(const std::vector<int4> &tiles, const WTask *d_tasks, int smem, int grid, cudaStream_t s)
+double run_tiles(const BatchTable &tab, const std::vector<int4> &tiles, const WTask *d_tasks, int smem, int grid,
+                 cudaStream_t s)
 {
     if (tiles.empty()) return 0.0;
     DBuf<int4> dt;
@@ -280,7 +284,7 @@ double run_tiles(const std::vector<int4> &tiles, const WTask *d_tasks, int smem,
     MGM_CUDA(cudaEventCreate(&e1));
     MGM_CUDA(cudaEventRecord(e0, s));
     k_weights_persistent<<<std::max(1, std::min<int>(grid, (int)tiles.size())), kBatchCta, smem, s>>>(
-        dt.p, (int)tiles.size(), d_tasks, counter.p);
+        tab, dt.p, (int)tiles.size(), d_tasks, counter.p);
     MGM_LAUNCHED();
     MGM_CUDA(cudaEventRecord(e1, s));
     MGM_CUDA(cudaEventSynchronize(e1));
@@ -337,7 +341,7 @@ void batch_setup(mgm_batch *b, bool autotune)
             L.p_w64.alloc((size_t)std::max<long long>(L.p_nnz, 1));
         }
     }
-    upload_level_table(b);
+    const BatchTable tab = level_table(b);
     // task list, bucketed by system order N (largest first)
     std::vector<std::vector<WTask>> bucket(kMaxN + 1);
     std::vector<int> max_m(kMaxN + 1, 0);
@@ -396,7 +400,7 @@ void batch_setup(mgm_batch *b, bool autotune)
                 const long long sample = std::min<long long>(count, (long long)sms * bud[bi].ctas * g * 2);
                 std::vector<int4> tl;
                 make_tiles(tl, span[N].first, sample, g, slot);
-                const double ms = run_tiles(tl, d_tasks.p, bud[bi].smem, sms * bud[bi].ctas, s);
+                const double ms = run_tiles(tab, tl, d_tasks.p, bud[bi].smem, sms * bud[bi].ctas, s);
                 b->tuning_ms += ms;
                 const double per = ms * 1e3 / (double)sample;
                 if (per < tbest) { tbest = per; gbest = g; }
@@ -428,7 +432,7 @@ void batch_setup(mgm_batch *b, bool autotune)
     b->tiles = (int)tiles.size();
     b->smem_bytes = B.smem;
     b->ctas_per_sm = B.ctas;
-    b->weights_ms = run_tiles(tiles, d_tasks.p, B.smem, sms * B.ctas, s);
+    b->weights_ms = run_tiles(tab, tiles, d_tasks.p, B.smem, sms * B.ctas, s);
     batch_prepare_solver(b);
     b->setup_done = true;
 }
