@@ -228,11 +228,20 @@ inline void launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cud
 
 // Programmatic dependent launch (griddepcontrol, sm_90 and later).  A kernel
 // launched by launch_pdl may have its CTAs scheduled while its predecessor on
-// the stream is still finishing; pdl_enter, its first statement, waits until
-// the predecessor grid has completed and its memory operations are visible,
-// then allows the kernel's own successor to be scheduled early.  Launched
-// the ordinary way, pdl_enter returns at once.  Every kernel launched by
-// launch_pdl calls pdl_enter before it reads or writes any buffer.
+// the stream is still finishing.  Its wait (pdl_enter here, pdl_wait of rows.cuh)
+// returns once the predecessor grid has completed and its memory operations are
+// visible; launched the ordinary way, it returns at once.  What the chained
+// kernels must keep to:
+//   - every thread executes the wait, also one that returns early, before it
+//     writes anything: a completed kernel then means that all before it have
+//     completed, which the write-after-read hazards of the chain rely on;
+//   - before the wait only what set-up wrote is read (operators, indices, lists,
+//     tags, diagonals).  Set-up ends with a synchronisation, and the first launch
+//     of a chain is an ordinary one;
+//   - a kernel that allows its successor before its own wait (pdl_wait<true>)
+//     may be resident with several others of the chain and gathers vectors from
+//     L2, not through L1.
+// pdl_enter: the wait first, the successor allowed after it.
 __device__ __forceinline__ void pdl_enter()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -257,11 +266,11 @@ inline void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, c
     MGM_LAUNCHED();
 }
 
-// The launches of one V-cycle or smoothing pass.  With chaining enabled,
-// a kernel whose predecessor on the stream is a kernel of the same chain is
-// launched by launch_pdl (such kernels begin with pdl_enter); the first
-// launch of a chain, and a launch after an event record (broken()), is an
-// ordinary launch.
+// The launches of one V-cycle, Arnoldi step, smoothing pass or reference cycle.
+// With chaining enabled, a kernel whose predecessor on the stream is a kernel of
+// the same chain is launched by launch_pdl (and keeps to its rules); the first
+// launch of a chain, and a launch after an event record or a copy (broken()), is
+// an ordinary launch.
 struct Chain {
     bool enabled = false;
     bool after_kernel = false;
@@ -272,7 +281,7 @@ struct Chain {
         else launch_k(kern, grid, block, smem, s, args...);
         after_kernel = true;
     }
-    // an ordinary launch of a kernel without pdl_enter inside the chain
+    // an ordinary launch of a kernel without the wait inside the chain
     template <class... P, class... A>
     void plain(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
     {

@@ -359,7 +359,7 @@ __device__ __forceinline__ T ell_row_dot_o(const short *__restrict__ off, const 
 // Levels below kVecMinRows rows: two chained launches (k_bnd_exact,
 // k_level_c1), each with its operands in registers before its wait.
 // The larger levels (k_level_v4): one launch in three parts --
-//   boundary  a warp per boundary row: e[b] (and out[b]); then one release
+//   boundary  8 lanes per boundary row: e[b] (and out[b]); then one release
 //             increment of sync[0] per CTA;
 //   far       the interior rows without boundary neighbours;
 //   near      a thread per near row, after a bounded wait for the boundary

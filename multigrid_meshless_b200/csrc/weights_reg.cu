@@ -23,11 +23,12 @@
 // symmetric RBF block, the scaling of the left half.
 //
 // Bound: latency at 24 warps per SM, then the shared-memory words of t (12
-// broadcast 16-byte loads per 48 FP64 instructions of a warp).  Measured, 30
-// nodes with 15 monomials: 76.5 ns per system against 209 in shared memory (20
-// nodes with 10: 34 against 92), 94 with the division after the update; a whole
-// column per thread (12 warps per SM) 101, two warps per 32 columns with t
-// computed by every warp 113.
+// broadcast 16-byte loads per 48 FP64 instructions of a warp).  Measured on 20k
+// systems, 30 nodes with 15 monomials: 76.9 ns per system against 212 in shared
+// memory (20 nodes with 10: 33.4 against 92.9; 47 with 15: 173 against 682),
+// 86.1 with the division after the update.  Before the operators' rows were one
+// pass, with the division after the update: 94, a whole column per thread (12
+// warps per SM) 101, two warps per 32 columns with t computed by every warp 113.
 #include <algorithm>
 
 #include "mgm_internal.cuh"
@@ -77,9 +78,9 @@ __device__ __forceinline__ double div_by(double a, double b, double y, bool usab
 }
 
 // Orders above 32 give the division its own warp, which works a step ahead: 8
-// CTAs per SM hide the division's chain at order 30 (33.9 ns per system, 35.2
-// with the warp), 4 or fewer do not (order 35 54.9 -> 53.2, 45 88.0 -> 76.5, 53
-// 184 -> 160, 62 228 -> 183).
+// CTAs per SM hide the division's chain at order 30 (33.4 ns per system, 37.0
+// with the warp), 4 or fewer do not (order 35 60.4 -> 52.9, 45 86.1 -> 76.9, 53
+// 179 -> 150, 62 219 -> 173).
 constexpr bool reg_ahead(int NT) { return NT > 32; }
 // a warp per 16 columns, and the warp that divides
 constexpr int reg_threads(int NT, int cols) { return (cols + 15) / 16 * 32 + (reg_ahead(NT) ? 32 : 0); }
