@@ -44,15 +44,7 @@ __device__ __forceinline__ double block_sum_d(double v, double *sm)
 // ---------------------------------------------------------------------------
 // Row work of the V-cycle kernels, shared by the one-operation kernels and
 // the fused coarse-level V-cycle (k_coarse_vcycle), which therefore give the
-// same bits.  COH: the vectors (r, e, d, q) are loaded from L2, past the
-// SM's L1 and the read-only path -- in the fused kernel other CTAs rewrite
-// them between passes; the operators are read-only throughout.
-template <bool COH, class T>
-__device__ __forceinline__ T ldv(const T *p)
-{
-    if constexpr (COH) return __ldcg(p);
-    else return *p;
-}
+// same bits.
 
 // A boundary row by the lanes of a warp: its stencil (fetch: the first 64
 // slots), then its exact solve from the current e (value: lane 0).  A
@@ -308,11 +300,11 @@ __device__ __forceinline__ T row0_dot_warp(int k, Op operand)
 // compact FP32 path: FP32 weights, neighbours stored as int16 offsets c - base
 // (6 bytes per stencil slot instead of 8)
 // ---------------------------------------------------------------------------
-// The gathered vector x is read through the read-only path unless COHERENT
-// (the fused coarse V-cycle, where other CTAs rewrite x between passes).
-template <class T, class X, bool COHERENT = false>
-__device__ __forceinline__ T ell_row_dot_o(const short *__restrict__ off, const T *__restrict__ A,
-                                           const X *__restrict__ x, long n, int k, long i, int base)
+// A row of the fused coarse V-cycle: the vectors are loaded from L2, past the
+// SM's L1 and the read-only path, because other CTAs rewrite them between passes.
+template <class T>
+__device__ __forceinline__ T ell_row_dot_o(const short *__restrict__ off, const T *__restrict__ A, const T *x, long n,
+                                           int k, long i, int base)
 {
     T s = T(0);
     int j = 0;
@@ -326,11 +318,11 @@ __device__ __forceinline__ T ell_row_dot_o(const short *__restrict__ off, const 
             a[q] = __ldg(A + o);
         }
 #pragma unroll
-        for (int q = 0; q < 8; q++) s = fma_rn(a[q], (T)(COHERENT ? __ldcg(x + c[q]) : __ldg(x + c[q])), s);
+        for (int q = 0; q < 8; q++) s = fma_rn(a[q], __ldcg(x + c[q]), s);
     }
     for (; j < k; j++) {
         const long o = (long)j * n + i;
-        s = fma_rn(A[o], (T)ldv<COHERENT>(x + base + (int)off[o]), s);
+        s = fma_rn(A[o], __ldcg(x + base + (int)off[o]), s);
     }
     return s;
 }
@@ -718,32 +710,32 @@ static void launch_c1(const SolveLevel<T> &L, T *e, T *out, T c1, T c2, int firs
     else launch(k_level_c1<MODE, T, 40, IDX>, grid, 128, 0, s, a);
 }
 
-template <class T, bool COHERENT = false>
+// the fused coarse V-cycle's transfers and dense solve (vectors from L2)
+template <class T>
 __device__ __forceinline__ void restrict_row(int i, int n, int k, const short *__restrict__ off,
                                              const int *__restrict__ base, const T *__restrict__ rw,
-                                             const uint8_t *__restrict__ btag, const T *__restrict__ qf,
-                                             T *__restrict__ rc)
+                                             const uint8_t *__restrict__ btag, const T *qf, T *rc)
 {
     if (btag[i] || i == 0) { rc[i] = T(0); return; }
-    rc[i] = ell_row_dot_o<T, T, COHERENT>(off, rw, qf, n, k, i, base[i]);
+    rc[i] = ell_row_dot_o(off, rw, qf, n, k, i, base[i]);
 }
 // (P e_c)[0] of the compact prolongation, by warp 0 of a CTA (row0_dot_warp)
-template <class T, bool COH = false>
+template <class T>
 __device__ __forceinline__ T prolong_shift_warp(int n, int k, const short *__restrict__ off,
                                                 const int *__restrict__ base, const T *__restrict__ pw, const T *ec)
 {
     const int b0 = base[0];
     return row0_dot_warp<T>(k, [&](int j, T &a, T &x) {
         a = pw[(long)j * n];
-        x = ldv<COH>(ec + b0 + (int)off[(long)j * n]);
+        x = __ldcg(ec + b0 + (int)off[(long)j * n]);
     });
 }
-template <class T, bool COHERENT = false>
+template <class T>
 __device__ __forceinline__ void prolong_row(int i, int n, int k, const short *__restrict__ off,
                                             const int *__restrict__ base, const T *__restrict__ pw, const T *ec, T *ef,
                                             T shift)
 {
-    ef[i] = ldv<COHERENT>(ef + i) + (ell_row_dot_o<T, T, COHERENT>(off, pw, ec, n, k, i, base[i]) - shift);
+    ef[i] = __ldcg(ef + i) + (ell_row_dot_o(off, pw, ec, n, k, i, base[i]) - shift);
 }
 
 // Restriction into a level: r_c[i] = sum_j Rw[j][i] q_f[...] on interior rows
@@ -1185,12 +1177,12 @@ static void launch_tiled(const SolveLevel<float> &L, const float *e, float *out,
 }
 
 // e = inv * r, one warp per row of the dense coarsest inverse
-template <class T, bool COH = false>
+template <class T>
 __device__ __forceinline__ void dense_row_warp(int w, int lane, int n, const T *__restrict__ inv, const T *r, T *e)
 {
     const T *row = inv + (long)w * n;
     T s = T(0);
-    for (int j = lane; j < n; j += 32) s += row[j] * ldv<COH>(r + j);
+    for (int j = lane; j < n; j += 32) s += row[j] * __ldcg(r + j);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) e[w] = s;
 }
@@ -1296,7 +1288,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_coarse_vcycle(const __grid_co
                 out[i] = mode == 0 ? ei : T(0);
                 continue;
             }
-            const T s = ell_row_dot_o<T, T, true>(L.off, L.A, e, L.ld, L.k, i, i);
+            const T s = ell_row_dot_o(L.off, L.A, e, L.ld, L.k, i, i);
             const T ri = __ldcg(L.r + i), dprev = mode == 0 && !first ? __ldcg(L.d + i) : T(0);
             if (mode == 0) step_out<0>(g, i, ri, ei, dprev, L.dinv[i], s);
             else step_out<1>(g, i, ri, ei, dprev, L.dinv[i], s);
@@ -1332,23 +1324,23 @@ __global__ void __launch_bounds__(kFusedThreads) k_coarse_vcycle(const __grid_co
         if (!smooth(l, true)) return;
         if (!pass(l, 1, T(0), T(0), 0, L.q)) return;
         for (int i = tid; i < C.n; i += nth)
-            restrict_row<T, true>(i, C.n, C.kr, C.r_off, C.r_base, C.r_w, C.btag, L.q, C.r);
+            restrict_row<T>(i, C.n, C.kr, C.r_off, C.r_base, C.r_w, C.btag, L.q, C.r);
         MGM_SYNC();
     }
     {
         const FusedLevel<T> &L = a.L[a.nl - 1];
-        for (int w = wid; w < a.cn; w += nwarp) dense_row_warp<T, true>(w, lane, a.cn, a.cinv, L.r, cur[a.nl - 1]);
+        for (int w = wid; w < a.cn; w += nwarp) dense_row_warp<T>(w, lane, a.cn, a.cinv, L.r, cur[a.nl - 1]);
         MGM_SYNC();
     }
     for (int l = a.nl - 2; l >= a.first; l--) {
         const FusedLevel<T> &L = a.L[l];
         if (threadIdx.x < 32) {
-            const T s = prolong_shift_warp<T, true>(L.n, L.kp, L.p_off, L.p_base, L.p_w, (const T *)cur[l + 1]);
+            const T s = prolong_shift_warp<T>(L.n, L.kp, L.p_off, L.p_base, L.p_w, (const T *)cur[l + 1]);
             if (threadIdx.x == 0) shift = s;
         }
         __syncthreads();
         for (int i = tid; i < L.n; i += nth)
-            prolong_row<T, true>(i, L.n, L.kp, L.p_off, L.p_base, L.p_w, (const T *)cur[l + 1], cur[l], shift);
+            prolong_row<T>(i, L.n, L.kp, L.p_off, L.p_base, L.p_w, (const T *)cur[l + 1], cur[l], shift);
         MGM_SYNC();
         if (!smooth(l, false)) return;
     }
