@@ -19,6 +19,11 @@ namespace mgm {
 
 constexpr int kBatchMaxRestart = 32;
 constexpr int kRowThreads = 768;  // most threads of a row kernel's CTA
+// Threads of the CTAs that gather rows of `bytes` per lane, two CTAs per SM: with
+// 768 the 64-column FP64 kernels have 40 registers, too few for their eight
+// gathers in flight (step of 107k rows 192 us, with 512 threads and 62 registers
+// 146; 181 in CTAs of 256).
+constexpr int row_threads(size_t bytes) { return bytes >= 16 ? 512 : kRowThreads; }
 
 template <class T, int Q>
 __device__ __forceinline__ void ldq(const T *p, T (&v)[Q])
@@ -114,19 +119,20 @@ __device__ __forceinline__ void row_dot_b(const int *__restrict__ col, const T *
 // Row-kernel shape: a CTA owns rpc consecutive rows, its warps step through
 // them together (warp w: rows w, w + warps, ...).  In the breadth-first order
 // consecutive rows share most neighbours, so a long run of rows per CTA has its
-// gathers served from L1: two CTAs of 24 warps per SM with all rows split among
-// them (FP32 step of 107k rows x 64 columns: 65% L1 hits, 80 us; 64 rows per
-// 8-warp CTA had 49%).  That needs about two rows per warp; below it, as for the
+// gathers served from L1: two CTAs of 24 warps (16 in FP64 with 64 columns) per SM
+// with all rows split among them (FP32 step of 107k rows x 64 columns 83 us, 51%
+// L1 hits; before the pairs went through shared memory the shape took the hits of
+// 64 rows per 8-warp CTA from 49% to 65%).  That needs about two rows per warp; below it, as for the
 // boundary rows, fewer warps per CTA and one or two rows per warp keep every SM
 // busy (3.6k boundary rows: 11 us, 17 as large CTAs).
 struct RowShape {
     int grid, threads, rpc;
 };
-inline RowShape row_shape(long rows)
+inline RowShape row_shape(long rows, size_t bytes)
 {
     if (rows >= 2L * 148 * 40) {
         const int rpc = (int)((rows + 295) / 296);
-        return {blocks_for(rows, rpc), kRowThreads, rpc};
+        return {blocks_for(rows, rpc), row_threads(bytes), rpc};
     }
     const int rpc = rows <= 8L * 148 * 5 ? 8 : 16;
     return {blocks_for(rows, rpc), 256, rpc};
@@ -137,7 +143,7 @@ inline RowShape row_shape(long rows)
 
 // exact solve of the boundary rows (they couple only to themselves and interior nodes)
 template <class T, int Q>
-__global__ void __launch_bounds__(kRowThreads, 2) k_b_bnd(int nbl, const int *__restrict__ list, const int *__restrict__ rp,
+__global__ void __launch_bounds__(row_threads(sizeof(T) * Q), 2) k_b_bnd(int nbl, const int *__restrict__ list, const int *__restrict__ rp,
                                                const int *__restrict__ col, const T *__restrict__ A,
                                                const T *__restrict__ dinv, const T *__restrict__ r, T *e, int B,
                                                int rpc)
@@ -213,7 +219,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_b_first(int n, const int *__
 
 // one Chebyshev step on interior rows: q = r - A e, d = c1 d + c2 D^-1 q, e' = e + d
 template <class T, int Q>
-__global__ void __launch_bounds__(kRowThreads, 2) k_b_cheb(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(row_threads(sizeof(T) * Q), 2) k_b_cheb(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                 const T *__restrict__ A, const T *__restrict__ dinv,
                                                 const uint8_t *__restrict__ btag, const T *__restrict__ r,
                                                 const T *__restrict__ e, T *__restrict__ eout, T *__restrict__ d,
@@ -242,7 +248,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_b_cheb(int n, const int *__r
 }
 
 template <class T, int Q>
-__global__ void __launch_bounds__(kRowThreads, 2) k_b_residual(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(row_threads(sizeof(T) * Q), 2) k_b_residual(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                     const T *__restrict__ A, const uint8_t *__restrict__ btag,
                                                     const T *__restrict__ r, const T *__restrict__ e,
                                                     T *__restrict__ qo, int B, int rpc)
@@ -267,7 +273,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_b_residual(int n, const int 
 
 // y = M x for a CSR transfer matrix (empty rows give 0)
 template <class T, int Q>
-__global__ void __launch_bounds__(kRowThreads, 2) k_b_restrict(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(row_threads(sizeof(T) * Q), 2) k_b_restrict(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                     const T *__restrict__ w, const T *__restrict__ x,
                                                     T *__restrict__ y, int B, int rpc)
 {
@@ -281,7 +287,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_b_restrict(int n, const int 
 
 // ef += P ec - (P ec)[row 0]
 template <class T, int Q>
-__global__ void __launch_bounds__(kRowThreads, 2) k_b_prolong(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(row_threads(sizeof(T) * Q), 2) k_b_prolong(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                    const T *__restrict__ w, const T *__restrict__ ec,
                                                    T *__restrict__ ef, int B, int rpc)
 {
@@ -309,7 +315,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_b_prolong(int n, const int *
 // A CTA of 128 threads owns 16 rows x 32 columns (2 x 2 per thread) and takes K
 // in tiles of 32, the next tile's loads in flight during the current one: 196
 // CTAs for 1560 rows x 64 columns, where 32 rows x 64 columns per CTA gave 49
-// and 234 us.
+// and 234 us.  Near the largest coarsest level too, where the inverse is read
+// twice from beyond L2: 7394 rows x 64 columns (FP32) 970 us -> 494.
 template <class T, int B>
 __global__ void __launch_bounds__(128) k_b_dense(int n, const T *__restrict__ inv, const T *__restrict__ R,
                                                  T *__restrict__ E)
@@ -403,7 +410,7 @@ __global__ void __launch_bounds__(256) k_b_resid64(int n, const int *__restrict_
 }
 
 template <class X, int Q>
-__global__ void __launch_bounds__(kRowThreads, 2) k_b_apply64(int n, const int *__restrict__ rp, const int *__restrict__ col,
+__global__ void __launch_bounds__(row_threads(sizeof(X) * Q), 2) k_b_apply64(int n, const int *__restrict__ rp, const int *__restrict__ col,
                                                    const double *__restrict__ A, const X *__restrict__ z,
                                                    double *__restrict__ w, int B, int rpc)
 {
@@ -767,7 +774,8 @@ void bsmooth(mgm_batch *b, BLev<T> &L, bool zero_start)
     const double lM = 1.05 * L.lmax, lm = L.lmax / b->cheb_ratio;
     const double th = 0.5 * (lM + lm), de = 0.5 * (lM - lm), sig = th / de;
     double rho = 1.0 / sig;
-    const RowShape sl = row_shape(L.n), sb = row_shape(L.nbl);
+    const RowShape sl = row_shape(L.n, sizeof(T) * Q), sb = row_shape(L.nbl, sizeof(T) * Q);
+    const RowShape sf = row_shape(L.n, 0);  // the first step gathers little: 54 us so, 73 on fewer threads (FP64)
     auto bnd = [&] {
         if (L.nbl == 0) return;
         k_b_bnd<T, Q><<<sb.grid, sb.threads, 0, s>>>(L.nbl, L.bnd_list, L.rp, L.col, L.A, L.dinv, L.r, L.e, B,
@@ -785,8 +793,8 @@ void bsmooth(mgm_batch *b, BLev<T> &L, bool zero_start)
             rho = rn;
         }
         if (step == 0 && zero_start)
-            k_b_first<T, Q><<<sl.grid, sl.threads, 0, s>>>(L.n, L.rp, L.col, L.A, L.dinv, L.btag, L.near, L.r, L.e2,
-                                                           L.d, B, (T)c2, sl.rpc);
+            k_b_first<T, Q><<<sf.grid, sf.threads, 0, s>>>(L.n, L.rp, L.col, L.A, L.dinv, L.btag, L.near, L.r, L.e2,
+                                                           L.d, B, (T)c2, sf.rpc);
         else
             k_b_cheb<T, Q><<<sl.grid, sl.threads, 0, s>>>(L.n, L.rp, L.col, L.A, L.dinv, L.btag, L.r, L.e, L.e2, L.d,
                                                            B, (T)c1, (T)c2, step == 0 ? 1 : 0, sl.rpc);
@@ -811,7 +819,7 @@ void bvcycle(mgm_batch *b, std::vector<BLev<T>> &Ls, int l)
     }
     bsmooth<T, Q>(b, L, true);  // from e = 0
     BLev<T> &C = Ls[l + 1];
-    const RowShape sl = row_shape(L.n), sc = row_shape(C.n);
+    const RowShape sl = row_shape(L.n, sizeof(T) * Q), sc = row_shape(C.n, sizeof(T) * Q);
     k_b_residual<T, Q><<<sl.grid, sl.threads, 0, s>>>(L.n, L.rp, L.col, L.A, L.btag, L.r, L.e, L.q, B,
                                                        sl.rpc);
     MGM_LAUNCHED();
@@ -866,7 +874,7 @@ void bfgmres(mgm_batch *b, int nrhs, int *vcycles, double *rel_res)
     if constexpr (sizeof(T) == 8) Z = b->Z64.p; else Z = b->Z32.p;
     double *V = b->V.p, *X = b->X.p, *hp = b->h_pinned, *dsc = b->hsc.p;
     const int gres = dot_grid(n);
-    const RowShape sl = row_shape(n);
+    const RowShape sl = row_shape(n, sizeof(T) * Q);
     const int gdot = (int)std::max(1L, std::min<long>((n + (256 / B) - 1) / (256 / B), 148L * 8));
     const size_t part_need = std::max({(size_t)gres * 2 * B, (size_t)gdot * 8 * B, (size_t)148 * 16 * B});
     if (b->part.n < part_need) b->part.alloc(part_need);
