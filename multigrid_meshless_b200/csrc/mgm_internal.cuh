@@ -88,11 +88,17 @@ void *dev_alloc(size_t bytes);
 void dev_free(void *p, size_t bytes) noexcept;
 void trim_memory() noexcept;  // gives back what the pool holds beyond its bound
 
-// at the top of every entry point: the bound holds again when the call returns,
-// with an error too
+// at the top of every entry point: when the call returns, with an error too, the
+// pool's bound holds again and the thread names the stream it named before (none,
+// or the calling entry point's), so that no stream outlives its owner here
 struct TrimScope {
-    TrimScope() = default;
-    ~TrimScope() { trim_memory(); }
+    cudaStream_t before;
+    TrimScope() : before(alloc_stream()) {}
+    ~TrimScope()
+    {
+        trim_memory();
+        alloc_stream(before);
+    }
     TrimScope(const TrimScope &) = delete;
     TrimScope &operator=(const TrimScope &) = delete;
 };
