@@ -431,7 +431,8 @@ __global__ void __launch_bounds__(256) k_decode_bwd(int n, const bf16 *__restric
 
 // Backward pass of a layer on the tensor cores.  The activations and weights
 // are BF16; the FP32 gradients dz enter as three BF16 parts whose sum is the
-// FP32 value (8 significand bits each), so every product is exact and the
+// FP32 value (8 significand bits each; below 2^-110 the last part falls under
+// BF16's smallest number), so every product is exact and the
 // FP32 accumulation is the only rounding, as it was with FP32 multiply-adds on
 // the CUDA cores.  The small parts are accumulated before the large one, and a
 // tile's sums start from zero and are added to the running FP32 sums, which
